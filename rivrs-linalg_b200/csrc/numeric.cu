@@ -45,6 +45,7 @@
 
 #include <thread>
 
+#include "block.cuh"
 #include "dense.cuh"
 #include "front.cuh"
 #include "mlp.cuh"
@@ -237,232 +238,6 @@ __global__ void k_tpp(const int32_t* ids, int n, DFront* F, Arenas A, DevOpts o)
   if (w >= n) return;
   __shared__ int cnt[8][2];
   warp_tpp_front(ids[w], F, A, o, cnt[threadIdx.x >> 5]);
-}
-
-constexpr int NT = APTP_THREADS;  // threads of the CTA APTP kernel
-constexpr int IBMAX = 32; // inner block size supported by the kernels
-
-struct CtaShared {
-  double T[IBMAX][IBMAX + 1];
-  double Lj[IBMAX];
-  int bperm[IBMAX];
-  int8_t bdt[IBMAX];
-  double bdd[IBMAX];
-  double bdo[IBMAX];
-  int bnelim, eff, n1, n2, end_pos, k;
-  int tmpi[NT];
-  double tmpd[NT];
-};
-
-// Complete pivoting on the bs x bs diagonal block held in shared memory
-// (factor_block_diagonal, factor.rs:891-1153).  Per pivot step, warp 0 finds
-// the pivot (lane = column, its rows in registers; the reduction keeps the
-// largest magnitude and, among equal ones, the smallest (column, row) key: the
-// reference's column-then-row scan with a strict >), performs the symmetric
-// swaps, the reciprocal and the scaling of the pivot column(s); then every
-// warp takes part in the rank-1 / rank-2 update (warps take columns, lanes
-// rows).  Two CTA barriers per step; every entry gets the same operations as
-// in the reference's loops.
-__device__ void cta_block_factor(CtaShared& sh, int bs, double small) {
-  static_assert(NT == 256 && IBMAX == 32, "the update's column split assumes 8 warps and 32-column blocks");
-  double(*T)[IBMAX + 1] = sh.T;
-  __shared__ int s_kind;
-  __shared__ double s_d[3];
-  // column maxima of the trailing triangle after each update (bits of |v| and the (column, row) key of the
-  // first maximum in row order), left by the updating warps for the next step's pivot search
-  __shared__ unsigned s_chi[IBMAX], s_clo[IBMAX], s_ckey[IBMAX];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < IBMAX) { sh.bperm[tid] = tid; sh.bdt[tid] = PT_DELAYED; sh.bdd[tid] = 0; sh.bdo[tid] = 0; }
-  __syncthreads();
-  // swap_symmetric_block limited to the block (warp 0)
-  auto swp = [&](int i, int j) {
-    if (i == j) return;
-    if (i > j) { int t = i; i = j; j = t; }
-    if (lane == 0) {
-      double t = T[i][i]; T[i][i] = T[j][j]; T[j][j] = t;
-      int p = sh.bperm[i]; sh.bperm[i] = sh.bperm[j]; sh.bperm[j] = p;
-    }
-    if (lane < i) { double t = T[i][lane]; T[i][lane] = T[j][lane]; T[j][lane] = t; }
-    if (lane > i && lane < j) { double t = T[lane][i]; T[lane][i] = T[j][lane]; T[j][lane] = t; }
-    if (lane > j && lane < bs) { double t = T[lane][i]; T[lane][i] = T[lane][j]; T[lane][j] = t; }
-    __syncwarp();
-  };
-  // each updated column j0 + 8q of this warp: the maximum of |T[i][j]| over rows j <= i < bs (the lanes'
-  // new values) and the smallest row holding it, as the scan in row order finds them (entries that are not
-  // > 0, NaN included, never count)
-  auto col_maxima = [&](int j0, int i, const double* nvq) {
-#pragma unroll
-    for (int q = 0; q < IBMAX / 8; ++q) {
-      const int j = j0 + 8 * q;
-      if (j < bs) {  // uniform over the warp
-        const double a = (i >= j && i < bs) ? fabs(nvq[q]) : 0.0;
-        const bool pos = a > 0.0;
-        const unsigned long long bits = pos ? (unsigned long long)__double_as_longlong(a) : 0ull;
-        const unsigned h1 = (unsigned)(bits >> 32), l1 = (unsigned)bits;
-        const unsigned mh = __reduce_max_sync(0xffffffffu, h1);
-        const unsigned ml = __reduce_max_sync(0xffffffffu, h1 == mh ? l1 : 0u);
-        const unsigned kk = __reduce_min_sync(0xffffffffu, (pos && h1 == mh && l1 == ml) ? (unsigned)(j * 64 + i)
-                                                                                          : 0xffffffffu);
-        if (lane == 0) { s_chi[j] = mh; s_clo[j] = ml; s_ckey[j] = kk; }
-      }
-    }
-  };
-  int k = 0;
-  for (;;) {
-    const int cur = k;
-    if (warp == 0) {
-      int kind = 0;  // 0 stop, 1 1x1 (+ rank-1 update), 2 2x2 (+ rank-2 update)
-      if (cur < bs) {
-        // arg-max over the lower triangle of [cur, bs)^2: lane = column, its first maximum in row order
-        unsigned hi = 0, lo = 0, key = 0xffffffffu;
-        if (lane >= cur && lane < bs) {
-          if (cur == 0) {  // the first step scans the block
-            double col[IBMAX];
-#pragma unroll
-            for (int i = 0; i < IBMAX; ++i) col[i] = T[i][lane];
-            // four interleaved scans (rows i mod 4), each keeping its first maximum,
-            // merged to the first maximum in row order
-            double b4[4] = {0.0, 0.0, 0.0, 0.0};
-            unsigned k4[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
-#pragma unroll
-            for (int i = 0; i < IBMAX; ++i)
-              if (i >= lane && i < bs) {
-                const double v = fabs(col[i]);
-                if (v > b4[i & 3]) { b4[i & 3] = v; k4[i & 3] = (unsigned)(lane * 64 + i); }
-              }
-            double bv = 0.0;
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-              if (b4[q] > bv || (b4[q] == bv && k4[q] < key)) { bv = b4[q]; key = k4[q]; }
-            const unsigned long long bits = (unsigned long long)__double_as_longlong(bv);  // bv >= 0
-            hi = (unsigned)(bits >> 32);
-            lo = (unsigned)bits;
-          } else {  // left by the previous step's update
-            hi = s_chi[lane];
-            lo = s_clo[lane];
-            key = s_ckey[lane];
-          }
-        }
-        const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-        const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
-        key = __reduce_min_sync(0xffffffffu, (hi == mhi && lo == mlo) ? key : 0xffffffffu);
-        const double maxv = __longlong_as_double((long long)(((unsigned long long)mhi << 32) | mlo));
-        int mr = cur, mc = cur;
-        if (key != 0xffffffffu) { mc = (int)(key / 64); mr = (int)(key % 64); }
-        if (maxv >= small) {
-          if (mr == mc) {
-            // the pivot's reciprocal from its value before the swap (the same number), so
-            // the division overlaps the swap
-            const double dkk = T[mr][mr], inv = 1.0 / dkk;
-            swp(cur, mr);
-            if (lane > cur && lane < bs) T[lane][cur] = __dmul_rn(T[lane][cur], inv);
-            if (lane == 0) { sh.bdt[cur] = PT_1X1; sh.bdd[cur] = dkk; s_d[0] = dkk; }
-            kind = 1;
-          } else {
-            const int t = mr, mi = mc;
-            const double amm = T[mi][mi], att = T[t][t], atm = T[t][mi];
-            const double delta = __dsub_rn(__dmul_rn(amm, att), __dmul_rn(atm, atm));
-            const int remaining = bs - cur;
-            if (remaining < 2) {
-              const int pp = fabs(amm) >= fabs(att) ? mi : t;
-              const double dkk = T[pp][pp], inv = 1.0 / dkk;
-              swp(cur, pp);
-              if (!(fabs(dkk) < small)) {
-                if (lane > cur && lane < bs) T[lane][cur] = __dmul_rn(T[lane][cur], inv);
-                if (lane == 0) { sh.bdt[cur] = PT_1X1; sh.bdd[cur] = dkk; s_d[0] = dkk; }
-                kind = 1;  // the rank-1 update is empty here
-              }
-            } else if (fabs(delta) >= __dmul_rn(__dmul_rn(0.5, atm), atm)) {
-              // the swaps bring (mi, t) to (cur, cur + 1): a11 = amm, a22 = att, a21 = atm, and the
-              // determinant a11 a22 - a21 a21 is delta; its reciprocal overlaps the swaps
-              const double inv_det = 1.0 / delta;
-              swp(cur, mi);
-              const int nt = (t == cur) ? mi : t;
-              swp(cur + 1, nt);
-              const double a11 = T[cur][cur], a22 = T[cur + 1][cur + 1], a21 = T[cur + 1][cur];
-              if (lane >= cur + 2 && lane < bs) {
-                const double ai1 = T[lane][cur], ai2 = T[lane][cur + 1];
-                T[lane][cur] = __dmul_rn(__dsub_rn(__dmul_rn(ai1, a22), __dmul_rn(ai2, a21)), inv_det);
-                T[lane][cur + 1] = __dmul_rn(__dsub_rn(__dmul_rn(ai2, a11), __dmul_rn(ai1, a21)), inv_det);
-              }
-              if (lane == 0) {
-                sh.bdt[cur] = PT_2X2; sh.bdt[cur + 1] = PT_2X2B;
-                sh.bdd[cur] = a11; sh.bdd[cur + 1] = a22; sh.bdo[cur] = a21;
-                s_d[0] = a11; s_d[1] = a21; s_d[2] = a22;
-              }
-              kind = 2;
-            } else {
-              const int pp = fabs(amm) >= fabs(att) ? mi : t;
-              const double dkk = T[pp][pp], inv = 1.0 / dkk;
-              swp(cur, pp);
-              if (lane > cur && lane < bs) T[lane][cur] = __dmul_rn(T[lane][cur], inv);
-              if (lane == 0) { sh.bdt[cur] = PT_1X1; sh.bdd[cur] = dkk; s_d[0] = dkk; }
-              kind = 1;
-            }
-          }
-        }
-      }
-      if (lane == 0) s_kind = kind;
-    }
-    __syncthreads();
-    const int kind = s_kind;
-    if (kind == 0) break;
-    const int i = lane;
-    double nv[IBMAX / 8] = {};  // the lane's (row's) new entries in the warp's columns
-    if (kind == 1) {  // T[i][j] -= T[i][cur] (T[j][cur] d), cur < j <= i
-      const double dkk = s_d[0];
-      if (i > cur && i < bs) {
-        const double lc = T[i][cur];
-        double lj[IBMAX / 8], tij[IBMAX / 8];
-#pragma unroll
-        for (int q = 0; q < IBMAX / 8; ++q) {
-          const int j = cur + 1 + warp + 8 * q;
-          const bool in = j <= i;
-          lj[q] = in ? T[j][cur] : 0.0;
-          tij[q] = in ? T[i][j] : 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < IBMAX / 8; ++q) {
-          const int j = cur + 1 + warp + 8 * q;
-          if (j <= i) {
-            nv[q] = __dsub_rn(tij[q], __dmul_rn(lc, __dmul_rn(lj[q], dkk)));
-            T[i][j] = nv[q];
-          }
-        }
-      }
-      col_maxima(cur + 1 + warp, i, nv);
-      k += 1;
-    } else {  // rank-2 over cur + 2 <= j <= i
-      const double a11 = s_d[0], a21 = s_d[1], a22 = s_d[2];
-      if (i >= cur + 2 && i < bs) {
-        const double c1 = T[i][cur], c2 = T[i][cur + 1];
-        double l1[IBMAX / 8], l2[IBMAX / 8], tij[IBMAX / 8];
-#pragma unroll
-        for (int q = 0; q < IBMAX / 8; ++q) {
-          const int j = cur + 2 + warp + 8 * q;
-          const bool in = j <= i;
-          l1[q] = in ? T[j][cur] : 0.0;
-          l2[q] = in ? T[j][cur + 1] : 0.0;
-          tij[q] = in ? T[i][j] : 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < IBMAX / 8; ++q) {
-          const int j = cur + 2 + warp + 8 * q;
-          if (j <= i) {
-            const double w1 = __dadd_rn(__dmul_rn(l1[q], a11), __dmul_rn(l2[q], a21));
-            const double w2 = __dadd_rn(__dmul_rn(l1[q], a21), __dmul_rn(l2[q], a22));
-            nv[q] = __dsub_rn(tij[q], __dadd_rn(__dmul_rn(c1, w1), __dmul_rn(c2, w2)));
-            T[i][j] = nv[q];
-          }
-        }
-      }
-      col_maxima(cur + 2 + warp, i, nv);
-      k += 2;
-    }
-    __syncthreads();
-  }
-  if (tid == 0) sh.bnelim = k;
-  __syncthreads();
 }
 
 // Full symmetric swap of positions i, j inside a view of `rows` rows
@@ -769,10 +544,10 @@ __device__ __forceinline__ void cta_aptp_front(CtaShared& sh, int* tpp_cnt, int 
       __syncwarp();
       WarpTpp T{Av, m, p, tid};
       int64_t add = T.run(gne, p, perm, D, &tpp_cnt[0], &tpp_cnt[1], o);
-      if (tid == 0) sh.tmpi[0] = (int)add;
+      if (tid == 0) sh.tmpi = (int)add;
     }
     __syncthreads();
-    gne += sh.tmpi[0];
+    gne += sh.tmpi;
     n1 += tpp_cnt[0];
     n2 += tpp_cnt[1];
   }

@@ -40,6 +40,13 @@ __device__ __forceinline__ void chain_enter() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Kernels of one wave's small and medium fronts (launch_beside): each lets the
+// next one start at once, touches nothing of the others' fronts, and before a
+// CTA ends waits for the launch before it, so that the stream goes on only
+// when all of them are complete.
+__device__ __forceinline__ void wave_kernel_enter() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wave_kernel_exit() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 struct DevOpts {
   double threshold;
   double small;

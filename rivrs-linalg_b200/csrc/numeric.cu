@@ -50,6 +50,7 @@
 #include "front.cuh"
 #include "mlp.cuh"
 #include "rvg_internal.h"
+#include "tpp.cuh"
 
 namespace rvg {
 
@@ -567,34 +568,22 @@ __global__ void __launch_bounds__(NT) k_aptp(const int32_t* ids, int n, DFront* 
 // next front from a work queue (*next, zero at launch) until the list is
 // done.  The host lists the fronts largest first, so the long ones start
 // early and the short ones fill in behind them.  Which CTA factors a front
-// changes nothing in its result.
-// One persistent launch for a wave's small and medium fronts: items
-// [0, na) are medium fronts (one CTA each, listed largest first), items
-// [na, na + ceil(nt / 8)) groups of 8 small fronts (TPP, one warp each),
-// taken in order from one atomic counter, so the small fronts fill the
-// multiprocessors the long medium fronts leave.  Which CTA or warp takes a
-// front changes nothing in its arithmetic.
-__global__ void __launch_bounds__(NT) k_front_queue(const int32_t* ids, int na, const int32_t* tids, int nt,
-                                                    int32_t* next, DFront* F, Arenas A, DevOpts o) {
-  static_assert(NT == 256, "a group of small fronts is one per warp of the CTA");
+// changes nothing in its result.  
+__global__ void __launch_bounds__(NT) k_front_queue(const int32_t* ids, int na, int32_t* next, DFront* F, Arenas A,
+                                                       DevOpts o) {
   __shared__ CtaShared sh;
   __shared__ int tpp_cnt[2];
-  __shared__ int wcnt[NT / 32][2];
   __shared__ int s_i;
-  const int ng = (nt + 7) / 8;
+  wave_kernel_enter();
   for (;;) {
     if (threadIdx.x == 0) s_i = atomicAdd(next, 1);
     __syncthreads();
     const int i = s_i;
     __syncthreads();  // every thread has read s_i before thread 0 takes the next item
-    if (i >= na + ng) break;
-    if (i < na) {
-      cta_aptp_front(sh, tpp_cnt, ids[i], F, A, o);
-    } else {
-      const int wl = threadIdx.x >> 5, f = (i - na) * 8 + wl;
-      if (f < nt) warp_tpp_front(tids[f], F, A, o, wcnt[wl]);
-    }
+    if (i >= na) break;
+    cta_aptp_front(sh, tpp_cnt, ids[i], F, A, o);
   }
+  wave_kernel_exit();
 }
 
 }  // namespace rvg
@@ -1781,6 +1770,26 @@ static void launch_chain(const rvg_handle* h, void (*kern)(KP...), dim3 grid, di
   (void)cudaLaunchKernelEx(&cfg, kern, args...);  // a failure stays the thread's last error, checked as for <<<>>>
 }
 
+// The launches of a wave's small and medium fronts touch different fronts, so
+// all but the first may start while the one before still runs (programmatic
+// stream serialization; wave_kernel_enter / _exit).  Together they are complete
+// when the last one is.
+template <typename... KP, typename... AP>
+static void launch_beside(bool beside, void (*kern)(KP...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                          AP... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = beside ? 1 : 0;
+  (void)cudaLaunchKernelEx(&cfg, kern, args...);  // a failure stays the thread's last error
+}
+
 int launch_syrk(rvg_handle* h, const SyrkArgs& ga, int64_t kmax, bool mixed) {
   cudaStream_t st = h->st;
   if (mixed) {
@@ -2359,6 +2368,46 @@ int refactor_fp64(rvg_handle* h, const std::vector<int32_t>& redo, const Arenas&
   return RVG_OK;
 }
 
+// Launches of a wave's TPP fronts (one CTA each, k_tpp_cta), which sorts them
+// by size, largest first.  A launch's CTAs all reserve the shared memory of its
+// largest front, so the fronts are split where 8, 4, 2 or 1 of them fit on a
+// multiprocessor (28 / 56 / 112 / 226 KB; larger ones stay in global memory),
+// and a smaller class joins the launch above it while that still runs in one
+// go (fewer launches; the multiprocessors have room).  Threads: a front's steps
+// are latency bound, so 256 while every CTA is resident at that width; where a
+// class has several rounds of CTAs its fronts share the issue slots, and two
+// warps per front waste fewer of them on the decisions every warp repeats.
+struct TppLaunch { int first, count, threads; size_t smem; };
+
+std::vector<TppLaunch> plan_tpp(const rvg_handle* h, std::vector<int32_t>& ids) {
+  std::vector<TppLaunch> out;
+  if (ids.empty()) return out;
+  auto bytes = [&](int32_t s) {
+    const DFront& f = h->h_fronts[s];
+    return (size_t)tpp_ld(f.m) * f.k * 8 + (size_t)f.k * 4;
+  };
+  std::stable_sort(ids.begin(), ids.end(), [&](int32_t a, int32_t b) { return bytes(a) > bytes(b); });
+  constexpr size_t KB = 1024;
+  const size_t lim[5] = {SIZE_MAX, TPP_SMEM_MAX, 112 * KB, 56 * KB, 28 * KB};  // class c: at most lim[c] bytes
+  const int per_sm[5] = {8, 1, 2, 4, 8};
+  const int n = (int)ids.size();
+  int i = 0;
+  while (i < n) {
+    const size_t b = bytes(ids[i]);
+    int c = 4;
+    while (b > lim[c]) --c;
+    const int cap = per_sm[c] * h->nsm;
+    int e = i;
+    while (e < n && (c == 4 || bytes(ids[e]) > lim[c + 1])) ++e;
+    if (c > 0 && e - i < cap) e = std::min(n, i + cap) == n ? n : e;  // the rest fits beside it
+    TppLaunch t{i, e - i, 0, c == 0 ? 0 : b};
+    t.threads = t.count <= cap ? 256 : (c == 4 ? 64 : 128);
+    out.push_back(t);
+    i = e;
+  }
+  return out;
+}
+
 // The numeric factorization proper: the level-set schedule of
 // factor_tree_levelset (numeric.rs:1957-2163) with every front of a wave
 // processed by the same launches.
@@ -2499,6 +2548,8 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
       const DFront &fa = h->h_fronts[a], &fb = h->h_fronts[b];
       return (double)fa.k * fa.m * fa.m > (double)fb.k * fb.m * fb.m;
     });
+    const std::vector<TppLaunch> tpp_launches = plan_tpp(h, tpp_ids);
+    int n_small_launches = 0;
     std::vector<ScatterItem> sitems;
     for (int64_t s : wave)
       for (int64_t e = P.amap_ptr[s]; e < P.amap_ptr[s + 1]; e += 256) sitems.push_back(ScatterItem{(int32_t)s, 0, e});
@@ -2604,18 +2655,25 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
     }
     // ---- dense factorization
     mark(h, -1);
-    if (!tpp_ids.empty() || !aptp_ids.empty()) {
-      // the wave's small and medium fronts in one persistent launch (profiling: part "aptp")
+    // the wave's small and medium fronts (profiling: part "aptp")
+    bool group = false;  // a launch of the group has gone out: the next ones may start beside it
+    if (!aptp_ids.empty()) {
       if (!h->aptp_ctas) {  // resident CTAs of the queue kernel on this device
-        int occ = 0, sms = 0;
+        int occ = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_front_queue, NT, 0));
-        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-        h->aptp_ctas = std::max(1, occ) * std::max(1, sms);
+        h->aptp_ctas = std::max(1, occ) * std::max(1, h->nsm);
       }
-      const int na = (int)aptp_ids.size(), nt = (int)tpp_ids.size(), items = na + (nt + 7) / 8;
-      k_front_queue<<<(unsigned)std::min(items, h->aptp_ctas), NT, 0, st>>>(
-          (const int32_t*)(D + o_aptp), na, (const int32_t*)(D + o_tpp), nt, (int32_t*)(D + o_q), h->d_fronts, A,
-          dop);
+      const int na = (int)aptp_ids.size();
+      k_front_queue<<<(unsigned)std::min(na, h->aptp_ctas), NT, 0, st>>>((const int32_t*)(D + o_aptp), na,
+                                                                          (int32_t*)(D + o_q), h->d_fronts, A, dop);
+      group = true;
+      n_small_launches++;
+    }
+    for (const TppLaunch& t : tpp_launches) {
+      launch_beside(group, k_tpp_cta, (unsigned)t.count, (unsigned)t.threads, t.smem, st,
+                    (const int32_t*)(D + o_tpp) + t.first, h->d_fronts, A, dop, (int)(t.smem > 0));
+      group = true;
+      n_small_launches++;
     }
     mark(h, RVG_PART_APTP);
     if (learned) {  // the routes of the large fronts (the device is busy with the fronts queued above)
@@ -2708,7 +2766,7 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
       h->syrk_flops += 2.0 * (double)f.ne * (double)f.nfs * (double)(f.nfs + 1) / 2.0;
     }
     h->launches += 1 + (int64_t)eitems.size() * 0 + (sitems.empty() ? 0 : 1) +
-                   ((tpp_ids.empty() && aptp_ids.empty()) ? 0 : 1) + (witems.empty() ? 0 : 1) + (gitems.empty() ? 0 : 1) + 2 +
+                   n_small_launches + (witems.empty() ? 0 : 1) + (gitems.empty() ? 0 : 1) + 2 +
                    (dly_ids.empty() ? 0 : 1) + (zitems.empty() ? 0 : 1);
     for (size_t q = 0; q < maxch; ++q) h->launches += eitems[q].empty() ? 0 : 1;
     if (h->profiling) {  // the device memory in use (profiling runs only: the query costs host time)
@@ -2905,6 +2963,7 @@ rvg_status rvg_create(int64_t n, int64_t nsup, const int64_t* sup_begin, const i
   CK(cudaMallocHost((void**)&h->h_norms, 4 * sizeof(double)));
   if (o.graph_refactor == 2 && (rc = vm_create(h.get()))) return (rvg_status)rc;  // address-stable arenas
   if ((rc = presize_arenas(h.get()))) return (rvg_status)rc;
+  CK(cudaFuncSetAttribute(k_tpp_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TPP_SMEM_MAX));
   CK(cudaFuncSetAttribute(k_syrk_lower, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G_SMEM));
   CK(cudaFuncSetAttribute(k_syrk_inner, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G_SMEM));
   CK(cudaFuncSetAttribute(k_syrk_tc<1, TC_TF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));

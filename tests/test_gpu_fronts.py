@@ -1,0 +1,62 @@
+"""Small and medium fronts of given shapes, bit for bit against the oracle: two
+leaf fronts of k columns and k + r rows under one dense root of order r."""
+import numpy as np
+import pytest
+
+from test_gpu_parity import assert_parity, run_both
+
+pytestmark = pytest.mark.gpu
+
+
+def arrow_system(rv, k, r, seed, kind):
+    rng = np.random.default_rng(seed)
+    n = 2 * k + r
+    a = rng.standard_normal((n, n))
+    a = a + a.T
+    a[:k, k:2 * k] = 0.0
+    a[k:2 * k, :k] = 0.0
+    d = np.arange(2 * k)
+    if kind == "delay":  # tiny diagonals: 2x2 pivots and delayed columns
+        a[d, d] *= 1e-6
+        a[:k, :k] *= 1e-3
+    elif kind == "zero":  # an all-zero column inside a front, and ties
+        a = np.sign(a) * (np.abs(a) > 0.7)
+        a[k // 2, :] = 0.0
+        a[:, k // 2] = 0.0
+        a[2 * k:, 2 * k:] += 50.0 * np.eye(r)
+    return rv.problems.from_scipy(f"arrow{k}_{r}_{kind}", a)
+
+
+def check(rv, orc, k, r, kind, **opts):
+    s = arrow_system(rv, k, r, 100 * k + r, kind)
+    solver, ref, b = run_both(rv, orc, s, order=np.arange(s.n, dtype=np.int64), **opts)
+    assert_parity(rv, s, solver, ref, b, bwd=1e-8 if kind == "zero" else 1e-12)
+    solver.close()
+    ref.close()
+
+
+# (k, r): one column, odd sizes, warp remainders; then fronts on either side of the 28, 56, 112 and 226 KB of
+# shared memory at which the launch changes, the last one too large for it
+@pytest.mark.parametrize("k,r", [(1, 3), (2, 1), (5, 33), (31, 32), (31, 82), (31, 90), (31, 200), (31, 430),
+                                 (31, 880), (31, 940)])
+@pytest.mark.parametrize("kind", ["plain", "delay", "zero"])
+def test_tpp_fronts(rv, orc, k, r, kind):
+    check(rv, orc, k, r, kind, nemin=1)
+
+
+@pytest.mark.parametrize("k", [40, 77, 128])
+@pytest.mark.parametrize("kind", ["plain", "delay", "zero"])
+def test_small_leaf_fronts(rv, orc, k, kind):
+    check(rv, orc, k, 60, kind)
+
+
+# 32-column blocks with and without a remainder, panels and tiles of 32 rows and one more or less
+@pytest.mark.parametrize("k,r", [(32, 1), (33, 31), (63, 32), (64, 33), (65, 100), (97, 64), (300, 37)])
+@pytest.mark.parametrize("kind", ["plain", "delay", "zero"])
+def test_medium_fronts(rv, orc, k, r, kind):
+    check(rv, orc, k, r, kind, small_leaf_threshold=0)
+
+
+@pytest.mark.parametrize("ib,nb", [(8, 32), (17, 64), (32, 96)])
+def test_medium_fronts_block_sizes(rv, orc, ib, nb):
+    check(rv, orc, 150, 45, "delay", small_leaf_threshold=0, inner_block_size=ib, outer_block_size=nb)

@@ -48,6 +48,8 @@ struct CtaShared {
   double bdo[IBMAX];
   int bnelim, eff, n1, n2, end_pos, k;
   int tmpi;
+  double dinv[IBMAX];
+  alignas(16) double TT[IBMAX][IBMAX + 2];  // the factored block transposed: TT[l][j] = L(j, l) (panel_rows)
   // cta_block_factor only
   double Tb[IBMAX][IBMAX + 1];  // the other buffer of the trailing block
   double Lc[IBMAX][IBMAX + 1];  // Lc[c][r]: finished column c at the row of original index r
@@ -229,6 +231,76 @@ __device__ void cta_block_factor(CtaShared& sh, int bs, double small) {
   if (warp == 0) sh.bperm[lane] = id;
   if (tid == 0) sh.bnelim = cur;
   __syncthreads();
+}
+
+// The reciprocals each panel row's D^-1 step uses, 1 / d (1x1) or 1 / det
+// (first column of a 2x2), by 32 threads (c = pivot).
+__device__ __forceinline__ double pivot_inv(int c, int n, const int8_t* bdt, const double* bdd, const double* bdo) {
+  if (c >= n) return 0.0;
+  if (bdt[c] == PT_1X1) return 1.0 / bdd[c];
+  if (bdt[c] == PT_2X2 && c + 1 < IBMAX)
+    return 1.0 / __dsub_rn(__dmul_rn(bdd[c], bdd[c + 1]), __dmul_rn(bdo[c], bdo[c]));
+  return 0.0;
+}
+
+// One panel row (apply_and_check, factor.rs:1295-1408) in registers, x[j] =
+// its entry in the block's column j: x L11^-T over the n eliminated columns,
+// then D^-1.  The outer loop is over the finished column l, the inner one
+// over the later columns j: each x[j] still takes its terms in ascending l,
+// but the n - l updates of a step are independent (the loop over j first is
+// one dependent chain of n (n - 1) / 2 multiply-adds).  TT holds L11 by
+// columns, so the inner loop reads two entries per shared-memory load.
+// Returns the first pivot (1x1 or 2x2 start) with an entry at or above bound.
+__device__ __forceinline__ int panel_row(double (&x)[IBMAX], const double (*TT)[IBMAX + 2], const int8_t* bdt,
+                                         const double* bdd, const double* bdo, const double* dinv, int n,
+                                         double bound) {
+#pragma unroll
+  for (int l = 0; l + 1 < IBMAX; ++l) {
+    if (l + 1 >= n) break;
+    const double nx = -x[l];
+#pragma unroll
+    for (int j = (l + 1) & ~1; j < IBMAX; j += 2) {
+      const double2 t = *reinterpret_cast<const double2*>(&TT[l][j]);
+      if (j > l && j < n) x[j] = __fma_rn(nx, t.x, x[j]);
+      if (j + 1 < n) x[j + 1] = __fma_rn(nx, t.y, x[j + 1]);
+    }
+  }
+  int fail = n;
+#pragma unroll
+  for (int c = 0; c < IBMAX; ++c) {
+    if (c >= n) continue;
+    bool bad = false;
+    if (bdt[c] == PT_1X1) {
+      x[c] = __dmul_rn(x[c], dinv[c]);
+      bad = fabs(x[c]) >= bound;
+    } else if (bdt[c] == PT_2X2 && c + 1 < IBMAX) {
+      const double A_ = bdd[c], B_ = bdo[c], C_ = bdd[c + 1], inv_det = dinv[c];
+      const int d = c + 1 < IBMAX ? c + 1 : c;
+      const double x1 = x[c], x2 = x[d];
+      x[c] = __dmul_rn(__dsub_rn(__dmul_rn(x1, C_), __dmul_rn(x2, B_)), inv_det);
+      x[d] = __dmul_rn(__dsub_rn(__dmul_rn(x2, A_), __dmul_rn(x1, B_)), inv_det);
+      bad = fabs(x[c]) >= bound || fabs(x[d]) >= bound;
+    }
+    if (bad && c < fail) fail = c;
+  }
+  return fail;
+}
+
+// W = L D of the row (compute_ld_into, factor.rs:1536-1563), column c to
+// w[c * ldw], for the n columns of x.
+__device__ __forceinline__ void panel_row_w(const double (&x)[IBMAX], const int8_t* bdt, const double* bdd,
+                                            const double* bdo, int n, double* w, int64_t ldw) {
+#pragma unroll
+  for (int c = 0; c < IBMAX; ++c) {
+    if (c >= n) continue;
+    if (bdt[c] == PT_1X1) {
+      w[c * ldw] = __dmul_rn(x[c], bdd[c]);
+    } else if (bdt[c] == PT_2X2 && c + 1 < IBMAX) {
+      const int d = c + 1 < IBMAX ? c + 1 : c;
+      w[c * ldw] = __dadd_rn(__dmul_rn(x[c], bdd[c]), __dmul_rn(x[d], bdo[c]));
+      w[d * ldw] = __dadd_rn(__dmul_rn(x[c], bdo[c]), __dmul_rn(x[d], bdd[d]));
+    }
+  }
 }
 
 }  // namespace rvg

@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(LF_PANEL_T) k_lf_panel(LFArgs A) {
   LFState* st = A.st;
   const int bnelim = st->bnelim;
   if (bnelim == 0) return;
-  __shared__ double T[IBMAX][IBMAX + 1];
+  __shared__ alignas(16) double TT[IBMAX][IBMAX + 2];  // TT[l][j] = L11(j, l)
   __shared__ int bperm[IBMAX];
   __shared__ int8_t bdt[IBMAX];
   __shared__ double bdd[IBMAX], bdo[IBMAX], dinv[IBMAX];
@@ -228,21 +228,15 @@ __global__ void __launch_bounds__(LF_PANEL_T) k_lf_panel(LFArgs A) {
       v[u] = (j < bs && i < bs && i >= j) ? st->T[i][j] : 0.0;
     }
 #pragma unroll
-    for (int u = 0; u < 16; ++u) T[h * 16 + u][j] = v[u];
+    for (int u = 0; u < 16; ++u) TT[j][h * 16 + u] = v[u];
   }
   if (threadIdx.x < IBMAX) {
     const int c = threadIdx.x;
     bperm[c] = st->bperm[c];
-    const int8_t t = st->bdt[c];
-    const double d = st->bdd[c], o = st->bdo[c];
-    bdt[c] = t;
-    bdd[c] = d;
-    bdo[c] = o;
-    // the reciprocal each row's D^-1 step uses: 1 / d (1x1) or 1 / det (2x2 first column)
-    double r = 0.0;
-    if (c < bnelim && t == PT_1X1) r = 1.0 / d;
-    else if (c < bnelim && t == PT_2X2 && c + 1 < IBMAX) r = 1.0 / __dsub_rn(__dmul_rn(d, st->bdd[c + 1]), __dmul_rn(o, o));
-    dinv[c] = r;
+    bdt[c] = st->bdt[c];
+    bdd[c] = st->bdd[c];
+    bdo[c] = st->bdo[c];
+    dinv[c] = pivot_inv(c, bnelim, st->bdt, st->bdd, st->bdo);
   }
   if (threadIdx.x == 0) s_fail = bnelim;
   __syncthreads();
@@ -274,38 +268,10 @@ __global__ void __launch_bounds__(LF_PANEL_T) k_lf_panel(LFArgs A) {
 #pragma unroll
     for (int i = 0; i < IBMAX; ++i)
       if (i < bs) A.pb[r + (int64_t)i * bm] = raw[i];
-#pragma unroll
-    for (int j = 1; j < IBMAX; ++j)
-      if (j < bnelim) {
-#pragma unroll
-        for (int l = 0; l < j; ++l) x[j] = __fma_rn(-x[l], T[j][l], x[j]);
-      }
-    // D^-1 over the pivots (the second column of a 2x2 is handled with its first)
-#pragma unroll
-    for (int c = 0; c < IBMAX; ++c) {
-      if (c >= bnelim) continue;
-      if (bdt[c] == PT_1X1) {
-        x[c] = __dmul_rn(x[c], dinv[c]);
-      } else if (bdt[c] == PT_2X2 && c + 1 < IBMAX) {
-        const double A_ = bdd[c], B_ = bdo[c], C_ = bdd[c + 1];
-        const double inv_det = dinv[c];
-        const double x1 = x[c], x2 = x[c + 1];
-        x[c] = __dmul_rn(__dsub_rn(__dmul_rn(x1, C_), __dmul_rn(x2, B_)), inv_det);
-        x[c + 1] = __dmul_rn(__dsub_rn(__dmul_rn(x2, A_), __dmul_rn(x1, B_)), inv_det);
-      }
-    }
+    const int fail = panel_row(x, TT, bdt, bdd, bdo, dinv, bnelim, bound);
 #pragma unroll
     for (int i = 0; i < IBMAX; ++i)
       if (i < bs) V(r, k + i) = x[i];
-    // first pivot (1x1 or 2x2 start) with an entry at or above 1/u
-    int fail = bnelim;
-#pragma unroll
-    for (int c = IBMAX - 1; c >= 0; --c) {
-      if (c >= bnelim || bdt[c] == PT_2X2B) continue;
-      const bool two = bdt[c] == PT_2X2;
-      const double x2 = c + 1 < IBMAX ? x[c + 1 < IBMAX ? c + 1 : c] : 0.0;
-      if (fabs(x[c]) >= bound || (two && fabs(x2) >= bound)) fail = c;
-    }
     if (fail < bnelim) atomicMin(&s_fail, fail);
   }
   __syncthreads();

@@ -255,18 +255,79 @@ __device__ void cta_swap(PanelView V, int64_t rows, int64_t i, int64_t j) {
   __syncthreads();
 }
 
-// W = L * D for one row of the panel (compute_ld_into, factor.rs:1536-1563)
-__device__ __forceinline__ void row_ld(const double* l, int64_t lstride, const CtaShared& sh, int nelim, double* w) {
-  int c = 0;
-  while (c < nelim) {
-    if (sh.bdt[c] == PT_1X1) { w[c] = __dmul_rn(l[c * lstride], sh.bdd[c]); c += 1; }
-    else {
-      double A_ = sh.bdd[c], B_ = sh.bdo[c], C_ = sh.bdd[c + 1];
-      double l1 = l[c * lstride], l2 = l[(c + 1) * lstride];
-      w[c] = __dadd_rn(__dmul_rn(l1, A_), __dmul_rn(l2, B_));
-      w[c + 1] = __dadd_rn(__dmul_rn(l1, B_), __dmul_rn(l2, C_));
-      c += 2;
+// The trailing update of one inner block inside a view, by the whole CTA:
+//   V(i, j) = fma(-W(i, c), L(j, c), V(i, j)), c = 0 .. n - 1 in order,
+// for ts <= j < nfsb, j <= i < bm, with W(i, c) = W[(i - ts) + c ldw] and
+// L(j, c) = V(j, k + c) (update_trailing, factor.rs:1418-1526).  A contraction,
+// so it runs on the FP64 tensor pipe (mma.sync m8n8k4, the fma chain per entry
+// in order, as in gemm64.cuh): one 32 x 32 tile per warp at a time, operands
+// straight from L1 / L2.  A tile's 8 x 16 DMMAs keep the pipe busy for ~2000
+// cycles against ~130 of loads (8 fragment loads per 16 DMMAs), so staging in
+// shared memory and the barriers it would cost buy nothing.
+__device__ void cta_trailing_update(PanelView V, int k, int ts, int bm, int nfsb, int n, const double* W, int ldw) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int fr = lane >> 2, fk = lane & 3, fc = fk * 2;
+  const int nrt = (bm - ts + 31) / 32, nct = (nfsb - ts + 31) / 32;
+  const int ld = (int)V.ld;
+  const double* L = V.a + (int64_t)k * ld;
+  int ct = 0, rt = warp;  // the warp's tile: column tile ct, the rt-th row tile from the diagonal down
+  for (;; rt += NT / 32) {
+    while (ct < nct && rt >= nrt - ct) { rt -= nrt - ct; ++ct; }
+    if (ct >= nct) break;
+    const int j0 = ts + ct * 32, i0 = ts + (ct + rt) * 32;
+    double acc[4][4][2];
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int j = j0 + ni * 8 + fc + q;
+        const double* col = V.a + (int64_t)j * ld;
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi) {
+          const int i = i0 + mi * 8 + fr;
+          acc[mi][ni][q] = (i < bm && j < nfsb && i >= j) ? col[i] : 0.0;
+        }
+      }
+    double af[2][4], bf[2][4];
+    auto load = [&](int kk, double* x, double* y) {
+      const int c = kk + fk;
+      const double* w = W + (int64_t)c * ldw - ts;
+      const double* l = L + (int64_t)c * ld;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int i = i0 + q * 8 + fr, j = j0 + q * 8 + fr;
+        x[q] = (c < n && i < bm) ? -w[i] : 0.0;
+        y[q] = (c < n && j < nfsb) ? l[j] : 0.0;
+      }
+    };
+    auto mma = [&](const double* x, const double* y) {
+#pragma unroll
+      for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni)
+          asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                       : "+d"(acc[mi][ni][0]), "+d"(acc[mi][ni][1])
+                       : "d"(x[mi]), "d"(y[ni]));
+    };
+    load(0, af[0], bf[0]);
+    for (int kk = 0; kk < n; kk += 8) {  // columns past n are zeros: they add exact zeros
+      load(kk + 4, af[1], bf[1]);
+      mma(af[0], bf[0]);
+      if (kk + 8 < n) load(kk + 8, af[0], bf[0]);
+      if (kk + 4 < n) mma(af[1], bf[1]);
     }
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int j = j0 + ni * 8 + fc + q;
+        double* col = V.a + (int64_t)j * ld;
+#pragma unroll
+        for (int mi = 0; mi < 4; ++mi) {
+          const int i = i0 + mi * 8 + fr;
+          if (i < bm && j < nfsb && i >= j) col[i] = acc[mi][ni][q];
+        }
+      }
   }
 }
 
@@ -274,33 +335,45 @@ __device__ __forceinline__ void row_ld(const double* l, int64_t lstride, const C
 // columns, NFS boundary `nfsb`), executed by the whole CTA.  D entries go to
 // VD (view-relative), the view-local column order to lp.  Returns the number
 // of eliminated columns.
-__device__ int cta_factor_inner(CtaShared& sh, PanelView V, int64_t bm, int pl, int64_t nfsb, DRec VD, int32_t* lp,
+//
+// Per 32 columns: the block (latency bound, block.cuh), the panel rows (one
+// row per thread in registers, W = L D formed while the row is there), the
+// trailing update (FP64 tensor pipe).  A 368 x 368 front took 500 us per 32
+// columns when the panel row lived in local memory (its loops had run-time
+// bounds) and the update re-read W and L from global memory for every entry.
+__device__ int cta_factor_inner(CtaShared& sh, PanelView V, int bm, int pl, int nfsb, DRec VD, int32_t* lp,
                                 double* bk, int64_t ldb, double* W, const DevOpts& o) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ib = o.ib;
+  const double bound = 1.0 / o.threshold;
   for (int i = tid; i < pl; i += NT) lp[i] = i;
   if (tid == 0) { sh.k = 0; sh.end_pos = pl; sh.n1 = 0; sh.n2 = 0; }
   __syncthreads();
   while (true) {
     int k = sh.k, end_pos = sh.end_pos;
     if (k >= end_pos) break;
-    int bs = min(end_pos - k, ib), be = k + bs;
-    int64_t rows = bm - k;
-    // 1. backup a[k..bm, k..k+bs]
-    for (int j = 0; j < bs; ++j)
-      for (int64_t i = tid; i < rows; i += NT) bk[i + j * ldb] = V(k + i, k + j);
-    // 2. load the diagonal block, factor it with the whole CTA
-    for (int t = tid; t < bs * bs; t += NT) {
-      int i = t % bs, j = t / bs;
-      if (i >= j) sh.T[i][j] = V(k + i, k + j);
+    const int bs = min(end_pos - k, ib), be = k + bs;
+    const int rows = bm - k;
+    // 1. backup a[k..bm, k..k+bs] (the panel rows are read back from it), 2. load the diagonal block
+    for (int i = tid; i < rows; i += NT) {
+      const double* src = &V(k + i, k);
+#pragma unroll
+      for (int h = 0; h < IBMAX; h += 16) {
+        double v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = (h + j < bs && (i >= bs || i >= h + j)) ? src[(int64_t)(h + j) * V.ld] : 0.0;
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (h + j < bs) {
+            bk[i + (h + j) * ldb] = v[j];
+            if (i < bs) sh.T[i][h + j] = v[j];
+          }
+      }
     }
     __syncthreads();
     cta_block_factor(sh, bs, o.small);
-    int bnelim = sh.bnelim;
-    if (bnelim == 0) {
-      for (int j = 0; j < bs; ++j)
-        for (int64_t i = tid; i < rows; i += NT) V(k + i, k + j) = bk[i + j * ldb];
-      __syncthreads();
+    const int bnelim = sh.bnelim;
+    if (bnelim == 0) {  // (the panel and the block are as they were)
       for (int off = 0; off < bs; ++off) {
         end_pos -= 1;
         if (k + off < end_pos) {
@@ -313,63 +386,56 @@ __device__ int cta_factor_inner(CtaShared& sh, PanelView V, int64_t bm, int pl, 
       __syncthreads();
       continue;
     }
-    // write the factored block back (lower triangle) and zero the D
-    // off-diagonals of 2x2 pivots (step 4) both there and in the L11 copy
-    for (int t = tid; t < bs * bs; t += NT) {
-      int i = t % bs, j = t / bs;
-      if (i >= j) V(k + i, k + j) = sh.T[i][j];
-    }
-    __syncthreads();
-    if (tid == 0) {
-      int bc = 0;
-      while (bc < bnelim) {
-        if (sh.bdt[bc] == PT_2X2) { V(k + bc + 1, k + bc) = 0.0; sh.T[bc + 1][bc] = 0.0; bc += 2; }
-        else bc += 1;
+    // the factored block back (lower triangle), the D off-diagonals of 2x2 pivots zeroed (step 4) both
+    // there and in the L11 copy of the panel's rows
+    for (int t = tid; t < IBMAX * IBMAX; t += NT) {
+      const int i = t % IBMAX, j = t / IBMAX;
+      if (i >= j && i < bs) {
+        const double v = (i == j + 1 && j < bnelim && sh.bdt[j] == PT_2X2) ? 0.0 : sh.T[i][j];
+        V(k + i, k + j) = v;
+        sh.TT[j][i] = v;
       }
-      sh.eff = bnelim;
     }
-    // 5. row permutation of view columns 0..k
-    for (int64_t c = tid; c < k; c += NT) {
-      double buf[IBMAX];
-      for (int i = 0; i < bs; ++i) buf[i] = V(k + sh.bperm[i], c);
-      for (int i = 0; i < bs; ++i) V(k + i, c) = buf[i];
+    if (tid < IBMAX) {
+      sh.dinv[tid] = pivot_inv(tid, bnelim, sh.bdt, sh.bdd, sh.bdo);
+      // 6. column order: lane i takes the entry of lane bperm[i]
+      const int32_t ob = tid < bs ? lp[k + tid] : 0;
+      const int32_t nb = __shfl_sync(0xffffffffu, ob, sh.bperm[tid] & 31);
+      if (tid < bs) lp[k + tid] = nb;
     }
-    // 6. column order
-    if (tid == 0) {
-      int32_t ob[IBMAX];
-      for (int i = 0; i < bs; ++i) ob[i] = lp[k + i];
-      for (int i = 0; i < bs; ++i) lp[k + i] = ob[sh.bperm[i]];
-    }
-    __syncthreads();
-    // 3 + 7. permute each panel row, TRSM with L11, D^-1 scaling and the
-    // threshold scan (apply_and_check, factor.rs:1295-1408)
-    const double bound = 1.0 / o.threshold;
-    for (int64_t r = be + tid; r < bm; r += NT) {
-      double x[IBMAX];
-      for (int i = 0; i < bs; ++i) x[i] = V(r, k + sh.bperm[i]);
-      for (int j = 0; j < bnelim; ++j)
-        for (int l = 0; l < j; ++l) x[j] = __fma_rn(-x[l], sh.T[j][l], x[j]);
-      int c = 0;
-      while (c < bnelim) {
-        if (sh.bdt[c] == PT_1X1) { x[c] = __dmul_rn(x[c], 1.0 / sh.bdd[c]); c += 1; }
-        else {
-          double A_ = sh.bdd[c], B_ = sh.bdo[c], C_ = sh.bdd[c + 1];
-          double inv_det = 1.0 / __dsub_rn(__dmul_rn(A_, C_), __dmul_rn(B_, B_));
-          double x1 = x[c], x2 = x[c + 1];
-          x[c] = __dmul_rn(__dsub_rn(__dmul_rn(x1, C_), __dmul_rn(x2, B_)), inv_det);
-          x[c + 1] = __dmul_rn(__dsub_rn(__dmul_rn(x2, A_), __dmul_rn(x1, B_)), inv_det);
-          c += 2;
+    if (tid == 0) sh.eff = bnelim;
+    // 5. row permutation of view columns 0..k: a warp per column
+    {
+      const int src = lane < bs ? sh.bperm[lane] : 0;
+      for (int c0 = warp; c0 < k; c0 += 4 * (NT / 32)) {
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int c = c0 + u * (NT / 32);
+          v[u] = (c < k && lane < bs) ? V(k + src, c) : 0.0;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int c = c0 + u * (NT / 32);
+          if (c < k && lane < bs) V(k + lane, c) = v[u];
         }
       }
-      for (int i = 0; i < bs; ++i) V(r, k + i) = x[i];
-      int fail = bnelim;
-      c = 0;
-      while (c < bnelim) {
-        int w = sh.bdt[c] == PT_2X2 ? 2 : 1;
-        bool bad = fabs(x[c]) >= bound || (w == 2 && fabs(x[c + 1]) >= bound);
-        if (bad) { fail = c; break; }
-        c += w;
-      }
+    }
+    __syncthreads();
+    // 3 + 7. each panel row permuted, TRSM with L11, D^-1 scaling, the threshold scan (apply_and_check,
+    // factor.rs:1295-1408), and its W = L D for the update below (the pivots that pass keep theirs)
+    const int tsz = bm - be;
+    for (int r = tid; r < tsz; r += NT) {
+      double x[IBMAX];
+      const double* src = bk + bs + r;
+#pragma unroll
+      for (int i = 0; i < IBMAX; ++i) x[i] = i < bs ? src[sh.bperm[i] * ldb] : 0.0;
+      const int fail = panel_row(x, sh.TT, sh.bdt, sh.bdd, sh.bdo, sh.dinv, bnelim, bound);
+#pragma unroll
+      for (int i = 0; i < IBMAX; ++i)
+        if (i < bs) V(be + r, k + i) = x[i];
+      panel_row_w(x, sh.bdt, sh.bdd, sh.bdo, bnelim, W + r, tsz);
       if (fail < bnelim) atomicMin(&sh.eff, fail);
     }
     __syncthreads();
@@ -380,70 +446,66 @@ __device__ int cta_factor_inner(CtaShared& sh, PanelView V, int64_t bm, int pl, 
     if (eff < bnelim) {
       for (int t = tid; t < bs * bs; t += NT) {
         int i = t % bs, j = t / bs;
-        if (i < eff || j < eff) continue;
+        if (i < eff || j < eff || i < j) continue;
         int c = sh.bperm[j], r = sh.bperm[i];
         V(k + i, k + j) = (r >= c) ? bk[r + (int64_t)c * ldb] : bk[c + (int64_t)r * ldb];
       }
       for (int j = eff; j < bs; ++j) {
         int c = sh.bperm[j];
-        for (int64_t i = bs + tid; i < rows; i += NT) V(k + i, k + j) = bk[i + (int64_t)c * ldb];
+        for (int i = bs + tid; i < rows; i += NT) V(k + i, k + j) = bk[i + (int64_t)c * ldb];
       }
+      __syncthreads();
     }
-    __syncthreads();
     const int nelim = eff;
-    const int64_t ts = be, tsz = bm - be;
     // 10. Schur updates (update_trailing factor.rs:1418-1526, update_cross_terms 1669-1766)
     if (nelim > 0) {
-      for (int64_t i = tid; i < tsz; i += NT) row_ld(&V(ts + i, k), V.ld, sh, nelim, W + i * IBMAX);
-      __syncthreads();
-      // columns are independent: no barrier between them; L[j, :] is a
-      // warp-uniform (broadcast) read
-      for (int64_t j = ts; j < nfsb; ++j) {
-        const double* lj = &V(j, k);
-        for (int64_t i = j + tid; i < bm; i += NT) {
-          const double* w = W + (i - ts) * IBMAX;
-          double acc = V(i, j);
-          for (int c = 0; c < nelim; ++c) acc = __fma_rn(-w[c], lj[c * V.ld], acc);
-          V(i, j) = acc;
-        }
-      }
-      __syncthreads();
+      cta_trailing_update(V, k, be, bm, nfsb, nelim, W, tsz);
       if (nelim < bs) {
         const int nf = bs - nelim;
-        // failed x failed, and trailing x failed; W_blk from the failed rows
+        // failed x failed: W of the failed rows formed entry by entry, in column order
         for (int t = tid; t < nf * nf; t += NT) {
           int i = t % nf, j = t / nf;
           if (i < j) continue;
-          double wb[IBMAX];
-          row_ld(&V(k + nelim + i, k), V.ld, sh, nelim, wb);
+          const double* l = &V(k + nelim + i, k);
+          const double* lj = &V(k + nelim + j, k);
           double s = 0.0;
-          for (int c = 0; c < nelim; ++c) s = __dadd_rn(s, __dmul_rn(wb[c], V(k + nelim + j, k + c)));
+          int c = 0;
+          while (c < nelim) {
+            if (sh.bdt[c] == PT_1X1) {
+              s = __dadd_rn(s, __dmul_rn(__dmul_rn(l[c * V.ld], sh.bdd[c]), lj[c * V.ld]));
+              c += 1;
+            } else {
+              const double A_ = sh.bdd[c], B_ = sh.bdo[c], C_ = sh.bdd[c + 1];
+              const double l1 = l[c * V.ld], l2 = l[(c + 1) * V.ld];
+              s = __dadd_rn(s, __dmul_rn(__dadd_rn(__dmul_rn(l1, A_), __dmul_rn(l2, B_)), lj[c * V.ld]));
+              s = __dadd_rn(s, __dmul_rn(__dadd_rn(__dmul_rn(l1, B_), __dmul_rn(l2, C_)), lj[(c + 1) * V.ld]));
+              c += 2;
+            }
+          }
           V(k + nelim + i, k + nelim + j) = __dsub_rn(V(k + nelim + i, k + nelim + j), s);
         }
+        // trailing x failed
         for (int j = 0; j < nf; ++j) {
           const double* lj = &V(k + nelim + j, k);
-          for (int64_t i = tid; i < tsz; i += NT) {
-            const double* w = W + i * IBMAX;
+          for (int i = tid; i < tsz; i += NT) {
             double s = 0.0;
-            for (int c = 0; c < nelim; ++c) s = __dadd_rn(s, __dmul_rn(w[c], lj[c * V.ld]));
-            V(ts + i, k + nelim + j) = __dsub_rn(V(ts + i, k + nelim + j), s);
+            for (int c = 0; c < nelim; ++c) s = __dadd_rn(s, __dmul_rn(W[i + (int64_t)c * tsz], lj[c * V.ld]));
+            V(be + i, k + nelim + j) = __dsub_rn(V(be + i, k + nelim + j), s);
           }
         }
-        __syncthreads();
       }
     }
-    // 11. D entries and counts for the passed columns
-    if (tid == 0) {
-      int c = 0;
-      while (c < nelim) {
-        if (sh.bdt[c] == PT_1X1) {
-          VD.type[k + c] = PT_1X1; VD.diag[k + c] = sh.bdd[c]; VD.off[k + c] = 0.0; sh.n1++; c += 1;
-        } else if (c + 1 < nelim) {
-          VD.type[k + c] = PT_2X2; VD.type[k + c + 1] = PT_2X2B;
-          VD.diag[k + c] = sh.bdd[c]; VD.diag[k + c + 1] = sh.bdd[c + 1];
-          VD.off[k + c] = sh.bdo[c]; VD.off[k + c + 1] = 0.0; sh.n2++; c += 2;
-        } else c += 1;
+    // 11. D entries and counts for the passed columns (the adjusted nelim never splits a 2x2)
+    if (tid < 32) {
+      const int8_t t = lane < nelim ? sh.bdt[lane] : (int8_t)PT_DELAYED;
+      if (t != PT_DELAYED) {
+        VD.type[k + lane] = t;
+        VD.diag[k + lane] = sh.bdd[lane];
+        VD.off[k + lane] = t == PT_2X2 ? sh.bdo[lane] : 0.0;
       }
+      const int c1 = __popc(__ballot_sync(0xffffffffu, t == PT_1X1));
+      const int c2 = __popc(__ballot_sync(0xffffffffu, t == PT_2X2));
+      if (lane == 0) { sh.n1 += c1; sh.n2 += c2; }
     }
     __syncthreads();
     // 12. delay the failed columns to end_pos
@@ -486,7 +548,7 @@ __device__ __forceinline__ void cta_aptp_front(CtaShared& sh, int* tpp_cnt, int 
   int n1 = 0, n2 = 0;
   int gne = 0;
   if (p <= o.nb) {
-    gne = cta_factor_inner(sh, Av, m, p, p, D, lp, bk, m, W, o);
+    gne = cta_factor_inner(sh, Av, (int)m, p, p, D, lp, bk, m, W, o);
     n1 = sh.n1; n2 = sh.n2;
     for (int i = tid; i < p; i += NT) perm[i] = lp[i];
     __syncthreads();
@@ -497,7 +559,7 @@ __device__ __forceinline__ void cta_aptp_front(CtaShared& sh, int* tpp_cnt, int 
       int cs = gne, bcols = min(rem, o.nb);
       PanelView V{&Av(cs, cs), m};
       DRec VD{D.type + cs, D.diag + cs, D.off + cs};
-      int bne = cta_factor_inner(sh, V, m - cs, bcols, (int64_t)p - cs, VD, lp, bk, m, W, o);
+      int bne = cta_factor_inner(sh, V, (int)m - cs, bcols, p - cs, VD, lp, bk, m, W, o);
       n1 += sh.n1; n2 += sh.n2;
       // propagate the row permutation to columns 0..cs
       if (cs > 0) {
@@ -568,8 +630,9 @@ __global__ void __launch_bounds__(NT) k_aptp(const int32_t* ids, int n, DFront* 
 // next front from a work queue (*next, zero at launch) until the list is
 // done.  The host lists the fronts largest first, so the long ones start
 // early and the short ones fill in behind them.  Which CTA factors a front
-// changes nothing in its result.  
-__global__ void __launch_bounds__(NT) k_front_queue(const int32_t* ids, int na, int32_t* next, DFront* F, Arenas A,
+// changes nothing in its result.  Two CTAs per SM: one's block and panel
+// latency runs under the other's tensor-pipe update.
+__global__ void __launch_bounds__(NT, 2) k_front_queue(const int32_t* ids, int na, int32_t* next, DFront* F, Arenas A,
                                                        DevOpts o) {
   __shared__ CtaShared sh;
   __shared__ int tpp_cnt[2];

@@ -49,6 +49,7 @@ struct CtaShared {
   int bnelim, eff, n1, n2, end_pos, k;
   int tmpi;
   double dinv[IBMAX];
+  unsigned two;  // bit c: a 2x2 pivot starts at c
   alignas(16) double TT[IBMAX][IBMAX + 2];  // the factored block transposed: TT[l][j] = L(j, l) (panel_rows)
   // cta_block_factor only
   double Tb[IBMAX][IBMAX + 1];  // the other buffer of the trailing block
@@ -250,55 +251,64 @@ __device__ __forceinline__ double pivot_inv(int c, int n, const int8_t* bdt, con
 // but the n - l updates of a step are independent (the loop over j first is
 // one dependent chain of n (n - 1) / 2 multiply-adds).  TT holds L11 by
 // columns, so the inner loop reads two entries per shared-memory load.
-// Returns the first pivot (1x1 or 2x2 start) with an entry at or above bound.
-__device__ __forceinline__ int panel_row(double (&x)[IBMAX], const double (*TT)[IBMAX + 2], const int8_t* bdt,
-                                         const double* bdd, const double* bdo, const double* dinv, int n,
-                                         double bound) {
+// two: bit c set where a 2x2 pivot starts (a mask in a register: a type read
+// from shared memory would put a load before every column's branch).  Returns
+// the first pivot (1x1 or 2x2 start) with an entry at or above bound.
+// FULL: n = 32, the usual block: no column is tested against n.
+template <bool FULL>
+__device__ __forceinline__ int panel_row_t(double (&x)[IBMAX], const double (*TT)[IBMAX + 2], unsigned two,
+                                           const double* bdd, const double* bdo, const double* dinv, int n,
+                                           double bound) {
 #pragma unroll
   for (int l = 0; l + 1 < IBMAX; ++l) {
-    if (l + 1 >= n) break;
+    if (!FULL && l + 1 >= n) break;
     const double nx = -x[l];
 #pragma unroll
     for (int j = (l + 1) & ~1; j < IBMAX; j += 2) {
       const double2 t = *reinterpret_cast<const double2*>(&TT[l][j]);
-      if (j > l && j < n) x[j] = __fma_rn(nx, t.x, x[j]);
-      if (j + 1 < n) x[j + 1] = __fma_rn(nx, t.y, x[j + 1]);
+      if (j > l && (FULL || j < n)) x[j] = __fma_rn(nx, t.x, x[j]);
+      if (FULL || j + 1 < n) x[j + 1] = __fma_rn(nx, t.y, x[j + 1]);
     }
   }
-  int fail = n;
+  unsigned bad = 0;
 #pragma unroll
   for (int c = 0; c < IBMAX; ++c) {
-    if (c >= n) continue;
-    bool bad = false;
-    if (bdt[c] == PT_1X1) {
-      x[c] = __dmul_rn(x[c], dinv[c]);
-      bad = fabs(x[c]) >= bound;
-    } else if (bdt[c] == PT_2X2 && c + 1 < IBMAX) {
-      const double A_ = bdd[c], B_ = bdo[c], C_ = bdd[c + 1], inv_det = dinv[c];
-      const int d = c + 1 < IBMAX ? c + 1 : c;
+    if ((!FULL && c >= n) || (c > 0 && (two >> (c - 1)) & 1)) continue;  // (a second column goes with its first)
+    const int d = c + 1 < IBMAX ? c + 1 : c;
+    if ((two >> c) & 1) {
+      const double A_ = bdd[c], B_ = bdo[c], C_ = bdd[d], inv_det = dinv[c];
       const double x1 = x[c], x2 = x[d];
       x[c] = __dmul_rn(__dsub_rn(__dmul_rn(x1, C_), __dmul_rn(x2, B_)), inv_det);
       x[d] = __dmul_rn(__dsub_rn(__dmul_rn(x2, A_), __dmul_rn(x1, B_)), inv_det);
-      bad = fabs(x[c]) >= bound || fabs(x[d]) >= bound;
+      if (fabs(x[c]) >= bound || fabs(x[d]) >= bound) bad |= 1u << c;
+    } else {
+      x[c] = __dmul_rn(x[c], dinv[c]);
+      if (fabs(x[c]) >= bound) bad |= 1u << c;
     }
-    if (bad && c < fail) fail = c;
   }
-  return fail;
+  return bad ? __ffs(bad) - 1 : n;
+}
+__device__ __forceinline__ int panel_row(double (&x)[IBMAX], const double (*TT)[IBMAX + 2], unsigned two,
+                                         const double* bdd, const double* bdo, const double* dinv, int n,
+                                         double bound) {
+  return n == IBMAX ? panel_row_t<true>(x, TT, two, bdd, bdo, dinv, n, bound)
+                    : panel_row_t<false>(x, TT, two, bdd, bdo, dinv, n, bound);
 }
 
-// W = L D of the row (compute_ld_into, factor.rs:1536-1563), column c to
-// w[c * ldw], for the n columns of x.
-__device__ __forceinline__ void panel_row_w(const double (&x)[IBMAX], const int8_t* bdt, const double* bdd,
-                                            const double* bdo, int n, double* w, int64_t ldw) {
+// The row's W = L D (compute_ld_into, factor.rs:1536-1563) in place of x, for
+// its first n columns.
+__device__ __forceinline__ void panel_row_w(double (&x)[IBMAX], unsigned two, const double* bdd, const double* bdo,
+                                            int n) {
 #pragma unroll
   for (int c = 0; c < IBMAX; ++c) {
-    if (c >= n) continue;
-    if (bdt[c] == PT_1X1) {
-      w[c * ldw] = __dmul_rn(x[c], bdd[c]);
-    } else if (bdt[c] == PT_2X2 && c + 1 < IBMAX) {
-      const int d = c + 1 < IBMAX ? c + 1 : c;
-      w[c * ldw] = __dadd_rn(__dmul_rn(x[c], bdd[c]), __dmul_rn(x[d], bdo[c]));
-      w[d * ldw] = __dadd_rn(__dmul_rn(x[c], bdo[c]), __dmul_rn(x[d], bdd[d]));
+    if (c >= n || (c > 0 && (two >> (c - 1)) & 1)) continue;
+    const int d = c + 1 < IBMAX ? c + 1 : c;
+    if ((two >> c) & 1) {
+      const double l1 = x[c], l2 = x[d];
+      x[c] = __dadd_rn(__dmul_rn(l1, bdd[c]), __dmul_rn(l2, bdo[c]));
+      x[d] = __dadd_rn(__dmul_rn(l1, bdo[c]), __dmul_rn(l2, bdd[d]));
+    } else {
+      x[c] = __dmul_rn(x[c], bdd[c]);
     }
   }
 }

@@ -4,26 +4,30 @@
 // row-parallel step spread over the whole GPU and the pivot state kept on the
 // device, so the host issues a fixed launch sequence:
 //
-//   per 32-column inner block (view-local position k):
-//     lf_block   1 CTA    the previous inner block's delayed columns to the
-//                         end of the outer block (lf_delay_cta), complete
-//                         pivoting on the diagonal block, row permutation of
-//                         the outer block's earlier columns
-//     lf_panel   grid     backup, column permutation, TRSM, D^-1 scaling and
-//                         the a-posteriori threshold scan of every panel row
-//     lf_wi      grid     CTA 0 first (lf_post_cta): 2x2 boundary adjustment,
-//                         restore of the failed part of the diagonal block,
-//                         failed x failed cross term, D entries; then every
-//                         CTA: restore of the failed panel columns, W = L D,
-//                         the trailing x failed cross term
-//     k_syrk_dmma         rank-nelim update of the outer block's trailing
-//                         columns (region start read from the device)
-//   after the last inner block:
-//     lf_delay   1 CTA    its delayed columns to the end of the outer block
+//   per 256-column outer block, first:
+//     lf_begin   1 CTA    checks the block's start column, then complete
+//                         pivoting on its first 32-column diagonal block
+//   per 32-column inner block (view-local position k), two launches:
+//     lf_panel   grid     backup, column permutation, TRSM, D^-1 scaling,
+//                         W = L D and the a-posteriori threshold scan of every
+//                         panel row; the block's row permutation of the outer
+//                         block's earlier columns
+//     lf_update  grid     CTA 0: the NEXT inner block's 32 x 32 diagonal block
+//                         takes this block's update and is factored at once,
+//                         then this block's D entries; the other CTAs: the
+//                         rank-32 update of the outer block's trailing columns
+//                         on the FP64 tensor pipe.  The block is 32 dependent
+//                         pivot steps on one SM, so it runs beside the update
+//                         instead of after it.  When columns failed their
+//                         threshold test, nothing is known of the next block
+//                         yet: CTA 0 does the post-processing, the others also
+//                         restore the failed panel columns and form their
+//                         cross term, and the CTA that finishes last moves the
+//                         delayed columns and factors the next block.
 //   per 256-column outer block:
 //     lf_prop    grid     row permutation of the front's earlier columns
-//     lf_w       grid     W = L D for the rows below the outer block, into
-//                         the window of pending columns
+//                         (W of the rows below the outer block is in the window
+//                         of pending columns already: lf_panel wrote it)
 //     Schur GEMM          the deferred update (update_trailing), split in
 //                         two: the next outer block's columns take every
 //                         pending column at once (near field); the columns
@@ -45,18 +49,26 @@
 
 namespace rvg {
 
+// one inner block: its position, width, pivots found and eliminated, and the
+// factored block
+struct LFBlk {
+  int32_t k, bs, bnelim, eff;
+  uint32_t two;       // bit c: a 2x2 pivot starts at c
+  int32_t bperm[32];
+  int8_t bdt[32];
+  double bdd[32], bdo[32], dinv[32];  // dinv: what the rows' D^-1 step multiplies by (pivot_inv)
+  double T[32][33];   // factored block, 2x2 off-diagonals zeroed (the L11 of the TRSM)
+  double Tb[32][33];  // the block before factorization
+};
+
 struct LFState {
-  int32_t k, end_pos, bs, bnelim, eff, nelim;
-  int32_t gne, n1, n2, bne;
+  int32_t end_pos, gne, n1, n2, bne;
   // set when an outer block was launched for another start column than the
   // device reached (the host issues blocks ahead assuming no delays): every
   // later launch of the front returns at once until the host clears it
   int32_t spec_bad;
-  int32_t bperm[32];
-  int8_t bdt[32];
-  double bdd[32], bdo[32];
-  double T[32][33];   // factored block, 2x2 off-diagonals zeroed (the L11 of the TRSM)
-  double Tb[32][33];  // the block before factorization
+  int32_t done;  // CTAs of a k_lf_update with failed columns that have finished
+  LFBlk b[2];    // inner block i is b[i & 1]: the update of block i factors block i + 1
 };
 
 struct LFArgs {
@@ -71,17 +83,105 @@ struct LFArgs {
   double* wo;       // pending W (column-major, ld wld): row i, pending column c at wo[(i - wrow0) + c * wld]
   int64_t wld, wrow0, wcol0;  // leading dimension, first row, this block's first pending column
   int64_t cs, bcols, nfsb;  // outer block start, width, NFS boundary (global p)
+  int par;          // which of the state's two blocks is the current inner block
+  int win;          // the rows below the outer block keep their W (the outer block joins the window)
   DevOpts o;
 };
 
 __global__ void k_lf_init(LFState* st, int32_t* perm, int64_t p) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) { st->gne = 0; st->n1 = 0; st->n2 = 0; st->spec_bad = 0; }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->gne = 0; st->n1 = 0; st->n2 = 0; st->spec_bad = 0; st->done = 0;
+  }
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < p; i += (int64_t)gridDim.x * blockDim.x)
     perm[i] = (int32_t)i;
 }
 
-__global__ void k_lf_begin_outer(LFArgs A) {
+// Complete pivoting on the diagonal block at view position k, into the state's
+// block q (1 CTA).  n > 0: the n columns from position upd on (the block before,
+// all of whose columns passed) are still to be applied: the entries first take
+// that update, one fma chain per entry in column order, as the tensor-pipe
+// tiles give the rest of the trailing columns.
+__device__ void lf_block_cta(const LFArgs& A, CtaShared& sh, int q, int k, int end_pos, int upd, int n) {
+  LFBlk& B = A.st->b[q];
+  const int tid = threadIdx.x;
+  PanelView V{A.a + A.cs + A.cs * A.m, A.m};
+  const int bs = min(end_pos - k, A.o.ib);
+  if (k >= end_pos) {  // no columns left in this outer block
+    if (tid == 0) { B.k = k; B.bs = 0; B.bnelim = 0; B.eff = 0; B.two = 0; }
+    return;
+  }
+  // 4 entries per thread, every load before the first store
+  constexpr int PER = IBMAX * IBMAX / NT;
+  const int i = tid % IBMAX, j0 = tid / IBMAX;
+  double v[PER];
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int j = j0 + u * (NT / IBMAX);
+    v[u] = (i < bs && j < bs && i >= j) ? V(k + i, k + j) : 0.0;
+  }
+  if (n > 0) {
+    const int64_t bm = A.m - A.cs;
+    double wv[PER], lv[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int c = j0 + u * (NT / IBMAX);
+      const bool in = i < bs && c < n;
+      wv[u] = in ? A.w[(k + i) + c * bm] : 0.0;
+      lv[u] = in ? V(k + i, upd + c) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int c = j0 + u * (NT / IBMAX);
+      sh.Tb[i][c] = wv[u];
+      sh.Lc[i][c] = lv[u];
+    }
+    __syncthreads();
+    for (int c = 0; c < n; ++c) {
+      const double w = -sh.Tb[i][c];
+#pragma unroll
+      for (int u = 0; u < PER; ++u) v[u] = __fma_rn(w, sh.Lc[j0 + u * (NT / IBMAX)][c], v[u]);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int j = j0 + u * (NT / IBMAX);
+    if (i < bs && j < bs && i >= j) { sh.T[i][j] = v[u]; B.Tb[i][j] = v[u]; }
+  }
+  __syncthreads();
+  cta_block_factor(sh, bs, A.o.small);
+  const int bnelim = sh.bnelim;
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int j = j0 + u * (NT / IBMAX);
+    if (i < bs && j < bs && i >= j) {
+      // (the D off-diagonal of a 2x2 pivot is zeroed in L; where no pivot was found the panel stays as it is)
+      const double t = (i == j + 1 && j < bnelim && sh.bdt[j] == PT_2X2) ? 0.0 : sh.T[i][j];
+      if (bnelim > 0) V(k + i, k + j) = t;
+      else if (n > 0) V(k + i, k + j) = v[u];
+      B.T[i][j] = t;
+    }
+  }
+  // (the row permutation of the view columns 0..k, step 5, is done by k_lf_panel's threads c < k)
+  if (tid < 32) {
+    if (bnelim > 0) {  // column order (step 6): lane i takes the entry of lane bperm[i]
+      const int32_t ob = tid < bs ? A.lp[k + tid] : 0;
+      const int32_t nbv = __shfl_sync(0xffffffffu, ob, sh.bperm[tid] & 31);
+      if (tid < bs) A.lp[k + tid] = nbv;
+    }
+    B.bperm[tid] = sh.bperm[tid];
+    B.bdt[tid] = sh.bdt[tid];
+    B.bdd[tid] = sh.bdd[tid];
+    B.bdo[tid] = sh.bdo[tid];
+    B.dinv[tid] = pivot_inv(tid, bnelim, sh.bdt, sh.bdd, sh.bdo);
+    const unsigned two = __ballot_sync(0xffffffffu, tid < bnelim && sh.bdt[tid] == PT_2X2);
+    if (tid == 0) { B.k = k; B.bs = bs; B.bnelim = bnelim; B.eff = bnelim; B.two = two; }
+  }
+}
+
+// Start of an outer block and its first inner block (1 CTA).
+__global__ void __launch_bounds__(NT) k_lf_begin_outer(LFArgs A) {
   chain_enter();
+  __shared__ CtaShared sh;
   LFState* st = A.st;
   if (st->spec_bad) return;
   if (st->gne != (int32_t)A.cs) {  // issued for a start column the factorization did not reach
@@ -89,156 +189,45 @@ __global__ void k_lf_begin_outer(LFArgs A) {
     if (threadIdx.x == 0) st->spec_bad = 1;
     return;
   }
-  if (threadIdx.x == 0) { st->k = 0; st->end_pos = (int32_t)A.bcols; st->bne = 0; }
+  if (threadIdx.x == 0) { st->end_pos = (int32_t)A.bcols; st->bne = 0; }
   for (int i = threadIdx.x; i < A.bcols; i += blockDim.x) A.lp[i] = i;
-}
-
-__device__ void lf_delay_cta(const LFArgs& A);
-
-// complete pivoting on the diagonal block (1 CTA); with after_delay set it
-// first moves the previous inner block's delayed columns to the end of the
-// outer block (lf_delay_cta, that block's last step)
-__global__ void __launch_bounds__(NT) k_lf_block(LFArgs A, int after_delay) {
-  chain_enter();
-  if (A.st->spec_bad) return;  // a block issued past a mispredicted start column
-  if (after_delay) {
-    lf_delay_cta(A);
-    __syncthreads();
-  }
-  __shared__ CtaShared sh;
-  LFState* st = A.st;
-  const int tid = threadIdx.x;
-  const int64_t cs = A.cs;
-  PanelView V{A.a + cs + cs * A.m, A.m};
-  const int k = st->k, end_pos = st->end_pos;
-  const int bs = min(end_pos - k, A.o.ib);
-  if (k >= end_pos) {  // no columns left in this outer block
-    if (tid == 0) { st->bs = 0; st->bnelim = 0; st->eff = 0; st->nelim = 0; }
-    return;
-  }
-  {
-    // the block's loads before any global store (4 per thread)
-    constexpr int PER = IBMAX * IBMAX / NT;
-    double v[PER];
-#pragma unroll
-    for (int u = 0; u < PER; ++u) {
-      const int t = tid + u * NT, i = t % IBMAX, j = t / IBMAX;
-      v[u] = (i < bs && j < bs && i >= j) ? V(k + i, k + j) : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < PER; ++u) {
-      const int t = tid + u * NT, i = t % IBMAX, j = t / IBMAX;
-      if (i < bs && j < bs && i >= j) { sh.T[i][j] = v[u]; st->Tb[i][j] = v[u]; }
-    }
-  }
   __syncthreads();
-  cta_block_factor(sh, bs, A.o.small);
-  const int bnelim = sh.bnelim;
-  if (bnelim > 0) {
-    for (int t = tid; t < bs * bs; t += NT) {
-      int i = t % bs, j = t / bs;
-      if (i >= j) V(k + i, k + j) = sh.T[i][j];
-    }
-    __syncthreads();
-    if (tid == 0) {
-      int bc = 0;
-      while (bc < bnelim) {
-        if (sh.bdt[bc] == PT_2X2) { V(k + bc + 1, k + bc) = 0.0; sh.T[bc + 1][bc] = 0.0; bc += 2; }
-        else bc += 1;
-      }
-    }
-    // (the row permutation of the view columns 0..k, step 5, is done by k_lf_panel's threads c < k)
-    if (tid < 32) {  // column order (step 6): lane i takes the entry of lane bperm[i]
-      const int32_t ob = tid < bs ? A.lp[k + tid] : 0;
-      const int32_t nbv = __shfl_sync(0xffffffffu, ob, sh.bperm[tid] & 31);
-      if (tid < bs) A.lp[k + tid] = nbv;
-    }
-    __syncthreads();
-  }
-  for (int t = tid; t < bs * bs; t += NT) {
-    int i = t % bs, j = t / bs;
-    if (i >= j) st->T[i][j] = sh.T[i][j];
-  }
-  if (tid < 32) {
-    st->bperm[tid] = sh.bperm[tid];
-    st->bdt[tid] = sh.bdt[tid];
-    st->bdd[tid] = sh.bdd[tid];
-    st->bdo[tid] = sh.bdo[tid];
-  }
-  if (tid == 0) { st->bs = bs; st->bnelim = bnelim; st->eff = bnelim; }
+  lf_block_cta(A, sh, 0, 0, (int)A.bcols, 0, 0);
 }
 
-// One row of W = L D over pivots [0, n) (l(c) = l[c * ld]; D given by type,
-// diagonal and off-diagonal; the second column of a 2x2 is written with its
-// first), 16 columns at a time: the chunk's L and D values are loaded before
-// any W store, so the row's memory latency is not paid per column.
-__device__ __forceinline__ void lf_w_row(const double* l, int64_t ld, int n, const int8_t* dt, const double* dd,
-                                         const double* dof, double* w, int64_t wld) {
-  for (int c0 = 0; c0 < n; c0 += 16) {
-    double lv[17], dv[17], ov[16];
-    int8_t tv[16];
-#pragma unroll
-    for (int u = 0; u < 17; ++u) {
-      const bool in = c0 + u < n;
-      lv[u] = in ? l[(int64_t)(c0 + u) * ld] : 0.0;
-      dv[u] = in ? dd[c0 + u] : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const bool in = c0 + u < n;
-      ov[u] = in ? dof[c0 + u] : 0.0;
-      tv[u] = in ? dt[c0 + u] : (int8_t)PT_DELAYED;
-    }
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const int64_t c = c0 + u;
-      if (tv[u] == PT_1X1) {
-        w[c * wld] = __dmul_rn(lv[u], dv[u]);
-      } else if (tv[u] == PT_2X2) {
-        w[c * wld] = __dadd_rn(__dmul_rn(lv[u], dv[u]), __dmul_rn(lv[u + 1], ov[u]));
-        w[(c + 1) * wld] = __dadd_rn(__dmul_rn(lv[u], ov[u]), __dmul_rn(lv[u + 1], dv[u + 1]));
-      }
-    }
-  }
-}
-
-// panel rows: backup, permute, TRSM, D^-1, threshold scan (grid over rows,
-// one row per thread, the row's 32 values in registers: every index into
-// them is a compile-time constant)
+// panel rows: backup, permute, TRSM, D^-1, threshold scan, W = L D (grid over
+// rows, one row per thread, the row's 32 values in registers: every index into
+// them is a compile-time constant).  W is formed for every pivot the block
+// found, before the scan's result over all rows is known: the pivots that pass
+// are a prefix, and the columns after them are written again by later blocks.
+// Rows below the outer block also leave it in the window of pending columns.
 constexpr int LF_PANEL_T = 64;
 __global__ void __launch_bounds__(LF_PANEL_T) k_lf_panel(LFArgs A) {
   chain_enter();
-  if (A.st->spec_bad) return;  // a block issued past a mispredicted start column
-  LFState* st = A.st;
-  const int bnelim = st->bnelim;
-  if (bnelim == 0) return;
   __shared__ alignas(16) double TT[IBMAX][IBMAX + 2];  // TT[l][j] = L11(j, l)
   __shared__ int bperm[IBMAX];
-  __shared__ int8_t bdt[IBMAX];
   __shared__ double bdd[IBMAX], bdo[IBMAX], dinv[IBMAX];
   __shared__ int s_fail;
-  const int bs = st->bs, k = st->k;
+  // everything the state holds of the block in one round trip
+  LFBlk* b = &A.st->b[A.par];
+  const int spec_bad = A.st->spec_bad, bnelim = b->bnelim, bs = b->bs, k = b->k;
+  const unsigned two = b->two;
   {
-    // the factored block: thread t takes column t / 2 (rows of one half), all loads before the stores
+    // the factored block: thread t takes column t / 2 (rows of one half); entries past the block's width
+    // are whatever an earlier block left and are never used
     const int j = threadIdx.x >> 1, h = threadIdx.x & 1;
     double v[16];
 #pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const int i = h * 16 + u;
-      v[u] = (j < bs && i < bs && i >= j) ? st->T[i][j] : 0.0;
-    }
+    for (int u = 0; u < 16; ++u) v[u] = b->T[h * 16 + u][j];
+    const int c = threadIdx.x & 31;
+    const int pc = b->bperm[c];
+    const double d0 = b->bdd[c], d1 = b->bdo[c], d2 = b->dinv[c];
+    if (spec_bad || bnelim == 0) return;  // a block issued past a mispredicted start column; nothing found
 #pragma unroll
     for (int u = 0; u < 16; ++u) TT[j][h * 16 + u] = v[u];
+    if (threadIdx.x < IBMAX) { bperm[c] = pc; bdd[c] = d0; bdo[c] = d1; dinv[c] = d2; }
+    if (threadIdx.x == 0) s_fail = bnelim;
   }
-  if (threadIdx.x < IBMAX) {
-    const int c = threadIdx.x;
-    bperm[c] = st->bperm[c];
-    bdt[c] = st->bdt[c];
-    bdd[c] = st->bdd[c];
-    bdo[c] = st->bdo[c];
-    dinv[c] = pivot_inv(c, bnelim, st->bdt, st->bdd, st->bdo);
-  }
-  if (threadIdx.x == 0) s_fail = bnelim;
   __syncthreads();
   const int64_t bm = A.m - A.cs;
   PanelView V{A.a + A.cs + A.cs * A.m, A.m};
@@ -260,50 +249,52 @@ __global__ void __launch_bounds__(LF_PANEL_T) k_lf_panel(LFArgs A) {
     // every load of the row before the first store: the backup may alias the
     // panel as far as the compiler knows, so a load placed after a store
     // would wait for it (one memory round trip per column)
-    double raw[IBMAX], x[IBMAX];
-#pragma unroll
-    for (int i = 0; i < IBMAX; ++i) raw[i] = i < bs ? V(r, k + i) : 0.0;
+    double x[IBMAX];
 #pragma unroll
     for (int i = 0; i < IBMAX; ++i) x[i] = i < bs ? V(r, k + bperm[i]) : 0.0;
+    double* pb = A.pb + r;  // the backup, in the block's column order
 #pragma unroll
     for (int i = 0; i < IBMAX; ++i)
-      if (i < bs) A.pb[r + (int64_t)i * bm] = raw[i];
-    const int fail = panel_row(x, TT, bdt, bdd, bdo, dinv, bnelim, bound);
+      if (i < bs) pb[i * bm] = x[i];
+    const int fail = panel_row(x, TT, two, bdd, bdo, dinv, bnelim, bound);
+    double* l = &V(r, k);
 #pragma unroll
     for (int i = 0; i < IBMAX; ++i)
-      if (i < bs) V(r, k + i) = x[i];
+      if (i < bs) l[i * A.m] = x[i];
+    panel_row_w(x, two, bdd, bdo, bnelim);
+    double* w = A.w + r;
+#pragma unroll
+    for (int i = 0; i < IBMAX; ++i)
+      if (i < bnelim) w[i * bm] = x[i];
+    if (A.win && r >= A.bcols) {
+      w = A.wo + (A.cs + r - A.wrow0) + (A.wcol0 + k) * A.wld;
+#pragma unroll
+      for (int i = 0; i < IBMAX; ++i)
+        if (i < bnelim) w[i * A.wld] = x[i];
+    }
     if (fail < bnelim) atomicMin(&s_fail, fail);
   }
   __syncthreads();
-  if (threadIdx.x == 0 && s_fail < bnelim) atomicMin(&st->eff, s_fail);
+  if (threadIdx.x == 0 && s_fail < bnelim) atomicMin(&b->eff, s_fail);
 }
 
-// 2x2 boundary, restore of the failed diagonal part, failed x failed term,
-// D entries: one CTA of 256 threads (CTA 0 of k_lf_wi, before its rows).  It
-// writes only the block's own rows, the D entries and the counters; the
-// adjusted eliminated count it stores in st->eff / st->nelim is the one every
-// CTA of k_lf_wi derives from st->eff itself (the adjustment is idempotent).
-__device__ __forceinline__ void lf_post_cta(const LFArgs& A) {
+// Restore of the failed diagonal part, failed x failed term, D entries of
+// block b, of whose pivots the first nelim passed: one CTA.  It writes only the
+// block's own rows, the D entries and the counters.
+__device__ __forceinline__ void lf_post_cta(const LFArgs& A, const LFBlk* b, int nelim) {
   LFState* st = A.st;
-  const int bnelim = st->bnelim, bs = st->bs, k = st->k;
+  const int bs = b->bs, k = b->k;
   const int tid = threadIdx.x;
-  if (bnelim == 0) {
-    if (tid == 0) st->nelim = 0;
-    return;
-  }
-  int eff = st->eff;
-  if (eff > 0 && st->bdt[eff - 1] == PT_2X2) eff -= 1;
   PanelView V{A.a + A.cs + A.cs * A.m, A.m};
-  if (eff < bnelim) {
+  if (nelim < b->bnelim) {
     for (int t = tid; t < bs * bs; t += blockDim.x) {
       int i = t % bs, j = t / bs;
-      if (i < eff || j < eff) continue;
-      int c = st->bperm[j], r = st->bperm[i];
-      V(k + i, k + j) = r >= c ? st->Tb[r][c] : st->Tb[c][r];
+      if (i < nelim || j < nelim || i < j) continue;
+      int c = b->bperm[j], r = b->bperm[i];
+      V(k + i, k + j) = r >= c ? b->Tb[r][c] : b->Tb[c][r];
     }
+    __syncthreads();
   }
-  __syncthreads();
-  const int nelim = eff;
   if (nelim > 0 && nelim < bs) {
     const int nf = bs - nelim;
     for (int t = tid; t < nf * nf; t += blockDim.x) {
@@ -316,11 +307,11 @@ __device__ __forceinline__ void lf_post_cta(const LFArgs& A) {
       double s = 0.0;
       int c = 0;
       while (c < nelim) {
-        if (st->bdt[c] == PT_1X1) {
-          s = __dadd_rn(s, __dmul_rn(__dmul_rn(l[c * A.m], st->bdd[c]), lj[c * A.m]));
+        if (b->bdt[c] == PT_1X1) {
+          s = __dadd_rn(s, __dmul_rn(__dmul_rn(l[c * A.m], b->bdd[c]), lj[c * A.m]));
           c += 1;
         } else {
-          const double A_ = st->bdd[c], B_ = st->bdo[c], C_ = st->bdd[c + 1];
+          const double A_ = b->bdd[c], B_ = b->bdo[c], C_ = b->bdd[c + 1];
           const double l1 = l[c * A.m], l2 = l[(c + 1) * A.m];
           const double w0 = __dadd_rn(__dmul_rn(l1, A_), __dmul_rn(l2, B_));
           const double w1 = __dadd_rn(__dmul_rn(l1, B_), __dmul_rn(l2, C_));
@@ -336,93 +327,28 @@ __device__ __forceinline__ void lf_post_cta(const LFArgs& A) {
     // D entries, one pivot column per lane (the adjusted nelim never splits a 2x2)
     DRec VD{A.D.type + A.cs, A.D.diag + A.cs, A.D.off + A.cs};
     const int c = tid;
-    const int8_t t = c < nelim ? st->bdt[c] : (int8_t)PT_DELAYED;
-    const bool one = t == PT_1X1;
-    const bool first = t == PT_2X2 && c + 1 < nelim;
-    const bool second = t == PT_2X2B;
-    if (one || first || second) {
-      VD.type[k + c] = one ? PT_1X1 : (first ? PT_2X2 : PT_2X2B);
-      VD.diag[k + c] = st->bdd[c];
-      VD.off[k + c] = first ? st->bdo[c] : 0.0;
+    const int8_t t = c < nelim ? b->bdt[c] : (int8_t)PT_DELAYED;
+    if (t != PT_DELAYED) {
+      VD.type[k + c] = t;
+      VD.diag[k + c] = b->bdd[c];
+      VD.off[k + c] = t == PT_2X2 ? b->bdo[c] : 0.0;
     }
-    const int n1 = __popc(__ballot_sync(0xffffffffu, one));
-    const int n2 = __popc(__ballot_sync(0xffffffffu, first));
-    if (tid == 0) {
-      st->n1 += n1; st->n2 += n2;
-      st->nelim = nelim;
-      st->eff = eff;
-    }
+    const int n1 = __popc(__ballot_sync(0xffffffffu, t == PT_1X1));
+    const int n2 = __popc(__ballot_sync(0xffffffffu, t == PT_2X2));
+    if (tid == 0) { st->n1 += n1; st->n2 += n2; }
   }
 }
 
-// Rows below the inner block (one thread per row): restore of the failed
-// panel columns from the backup, W = L D over the eliminated columns
-// (column-major, ld = rows of the view, indexed by absolute row) and the
-// trailing x failed cross term.  The rank-nelim update of the outer block's
-// trailing columns that follows is the DMMA GEMM (k_syrk_dmma with the
-// region start read from the device), the same fma chain per entry.
-__global__ void __launch_bounds__(256) k_lf_wi(LFArgs A) {
-  chain_enter();
-  if (A.st->spec_bad) return;  // a block issued past a mispredicted start column
-  LFState* st = A.st;
-  const int bnelim = st->bnelim;
-  if (bnelim > 0) {
-    const int bs = st->bs, k = st->k;
-    // the eliminated count: the panel's first failing column, one less where it would split a 2x2 (the
-    // value CTA 0 stores below)
-    int eff = st->eff;
-    if (eff > 0 && st->bdt[eff - 1] == PT_2X2) eff -= 1;
-    const int nelim = eff;
-    const int64_t bm = A.m - A.cs;
-    const int64_t ts = k + bs;
-    const int nf = bs - nelim;
-    __shared__ double Ls[IBMAX][IBMAX + 1];
-    __shared__ int bperm[IBMAX];
-    __shared__ int8_t bdt[IBMAX];
-    __shared__ double bdd[IBMAX], bdo[IBMAX];
-    PanelView V{A.a + A.cs + A.cs * A.m, A.m};
-    if (threadIdx.x < IBMAX) {
-      bperm[threadIdx.x] = st->bperm[threadIdx.x];
-      bdt[threadIdx.x] = st->bdt[threadIdx.x];
-      bdd[threadIdx.x] = st->bdd[threadIdx.x];
-      bdo[threadIdx.x] = st->bdo[threadIdx.x];
-    }
-    if (nelim > 0 && nf > 0)
-      for (int t = threadIdx.x; t < nf * nelim; t += blockDim.x) {
-        int jj = t % nf, c = t / nf;
-        Ls[jj][c] = V(k + nelim + jj, k + c);
-      }
-    __syncthreads();
-    const int64_t i = ts + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < bm) {
-      if (eff < bnelim)
-        for (int j = eff; j < bs; ++j) V(i, k + j) = A.pb[i + (int64_t)bperm[j] * bm];
-      if (nelim > 0) {
-        double* W = A.w + i;
-        lf_w_row(&V(i, k), A.m, nelim, bdt, bdd, bdo, W, bm);
-        for (int jj = 0; jj < nf; ++jj) {
-          double s = 0.0;
-          for (int c2 = 0; c2 < nelim; ++c2) s = __dadd_rn(s, __dmul_rn(W[(int64_t)c2 * bm], Ls[jj][c2]));
-          V(i, k + nelim + jj) = __dsub_rn(V(i, k + nelim + jj), s);
-        }
-      }
-    }
-  }
-  // the block's own rows, its D entries and counts (CTA 0, after its rows: the two touch different rows)
-  if (blockIdx.x == 0) lf_post_cta(A);  // uniform over the CTA
-}
-
-// delayed columns of the inner block to the end of the outer block (1 CTA)
-__device__ void lf_delay_cta(const LFArgs& A) {
-  LFState* st = A.st;
+// delayed columns of block b to the end of the outer block (1 CTA); returns the
+// new end of the columns still to be tried
+__device__ int lf_delay_cta(const LFArgs& A, const LFBlk* b, int nelim) {
   const int tid = threadIdx.x;
-  const int k = st->k, bs = st->bs, bnelim = st->bnelim, nelim = st->nelim;
-  int end_pos = st->end_pos;
-  if (bs == 0) return;
+  const int k = b->k, bs = b->bs;
+  int end_pos = A.st->end_pos;
   const int64_t bm = A.m - A.cs;
   PanelView V{A.a + A.cs + A.cs * A.m, A.m};
   __syncthreads();
-  if (bnelim == 0) {
+  if (b->bnelim == 0) {
     for (int off = 0; off < bs; ++off) {
       end_pos -= 1;
       if (k + off < end_pos) {
@@ -430,9 +356,8 @@ __device__ void lf_delay_cta(const LFArgs& A) {
         if (tid == 0) { int32_t t = A.lp[k + off]; A.lp[k + off] = A.lp[end_pos]; A.lp[end_pos] = t; }
       }
     }
-  } else if (nelim < bs) {
-    int nd = bs - nelim;
-    for (int i = nd - 1; i >= 0; --i) {
+  } else {
+    for (int i = bs - nelim - 1; i >= 0; --i) {
       int dp = k + nelim + i;
       end_pos -= 1;
       if (dp < end_pos) {
@@ -442,13 +367,86 @@ __device__ void lf_delay_cta(const LFArgs& A) {
     }
   }
   __syncthreads();
-  if (tid == 0) { st->k = k + nelim; st->end_pos = end_pos; st->bne = k + nelim; }
+  if (tid == 0) A.st->end_pos = end_pos;
+  return end_pos;
 }
-// the last inner block's delays (the others run at the start of the next k_lf_block)
-__global__ void __launch_bounds__(NT) k_lf_delay(LFArgs A) {
+
+// The rank-nelim update of the outer block's trailing columns, and the next
+// inner block (see the head of this file).  Grid: CTA 0, then CTAs whose warps
+// take the 32 x 32 lower tiles of rows [ts, bm), columns [ts, bcols) in turn.
+__global__ void __launch_bounds__(NT, 2) k_lf_update(LFArgs A, int next) {
   chain_enter();
-  if (A.st->spec_bad) return;  // a block issued past a mispredicted start column
-  lf_delay_cta(A);
+  __shared__ CtaShared sh;
+  __shared__ int s_last;
+  LFState* st = A.st;
+  const LFBlk* b = &st->b[A.par];
+  const int tid = threadIdx.x;
+  // the state in one round trip
+  const int spec_bad = st->spec_bad, bs = b->bs, bnelim = b->bnelim, k = b->k, end_pos = st->end_pos;
+  const unsigned two = b->two;
+  int nelim = b->eff;
+  if (spec_bad) return;  // a block issued past a mispredicted start column
+  // the eliminated count: the panel's first failing column, one less where it would split a 2x2
+  if (nelim > 0 && (two >> (nelim - 1)) & 1) nelim -= 1;
+  const int ts = k + bs;
+  const bool fail = nelim < bs;
+  if (blockIdx.x == 0) {
+    if (bs == 0) {  // nothing was left for this inner block
+      if (next) lf_block_cta(A, sh, A.par ^ 1, k, end_pos, 0, 0);
+      return;
+    }
+    if (!fail) {
+      if (next) lf_block_cta(A, sh, A.par ^ 1, ts, end_pos, k, nelim);
+      lf_post_cta(A, b, nelim);
+      if (tid == 0) st->bne = ts;
+      return;
+    }
+    if (bnelim > 0) lf_post_cta(A, b, nelim);
+  } else if (nelim > 0 || (fail && bnelim > 0)) {
+    const int bm = (int)(A.m - A.cs);
+    double* v = A.a + A.cs + A.cs * A.m;
+    PanelView V{v, A.m};
+    if (nelim > 0) {
+      const int bcols = (int)A.bcols;
+      const int nrt = (bm - ts + 31) / 32, nct = (bcols - ts + 31) / 32;
+      // the next diagonal block's entries are CTA 0's
+      const int skip = (next && !fail) ? ts + min(end_pos - ts, A.o.ib) : ts;
+      int ct = 0, rt = ((int)blockIdx.x - 1) * (NT / 32) + (tid >> 5);
+      const int step = ((int)gridDim.x - 1) * (NT / 32);
+      for (;; rt += step) {
+        while (ct < nct && rt >= nrt - ct) { rt -= nrt - ct; ++ct; }
+        if (ct >= nct) break;
+        warp_tile_update(v, A.m, ts + (ct + rt) * 32, ts + ct * 32, bm, bcols, A.w, bm, v + (int64_t)k * A.m, A.m,
+                         nelim, skip);
+      }
+    }
+    if (fail) {
+      // rows below the block: restore of the failed panel columns, the trailing x failed cross term
+      const int nf = bs - nelim;
+      for (int j = tid; j < nf * nelim; j += NT) sh.T[j % nf][j / nf] = V(k + nelim + j % nf, k + j / nf);
+      __syncthreads();
+      for (int64_t i = ts + (int64_t)(blockIdx.x - 1) * NT + tid; i < bm; i += (int64_t)(gridDim.x - 1) * NT) {
+        if (nelim < bnelim)
+          for (int j = nelim; j < bs; ++j) V(i, k + j) = A.pb[i + (int64_t)j * bm];
+        for (int jj = 0; jj < nf && nelim > 0; ++jj) {
+          double s = 0.0;
+          for (int c = 0; c < nelim; ++c) s = __dadd_rn(s, __dmul_rn(A.w[i + (int64_t)c * bm], sh.T[jj][c]));
+          V(i, k + nelim + jj) = __dsub_rn(V(i, k + nelim + jj), s);
+        }
+      }
+    }
+  }
+  if (!fail || bs == 0) return;
+  // columns failed: the last CTA to finish moves them to the end and factors the next block
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(&st->done, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();  // the other CTAs' writes
+  const int e2 = lf_delay_cta(A, b, nelim);
+  if (tid == 0) { st->done = 0; st->bne = k + nelim; }
+  if (next) lf_block_cta(A, sh, A.par ^ 1, k + nelim, e2, 0, 0);
 }
 
 // row permutation of the outer block applied to the front's earlier columns
@@ -471,23 +469,6 @@ __global__ void __launch_bounds__(256) k_lf_prop(LFArgs A) {
     int i = t % bc, c = t / bc;
     A.a[(A.cs + i) + (c0 + c) * A.m] = buf[t];
   }
-}
-
-// W = L D for the rows below the outer block, over its bne eliminated
-// columns, appended to the pending window
-__global__ void __launch_bounds__(128) k_lf_w(LFArgs A) {
-  chain_enter();
-  if (A.st->spec_bad) return;  // a block issued past a mispredicted start column
-  const int bne = A.st->bne;
-  const int64_t oe = A.cs + A.bcols;
-  const int64_t i = oe + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= A.m) return;
-  const int8_t* dt = A.D.type + A.cs;
-  const double* dd = A.D.diag + A.cs;
-  const double* dof = A.D.off + A.cs;
-  const double* l = A.a + i + A.cs * A.m;
-  double* w = A.wo + (i - A.wrow0) + A.wcol0 * A.wld;
-  lf_w_row(l, A.m, bne, dt, dd, dof, w, A.wld);
 }
 
 // end of an outer block: column order, delays to the end of the remaining

@@ -255,79 +255,85 @@ __device__ void cta_swap(PanelView V, int64_t rows, int64_t i, int64_t j) {
   __syncthreads();
 }
 
-// The trailing update of one inner block inside a view, by the whole CTA:
+// One warp's 32 x 32 tile of a rank-n update, n <= 32:
 //   V(i, j) = fma(-W(i, c), L(j, c), V(i, j)), c = 0 .. n - 1 in order,
-// for ts <= j < nfsb, j <= i < bm, with W(i, c) = W[(i - ts) + c ldw] and
-// L(j, c) = V(j, k + c) (update_trailing, factor.rs:1418-1526).  A contraction,
-// so it runs on the FP64 tensor pipe (mma.sync m8n8k4, the fma chain per entry
-// in order, as in gemm64.cuh): one 32 x 32 tile per warp at a time, operands
-// straight from L1 / L2.  A tile's 8 x 16 DMMAs keep the pipe busy for ~2000
-// cycles against ~130 of loads (8 fragment loads per 16 DMMAs), so staging in
-// shared memory and the barriers it would cost buy nothing.
-__device__ void cta_trailing_update(PanelView V, int k, int ts, int bm, int nfsb, int n, const double* W, int ldw) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// for i0 <= i < bm, j0 <= j < cmax, i >= j, with W(i, c) = W[i + c ldw] and
+// L(j, c) = L[j + c ldl]; entries with i < skip and j < skip are left alone.  A
+// contraction, so it runs on the FP64 tensor pipe (mma.sync m8n8k4, the fma
+// chain per entry in order, as in gemm64.cuh), operands straight from L1 / L2:
+// a tile's 8 x 16 DMMAs keep the pipe busy for ~2000 cycles against ~130 of
+// loads (8 fragment loads per 16 DMMAs), so staging in shared memory and the
+// barriers it would cost buy nothing.
+__device__ __forceinline__ void warp_tile_update(double* V, int64_t ld, int i0, int j0, int bm, int cmax,
+                                                 const double* W, int64_t ldw, const double* L, int64_t ldl, int n,
+                                                 int skip) {
+  const int lane = threadIdx.x & 31;
   const int fr = lane >> 2, fk = lane & 3, fc = fk * 2;
+  // offsets from the tile's corner: 32 columns stay far below 2^31
+  double* vt = V + i0 + (int64_t)j0 * ld + fr;
+  const double* wt = W + i0 + fr;
+  const double* lt = L + j0 + fr;
+  const int lv = (int)ld, lw = (int)ldw, ll = (int)ldl;
+  const int ni_ = bm - i0 - fr, nj_ = cmax - j0 - fc;  // rows 8 mi < ni_ and columns 8 ni + q < nj_ exist
+  const int dij = i0 + fr - j0 - fc;                   // i - j = dij + 8 (mi - ni) - q
+  double acc[4][4][2];
+#pragma unroll
+  for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int mi = 0; mi < 4; ++mi)
+        acc[mi][ni][q] = (8 * mi < ni_ && 8 * ni + q < nj_ && dij + 8 * (mi - ni) - q >= 0)
+                             ? vt[8 * mi + (8 * ni + fc + q) * lv]
+                             : 0.0;
+  double af[2][4], bf[2][4];
+  const int njl = cmax - j0 - fr;
+  auto load = [&](int kk, double* x, double* y) {
+    const int c = kk + fk;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      x[q] = (c < n && 8 * q < ni_) ? -wt[8 * q + c * lw] : 0.0;
+      y[q] = (c < n && 8 * q < njl) ? lt[8 * q + c * ll] : 0.0;
+    }
+  };
+  auto mma = [&](const double* x, const double* y) {
+#pragma unroll
+    for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+      for (int ni = 0; ni < 4; ++ni)
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                     : "+d"(acc[mi][ni][0]), "+d"(acc[mi][ni][1])
+                     : "d"(x[mi]), "d"(y[ni]));
+  };
+  load(0, af[0], bf[0]);
+  for (int kk = 0; kk < n; kk += 8) {  // columns past n are zeros: they add exact zeros
+    load(kk + 4, af[1], bf[1]);
+    mma(af[0], bf[0]);
+    if (kk + 8 < n) load(kk + 8, af[0], bf[0]);
+    if (kk + 4 < n) mma(af[1], bf[1]);
+  }
+#pragma unroll
+  for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int mi = 0; mi < 4; ++mi)
+        if (8 * mi < ni_ && 8 * ni + q < nj_ && dij + 8 * (mi - ni) - q >= 0 &&
+            (i0 + 8 * mi + fr >= skip || j0 + 8 * ni + fc + q >= skip))
+          vt[8 * mi + (8 * ni + fc + q) * lv] = acc[mi][ni][q];
+}
+
+// The trailing update of one inner block inside a view, by the whole CTA
+// (update_trailing, factor.rs:1418-1526): columns [ts, nfsb), rows [ts, bm),
+// lower, W(i, c) = W[(i - ts) + c ldw], L = the view's columns k .. k + n - 1.
+__device__ __noinline__ void cta_trailing_update(PanelView V, int k, int ts, int bm, int nfsb, int n, const double* W, int ldw) {
   const int nrt = (bm - ts + 31) / 32, nct = (nfsb - ts + 31) / 32;
-  const int ld = (int)V.ld;
-  const double* L = V.a + (int64_t)k * ld;
-  int ct = 0, rt = warp;  // the warp's tile: column tile ct, the rt-th row tile from the diagonal down
+  int ct = 0, rt = threadIdx.x >> 5;  // the warp's tile: column tile ct, the rt-th row tile from the diagonal down
   for (;; rt += NT / 32) {
     while (ct < nct && rt >= nrt - ct) { rt -= nrt - ct; ++ct; }
     if (ct >= nct) break;
-    const int j0 = ts + ct * 32, i0 = ts + (ct + rt) * 32;
-    double acc[4][4][2];
-#pragma unroll
-    for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int j = j0 + ni * 8 + fc + q;
-        const double* col = V.a + (int64_t)j * ld;
-#pragma unroll
-        for (int mi = 0; mi < 4; ++mi) {
-          const int i = i0 + mi * 8 + fr;
-          acc[mi][ni][q] = (i < bm && j < nfsb && i >= j) ? col[i] : 0.0;
-        }
-      }
-    double af[2][4], bf[2][4];
-    auto load = [&](int kk, double* x, double* y) {
-      const int c = kk + fk;
-      const double* w = W + (int64_t)c * ldw - ts;
-      const double* l = L + (int64_t)c * ld;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int i = i0 + q * 8 + fr, j = j0 + q * 8 + fr;
-        x[q] = (c < n && i < bm) ? -w[i] : 0.0;
-        y[q] = (c < n && j < nfsb) ? l[j] : 0.0;
-      }
-    };
-    auto mma = [&](const double* x, const double* y) {
-#pragma unroll
-      for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
-          asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                       : "+d"(acc[mi][ni][0]), "+d"(acc[mi][ni][1])
-                       : "d"(x[mi]), "d"(y[ni]));
-    };
-    load(0, af[0], bf[0]);
-    for (int kk = 0; kk < n; kk += 8) {  // columns past n are zeros: they add exact zeros
-      load(kk + 4, af[1], bf[1]);
-      mma(af[0], bf[0]);
-      if (kk + 8 < n) load(kk + 8, af[0], bf[0]);
-      if (kk + 4 < n) mma(af[1], bf[1]);
-    }
-#pragma unroll
-    for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int j = j0 + ni * 8 + fc + q;
-        double* col = V.a + (int64_t)j * ld;
-#pragma unroll
-        for (int mi = 0; mi < 4; ++mi) {
-          const int i = i0 + mi * 8 + fr;
-          if (i < bm && j < nfsb && i >= j) col[i] = acc[mi][ni][q];
-        }
-      }
+    warp_tile_update(V.a, V.ld, ts + (ct + rt) * 32, ts + ct * 32, bm, nfsb, W - ts, ldw, V.a + (int64_t)k * V.ld, V.ld,
+                     n, 0);
   }
 }
 
@@ -341,7 +347,7 @@ __device__ void cta_trailing_update(PanelView V, int k, int ts, int bm, int nfsb
 // trailing update (FP64 tensor pipe).  A 368 x 368 front took 500 us per 32
 // columns when the panel row lived in local memory (its loops had run-time
 // bounds) and the update re-read W and L from global memory for every entry.
-__device__ int cta_factor_inner(CtaShared& sh, PanelView V, int bm, int pl, int nfsb, DRec VD, int32_t* lp,
+__device__ __noinline__ int cta_factor_inner(CtaShared& sh, PanelView V, int bm, int pl, int nfsb, DRec VD, int32_t* lp,
                                 double* bk, int64_t ldb, double* W, const DevOpts& o) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ib = o.ib;
@@ -357,15 +363,18 @@ __device__ int cta_factor_inner(CtaShared& sh, PanelView V, int bm, int pl, int 
     // 1. backup a[k..bm, k..k+bs] (the panel rows are read back from it), 2. load the diagonal block
     for (int i = tid; i < rows; i += NT) {
       const double* src = &V(k + i, k);
-#pragma unroll
-      for (int h = 0; h < IBMAX; h += 16) {
+#pragma unroll 1
+      for (int h = 0; h < bs; h += 16) {
+        const double* s2 = src + (int64_t)h * V.ld;
+        double* b2 = bk + i + h * ldb;
+        const int lv = (int)V.ld, lb = (int)ldb;
         double v[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = (h + j < bs && (i >= bs || i >= h + j)) ? src[(int64_t)(h + j) * V.ld] : 0.0;
+        for (int j = 0; j < 16; ++j) v[j] = (h + j < bs && (i >= bs || i >= h + j)) ? s2[j * lv] : 0.0;
 #pragma unroll
         for (int j = 0; j < 16; ++j)
           if (h + j < bs) {
-            bk[i + (h + j) * ldb] = v[j];
+            b2[j * lb] = v[j];
             if (i < bs) sh.T[i][h + j] = v[j];
           }
       }
@@ -402,8 +411,9 @@ __device__ int cta_factor_inner(CtaShared& sh, PanelView V, int bm, int pl, int 
       const int32_t ob = tid < bs ? lp[k + tid] : 0;
       const int32_t nb = __shfl_sync(0xffffffffu, ob, sh.bperm[tid] & 31);
       if (tid < bs) lp[k + tid] = nb;
+      const unsigned two = __ballot_sync(0xffffffffu, tid < bnelim && sh.bdt[tid] == PT_2X2);
+      if (tid == 0) { sh.two = two; sh.eff = bnelim; }
     }
-    if (tid == 0) sh.eff = bnelim;
     // 5. row permutation of view columns 0..k: a warp per column
     {
       const int src = lane < bs ? sh.bperm[lane] : 0;
@@ -426,22 +436,31 @@ __device__ int cta_factor_inner(CtaShared& sh, PanelView V, int bm, int pl, int 
     // 3 + 7. each panel row permuted, TRSM with L11, D^-1 scaling, the threshold scan (apply_and_check,
     // factor.rs:1295-1408), and its W = L D for the update below (the pivots that pass keep theirs)
     const int tsz = bm - be;
+    const unsigned two = sh.two;
     for (int r = tid; r < tsz; r += NT) {
+      // leading dimensions the compiler may not see through: 32 column offsets each, hoisted out of this
+      // loop, would not leave registers for the row
+      int lb = (int)ldb, lv = (int)V.ld, lw = tsz;
+      asm volatile("" : "+r"(lb), "+r"(lv), "+r"(lw));
       double x[IBMAX];
       const double* src = bk + bs + r;
 #pragma unroll
-      for (int i = 0; i < IBMAX; ++i) x[i] = i < bs ? src[sh.bperm[i] * ldb] : 0.0;
-      const int fail = panel_row(x, sh.TT, sh.bdt, sh.bdd, sh.bdo, sh.dinv, bnelim, bound);
+      for (int i = 0; i < IBMAX; ++i) x[i] = i < bs ? src[sh.bperm[i] * lb] : 0.0;
+      const int fail = panel_row_t<false>(x, sh.TT, two, sh.bdd, sh.bdo, sh.dinv, bnelim, bound);
+      double* l = &V(be + r, k);
 #pragma unroll
       for (int i = 0; i < IBMAX; ++i)
-        if (i < bs) V(be + r, k + i) = x[i];
-      panel_row_w(x, sh.bdt, sh.bdd, sh.bdo, bnelim, W + r, tsz);
+        if (i < bs) l[i * lv] = x[i];
+      panel_row_w(x, two, sh.bdd, sh.bdo, bnelim);
+#pragma unroll
+      for (int i = 0; i < IBMAX; ++i)
+        if (i < bnelim) W[r + i * lw] = x[i];
       if (fail < bnelim) atomicMin(&sh.eff, fail);
     }
     __syncthreads();
     int eff = sh.eff;
     // 8. adjust_for_2x2_boundary (factor.rs:1161-1174)
-    if (eff > 0 && sh.bdt[eff - 1] == PT_2X2) eff -= 1;
+    if (eff > 0 && (two >> (eff - 1)) & 1) eff -= 1;
     // 9. partial restore of the failed columns
     if (eff < bnelim) {
       for (int t = tid; t < bs * bs; t += NT) {
@@ -2010,7 +2029,7 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
     ck(cudaStreamWaitEvent(st, cx.ev_far, 0), "cudaStreamWaitEvent (far-field update)");
     return irc;
   };
-  // Launches one outer block for start column S.gne (2 + 6 per inner block + the outer-block steps).
+  // Launches one outer block for start column S.gne (1 + 2 per inner block + the outer-block steps).
   auto issue = [&](const HostLF& S, int slot) -> Issued {
     Issued I{};
     I.before = S;
@@ -2022,39 +2041,31 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
     I.cs = cs; I.bcols = bcols; I.oe = oe;
     a.cs = cs;
     a.bcols = bcols;
-    launch_chain(h, k_lf_begin_outer, 1, 256, 0, st, a);
-    mk(RVG_PART_LF_SETUP);
+    I.window = two_level && oe < p;
+    a.win = I.window;
+    if (I.window) {  // this block's W joins the window [wd, gne + bne)
+      I.kadd = cs - wd;
+      a.wld = m - wrow;
+      a.wrow0 = wrow;
+      a.wcol0 = I.kadd;
+    }
+    launch_chain(h, k_lf_begin_outer, 1, NT, 0, st, a);
+    mk(RVG_PART_LF_BLOCK);
     const int64_t ninner = (bcols + ib - 1) / ib;
-    // the inner block's trailing update: rows and columns from ts = k + bs
-    // (device values) within the outer block's view
-    SyrkArgs gi{};
-    gi.C = a.a + cs + cs * m;
-    gi.ldc = m;
-    gi.W = a.w;
-    gi.ldw = bm;
-    gi.L = a.a + cs + cs * m;
-    gi.ldl = m;
-    gi.r1 = bm;
-    gi.c1 = bcols;
-    gi.Kdev = &a.st->nelim;
-    gi.dk = &a.st->k;
-    gi.dbs = &a.st->bs;
-    gi.skip = skip;
-    // per inner block: the diagonal block (after the previous inner block's delays), the panel rows, the
-    // post-processing with W = L D (k_lf_wi, its CTA 0 doing the block's own rows and D entries), the
-    // rank-nelim update; the last inner block's delays on their own
+    // per inner block: the panel rows, then its update beside the next inner block
     for (int64_t it = 0; it < ninner; ++it) {
-      launch_chain(h, k_lf_block, 1, NT, 0, st, a, it > 0 ? 1 : 0);
-      mk(RVG_PART_LF_BLOCK);
+      a.par = (int)(it & 1);
       launch_chain(h, k_lf_panel, blocks_for(bm, LF_PANEL_T), LF_PANEL_T, 0, st, a);
       mk(RVG_PART_LF_PANEL);
-      launch_chain(h, k_lf_wi, blocks_for(bm, 256), 256, 0, st, a);
-      launch_chain(h, k_syrk_inner, syrk_grid(gi), G_T, G_SMEM, st, gi);
+      // CTAs for the lower tiles right of column (it + 1) ib, where the trailing columns start if none was
+      // delayed (they take more tiles each otherwise), two per SM at most
+      const int64_t ts = std::min((it + 1) * ib, bcols), nrt = (bm - ts + 31) / 32, nct = (bcols - ts + 31) / 32;
+      const int64_t tiles = nct * nrt - nct * (nct - 1) / 2;
+      const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>((tiles + NT / 32 - 1) / (NT / 32), 2 * h->nsm));
+      launch_chain(h, k_lf_update, (unsigned)(1 + ctas), NT, 0, st, a, (int)(it + 1 < ninner));
       mk(RVG_PART_LF_UPDATE);
     }
-    launch_chain(h, k_lf_delay, 1, NT, 0, st, a);
-    mk(RVG_PART_LF_DELAY);
-    cx.launches += 2 + 4 * ninner;
+    cx.launches += 1 + 2 * ninner;
     if (two_level) {
       if (cs > 0) {
         launch_chain(h, k_lf_prop, (unsigned)((cs + LF_PROP_COLS - 1) / LF_PROP_COLS), 256,
@@ -2062,17 +2073,8 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
         cx.launches++;
         mk(RVG_PART_LF_PROP);
       }
-      if (oe < p) {
-        I.window = true;
-        // this block's W joins the window [wd, gne + bne)
-        const int64_t kadd = cs - wd;
-        I.kadd = kadd;
-        a.wld = m - wrow;
-        a.wrow0 = wrow;
-        a.wcol0 = kadd;
-        launch_chain(h, k_lf_w, blocks_for(m - oe, 128), 128, 0, st, a);
-        cx.launches++;
-        mk(RVG_PART_LF_W);
+      if (I.window) {
+        const int64_t kadd = I.kadd;
         // The next outer block is [g, g + min(rem - bcols, nb)); columns past
         // rem (delayed ones parked at the end) belong to no later block.  The
         // window is applied everywhere when it is full, or when the next block
@@ -3028,7 +3030,6 @@ rvg_status rvg_create(int64_t n, int64_t nsup, const int64_t* sup_begin, const i
   if ((rc = presize_arenas(h.get()))) return (rvg_status)rc;
   CK(cudaFuncSetAttribute(k_tpp_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TPP_SMEM_MAX));
   CK(cudaFuncSetAttribute(k_syrk_lower, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G_SMEM));
-  CK(cudaFuncSetAttribute(k_syrk_inner, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G_SMEM));
   CK(cudaFuncSetAttribute(k_syrk_tc<1, TC_TF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
   CK(cudaFuncSetAttribute(k_syrk_tc<2, TC_TF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
   CK(cudaFuncSetAttribute(k_syrk_tc<4, TC_TF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));

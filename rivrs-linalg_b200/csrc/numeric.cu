@@ -3240,11 +3240,16 @@ static int solve_common(rvg_handle* h, double* d_rhs, int64_t nrhs, int64_t ldb)
   const int64_t n = P.n;
   cudaStream_t st = h->st;
   if (n == 0 || nrhs == 0) return RVG_OK;
-  int rc = ensure(h->d_x, h->x_cap, (size_t)(n * nrhs), st);
+  // right-hand sides per pass: 8, 4, 2 or 1.  A pass costs the factor's read
+  // and the chain of its diagonal blocks whatever its width, so the last
+  // columns go through one pass of the next width up (5 to 7 as 8, 3 as 4)
+  // beside columns of zeros, not through several narrow ones
+  auto pass = [](int64_t left) { return left > 4 ? 8 : left > 2 ? 4 : (int)left; };
+  const int rmax = pass(nrhs);
+  const int64_t npad = nrhs / 8 * 8 + pass(nrhs % 8);
+  int rc = ensure(h->d_x, h->x_cap, (size_t)(n * npad), st);
   if (rc) return rc;
-  // right-hand sides per launch (a power of two up to 8) and the per-front
-  // solve workspace: forward results, then final values (R x m each)
-  const int rmax = nrhs >= 8 ? 8 : nrhs >= 4 ? 4 : nrhs >= 2 ? 2 : 1;
+  // the per-front solve workspace: forward results, then final values (R x m each)
   int64_t wneed = 0;
   std::vector<DFront> fr = h->h_fronts;
   for (auto& f : fr) { f.scratch = wneed; wneed += 2 * (int64_t)rmax * f.m; }
@@ -3257,6 +3262,7 @@ static int solve_common(rvg_handle* h, double* d_rhs, int64_t nrhs, int64_t ldb)
   k_perm_scale_in<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(d_rhs, ldb, nrhs, h->d_x, n, h->d_pfwd,
                                                                  h->has_scaling ? h->d_scal : nullptr);
   launches++;
+  if (npad > nrhs) CK(cudaMemsetAsync(h->d_x + n * nrhs, 0, (size_t)(n * (npad - nrhs)) * 8, st));
   // block layout of every wave: forward (diagonal then L21 blocks per front) and backward (diagonal blocks)
   const size_t nw = P.waves.size();
   Packer pk;
@@ -3331,7 +3337,8 @@ static int solve_common(rvg_handle* h, double* d_rhs, int64_t nrhs, int64_t ldb)
   };
   for (int64_t rh = 0; rh < nrhs;) {
     const int64_t left = nrhs - rh;
-    const int r = left >= 8 ? 8 : left >= 4 ? 4 : left >= 2 ? 2 : 1;
+    const int r = pass(left);
+    CK(cudaMemsetAsync(h->solve_work, 0xff, (size_t)wneed * 8, st));  // SF_EMPTY
     for (size_t w = 0; w < nw; ++w) {
       if (!nbf[w]) continue;
       CK(cudaMemsetAsync(h->sf_sync, 0, (size_t)(nbf[w] + 1) * 4, st));

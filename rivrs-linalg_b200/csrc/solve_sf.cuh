@@ -13,9 +13,9 @@
 //
 // forward, per front (y kept in the front's work vector v, rows < ne):
 //   diagonal block r (rows [64r, 64r + 64) of L11): y = x[col] - sum over the
-//     finished column blocks b < r of L[rows, b] y_b (each as soon as its flag
-//     is up), then the unit lower solve of the 64 x 64 diagonal block by one
-//     warp; publish y_r, raise flag r;
+//     finished column blocks b < r of L[rows, b] y_b (each as soon as it is
+//     there), then the unit lower solve of the 64 x 64 diagonal block;
+//     publish y_r;
 //   L21 block (rows >= ne): -sum over all column blocks of L[rows, b] y_b,
 //     added atomically into x at the parent's rows (siblings share rows).
 // backward, per front, in ticket order:
@@ -28,12 +28,25 @@
 //   column blocks, descending (x_final in v + m): z = D^-1 y on the block's
 //     columns (2x2 pairs may straddle blocks: y is still intact in v), minus
 //     the block's partial sums in group order, minus L[rows of later blocks,
-//     cols]^T x_final of those blocks (each once its flag is up), then the
-//     unit upper solve (L11^T) of the diagonal block by one warp;
-//     x[col] = x_final; raise the flag.
-// Per row (forward) and per column (backward) the sums run in ascending
-// column / row order inside each 64-block.  Up to 8 right-hand sides go
-// through one launch (template R), each L value read once for all of them.
+//     cols]^T x_final of those blocks (each once it is there), then the unit
+//     upper solve (L11^T) of the diagonal block; x[col] = x_final.
+//
+// The chain of diagonal blocks bounds a large front (212 blocks for order
+// 13,572), so what a block does between its predecessor's values and its own
+// is kept short:
+//   * the values are their own flags: the work vectors are filled with a
+//     pattern no value takes (SF_EMPTY; NaN results are stored as the
+//     canonical NaN), and a reader takes a value once it differs.  The next
+//     block of the chain polls the values themselves (one trip through L2
+//     instead of fence, flag, flag read and value read); the many blocks
+//     further away watch one value with one thread, to keep the traffic on
+//     those lines low;
+//   * the sums over 64 columns run as four interleaved chains;
+//   * the diagonal block is solved by eights: one thread per right-hand side
+//     solves 8 unknowns, then every row takes their update (16 short barriers
+//     instead of 64 warp-serial steps), with all right-hand sides side by side.
+// Up to 8 right-hand sides go through one launch (template R), each L value
+// read once for all of them.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -63,10 +76,10 @@ struct SfWave {
   double* part;     // backward partial sums: slot q at part + q R 64
   int32_t nfr, nblk;
   int32_t* ticket;  // zeroed before the launch
-  int32_t* flags;   // nblk entries, zeroed before the launch
+  int32_t* flags;   // nblk entries, zeroed before the launch (backward: gathers and partial sums)
   double* x;        // solution vectors, permuted order: right-hand side r at x + r ldx
   int64_t ldx;
-  double* work;     // per-front work at DFront::scratch: y (R x m) then x_final (R x m)
+  double* work;     // per-front work at DFront::scratch: y (R x m) then x_final (R x m); SF_EMPTY before the pass
   int32_t* err;
 };
 
@@ -83,6 +96,48 @@ __device__ __forceinline__ uint64_t sf_timer() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
+// A work value not written yet (all bits set).
+constexpr unsigned long long SF_EMPTY = ~0ull;
+__device__ __forceinline__ unsigned long long sf_peek(const double* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sf_publish(double* p, double v) {
+  const unsigned long long b = v != v ? 0x7ff8000000000000ull : (unsigned long long)__double_as_longlong(v);
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(b) : "memory");
+}
+// bounded wait for a published value
+__device__ __forceinline__ double sf_take(const double* p, int32_t* err) {
+  unsigned long long v = sf_peek(p);
+  if (v == SF_EMPTY) {
+    const uint64_t t0 = sf_timer();
+    while ((v = sf_peek(p)) == SF_EMPTY) {
+      if (sf_timer() - t0 > SF_TIMEOUT_NS) {
+        atomicExch(err, 2);
+        return 0.0;
+      }
+    }
+  }
+  return __longlong_as_double((long long)v);
+}
+// The R values of a block's column t (at src + r m, t < n) into dst[r][t], by the whole CTA.  far: one
+// thread watches the block's last column first.
+template <int R>
+__device__ __forceinline__ void sf_take_block(const double* src, int64_t m, int n, bool far, double (*dst)[SF_B],
+                                              int32_t* err) {
+  const int t = threadIdx.x;
+  if (far) {
+    if (t == 0) (void)sf_take(src + (R - 1) * m + n - 1, err);
+    __syncthreads();
+  }
+  if (t < n) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) dst[r][t] = sf_take(src + r * m + t, err);
+  }
+  __syncthreads();
+}
+
 // bounded wait for a published block (thread 0 of the CTA)
 __device__ __forceinline__ void sf_wait(const int32_t* flag, int32_t* err) {
   if (sf_ld_acquire(flag)) return;
@@ -127,7 +182,78 @@ __device__ __forceinline__ void sf_load_strip(const double* src, int64_t m, int 
   }
 }
 
-// R right-hand sides at once: every L value read is used R times.
+// acc[r] -= sum_c l[c] y[r][c] over a 64-column strip: four interleaved chains per right-hand side
+// (columns past the block hold l = 0, y is finite or the front's result is not)
+template <int R>
+__device__ __forceinline__ void sf_strip(const double (&l)[SF_B], int n, const double (*y)[SF_B], double (&acc)[R]) {
+  constexpr int W = R <= 2 ? 4 : 2;  // chains: enough right-hand sides fill the pipe by themselves
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    double s[W];
+#pragma unroll
+    for (int u = 0; u < W; ++u) s[u] = 0.0;
+#pragma unroll
+    for (int c = 0; c < SF_B; ++c)
+      if (c < n) s[c % W] = __fma_rn(-l[c], y[r][c], s[c % W]);
+#pragma unroll
+    for (int u = 0; u < W; ++u) acc[r] += s[u];
+  }
+}
+
+// Unit triangular solve of a diagonal block of n <= 64 rows held in shared
+// memory, row t of the R right-hand sides in acc of thread t; y is scratch.
+// Lower: L(t, j) = Ld[t][j], from the top; upper (the transpose): Ld[j][t],
+// from the bottom.  By eights: thread r solves the 8 unknowns of right-hand
+// side r, then every remaining row takes their update.
+template <int R, bool UPPER>
+__device__ __forceinline__ void sf_diag(const double (*Ld)[SF_B + 1], int n, double (*y)[SF_B], double (&acc)[R]) {
+  const int t = threadIdx.x;
+  const int nb = (n + 7) / 8;
+  for (int q = 0; q < nb; ++q) {
+    const int j0 = (UPPER ? nb - 1 - q : q) * 8, j1 = j0 + 8 < n ? j0 + 8 : n;
+    if (t >= j0 && t < j0 + 8) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) y[r][t] = t < n ? acc[r] : 0.0;
+    }
+    __syncthreads();
+    if (t < R) {
+      double v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = y[t][j0 + i];
+      if (!UPPER) {
+#pragma unroll
+        for (int j = 0; j < 7; ++j)
+#pragma unroll
+          for (int i = j + 1; i < 8; ++i)
+            if (j0 + i < n) v[i] = __fma_rn(-Ld[j0 + i][j0 + j], v[j], v[i]);
+      } else {
+#pragma unroll
+        for (int j = 7; j > 0; --j)
+          if (j0 + j < n) {
+#pragma unroll
+            for (int i = 0; i < j; ++i) v[i] = __fma_rn(-Ld[j0 + j][j0 + i], v[j], v[i]);
+          }
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) y[t][j0 + i] = v[i];
+    }
+    __syncthreads();
+    if (t >= j0 && t < j1) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) acc[r] = y[r][t];
+    } else if (UPPER ? t < j0 : (t >= j1 && t < n)) {
+      double l[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) l[j] = j0 + j < n ? (UPPER ? Ld[j0 + j][t] : Ld[t][j0 + j]) : 0.0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[r] = __fma_rn(-l[j], y[r][j0 + j], acc[r]);
+    }
+  }
+}
+
+// R right-hand sides at once: every L value is read once for all of them.
 template <int R>
 __global__ void __launch_bounds__(SF_B) k_sf_fwd(SfWave w, const DFront* F, Arenas A) {
   __shared__ int s_blk;
@@ -147,7 +273,6 @@ __global__ void __launch_bounds__(SF_B) k_sf_fwd(SfWave w, const DFront* F, Aren
     const int32_t* rows = A.idx + fr.idx;
     const int32_t* perm = rows + m;
     double* v = w.work + fr.scratch;  // y of right-hand side r at v + r m
-    int32_t* flags = w.flags + sf.blk0;
     const int b = blk - sf.blk0;
     const bool diag = b < sf.nbd;
     const int64_t r0 = diag ? (int64_t)b * SF_B : ne + (int64_t)(b - sf.nbd) * SF_B;
@@ -173,45 +298,18 @@ __global__ void __launch_bounds__(SF_B) k_sf_fwd(SfWave w, const DFront* F, Aren
       const int nc = (int)((c0 + SF_B < ne ? c0 + SF_B : ne) - c0);
       double lr[SF_B];
       if (row) sf_load_strip(L + i + c0 * m, m, nc, lr);
-      if (t == 0) sf_wait(&flags[cb], w.err);
-      __syncthreads();
-      if (t < nc) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) yb[r][t] = __ldcg(&v[r * m + c0 + t]);
-      }
-      __syncthreads();
-      if (row) {
-#pragma unroll
-        for (int c = 0; c < SF_B; ++c)
-          if (c < nc) {
-#pragma unroll
-            for (int r = 0; r < R; ++r) acc[r] = __fma_rn(-lr[c], yb[r][c], acc[r]);
-          }
-      }
+      sf_take_block<R>(v + c0, m, nc, !(diag && cb == b - 1), yb, w.err);
+      if (row) sf_strip<R>(lr, nc, yb, acc);
       __syncthreads();
     }
     if (diag) {
-      // unit lower solve of rows [r0, r1) by warp 0 (lane: rows r0 + lane, r0 + 32 + lane),
-      // on the diagonal block staged in shared memory above
+      __syncthreads();  // the staged diagonal block
+      sf_diag<R, false>(Ls, nr, yb, acc);
+      if (row) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) yb[r][t] = acc[r];
-      __syncthreads();
-      if (t < 32) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          double a0 = yb[r][t], a1 = yb[r][t + 32];
-          for (int j = 0; j < nr; ++j) {
-            const double yj = __shfl_sync(0xffffffffu, j < 32 ? a0 : a1, j & 31);
-            if (t > j && t < nr) a0 = __fma_rn(-Ls[t][j], yj, a0);
-            if (t + 32 > j && t + 32 < nr) a1 = __fma_rn(-Ls[t + 32][j], yj, a1);
-          }
-          if (t < nr) v[r * m + r0 + t] = a0;
-          if (t + 32 < nr) v[r * m + r0 + t + 32] = a1;
-        }
+        for (int r = 0; r < R; ++r) sf_publish(&v[r * m + i], acc[r]);
       }
-      __threadfence();
-      __syncthreads();
-      if (t == 0) sf_st_release(&flags[b], 1);
+      __syncthreads();  // Ls and yb are free again
     } else if (row) {
       const int32_t g = sf_row(rows, perm, ne, fr.k, i - ne);
 #pragma unroll
@@ -333,56 +431,47 @@ __global__ void __launch_bounds__(SF_B) k_sf_bwd(SfWave w, const DFront* F, Aren
 #pragma unroll
       for (int r = 0; r < R; ++r) acc[r] = __dsub_rn(acc[r], __ldcg(&slot[r * SF_B + t]));
     }
-    // rows of later diagonal blocks, from the last one down, as they finish
-    const int cb0 = nbr + npart;  // flag of column block q' at flags[cb0 + q']
+    // rows of later diagonal blocks, from the last one down, as they finish; each strip is in shared memory
+    // before the wait on its block
     for (int rblk = sf.nbd - 1; rblk > b; --rblk) {
       const int64_t i0 = (int64_t)rblk * SF_B;
       const int nr = (int)((i0 + SF_B < ne ? i0 + SF_B : ne) - i0);
-      double lr[SF_B];  // the strip, read before the wait on its block
-      if (t < nr) sf_load_strip(L + i0 + t + c0 * m, m, nc, lr);
-      if (t == 0) sf_wait(&flags[cb0 + (sf.nbd - 1 - rblk)], w.err);
-      __syncthreads();
-      if (t < nr) {
+      __syncthreads();  // the strip before it has been used
+      if (t < nr) sf_load_strip(L + i0 + t + c0 * m, m, nc, &Ls[t][0]);
+      sf_take_block<R>(xf + i0, m, nr, rblk != b + 1, xs, w.err);
+      if (col) {
+        double s[R][4];
 #pragma unroll
-        for (int r = 0; r < R; ++r) xs[r][t] = __ldcg(&xf[r * m + i0 + t]);
+        for (int r = 0; r < R; ++r) s[r][0] = s[r][1] = s[r][2] = s[r][3] = 0.0;
+        int rr = 0;
+        for (; rr + 4 <= nr; rr += 4)
 #pragma unroll
-        for (int c = 0; c < SF_B; ++c) Ls[t][c] = lr[c];
-      }
-      __syncthreads();
-      if (col)
-        for (int rr = 0; rr < nr; ++rr) {
+          for (int u = 0; u < 4; ++u) {
+            const double l = Ls[rr + u][t];
+#pragma unroll
+            for (int r = 0; r < R; ++r) s[r][u] = __fma_rn(-l, xs[r][rr + u], s[r][u]);
+          }
+        for (; rr < nr; ++rr) {
           const double l = Ls[rr][t];
 #pragma unroll
-          for (int r = 0; r < R; ++r) acc[r] = __fma_rn(-l, xs[r][rr], acc[r]);
+          for (int r = 0; r < R; ++r) s[r][0] = __fma_rn(-l, xs[r][rr], s[r][0]);
         }
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[r] += (s[r][0] + s[r][1]) + (s[r][2] + s[r][3]);
+      }
     }
     // the diagonal block: x_c = acc_c - sum_{c < i < c0 + nc} L(i, c) x_i, from the bottom
     __syncthreads();
-#pragma unroll
-    for (int r = 0; r < R; ++r) xs[r][t] = acc[r];
-    __syncthreads();
-    if (t < 32) {
+    sf_diag<R, true>(Ld, nc, xs, acc);
+    if (col) {
+      const int32_t g = sf_col(rows, perm, c0 + t);
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        double a0 = xs[r][t], a1 = xs[r][t + 32];
-        for (int j = nc - 1; j >= 0; --j) {
-          const double xj = __shfl_sync(0xffffffffu, j < 32 ? a0 : a1, j & 31);
-          if (t < j) a0 = __fma_rn(-Ld[j][t], xj, a0);
-          if (t + 32 < j) a1 = __fma_rn(-Ld[j][t + 32], xj, a1);
-        }
-        if (t < nc) {
-          xf[r * m + c0 + t] = a0;
-          w.x[r * w.ldx + sf_col(rows, perm, c0 + t)] = a0;
-        }
-        if (t + 32 < nc) {
-          xf[r * m + c0 + t + 32] = a1;
-          w.x[r * w.ldx + sf_col(rows, perm, c0 + t + 32)] = a1;
-        }
+        sf_publish(&xf[r * m + c0 + t], acc[r]);
+        w.x[r * w.ldx + g] = acc[r];
       }
     }
-    __threadfence();
-    __syncthreads();
-    if (t == 0) sf_st_release(&flags[blk - sf.blk0], 1);
+    __syncthreads();  // Ld and xs are free again
   }
 }
 

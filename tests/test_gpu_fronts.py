@@ -60,3 +60,31 @@ def test_medium_fronts(rv, orc, k, r, kind):
 @pytest.mark.parametrize("ib,nb", [(8, 32), (17, 64), (32, 96)])
 def test_medium_fronts_block_sizes(rv, orc, ib, nb):
     check(rv, orc, 150, 45, "delay", small_leaf_threshold=0, inner_block_size=ib, outer_block_size=nb)
+
+
+# every width a pass of the solve can have (8, 4, 2, 1 columns, the last one padded), over fronts of one and
+# several 64-column blocks with remainders
+@pytest.mark.parametrize("nrhs", [2, 3, 5, 7, 8, 9, 13])
+@pytest.mark.parametrize("k,r", [(40, 23), (130, 65), (449, 64)])
+def test_solve_widths(rv, orc, k, r, nrhs):
+    s = arrow_system(rv, k, r, k + nrhs, "plain")
+    solver, ref, b = run_both(rv, orc, s, order=np.arange(s.n, dtype=np.int64), nrhs=nrhs)
+    assert_parity(rv, s, solver, ref, b, bwd=1e-12)
+    solver.close()
+    ref.close()
+
+
+def test_solve_nan_right_hand_side(rv):
+    # a NaN travels through the blocks' published values instead of looking unpublished; other columns keep theirs
+    s = arrow_system(rv, 200, 70, 5, "plain")
+    solver = rv.SparseLDLT.analyze(s)
+    solver.factor()
+    b = rv.problems.rhs_uniform(s.n, 1, 3)
+    x = solver.solve(b)
+    bad = b.copy(order="F")
+    bad[7, 1] = np.frombuffer(b"\xff" * 8)[0]
+    y = solver.solve(bad)
+    assert np.isnan(y[:, 1]).any()
+    for j in (0, 2):
+        assert np.linalg.norm(y[:, j] - x[:, j]) <= 1e-10 * np.linalg.norm(x[:, j])
+    solver.close()

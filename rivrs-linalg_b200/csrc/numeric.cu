@@ -683,83 +683,124 @@ namespace rvg {
 // ---------------------------------------------------------------------------
 struct TileItem { int32_t front; int32_t ti; int32_t tj; int32_t pad; };
 
-// W = L21_NFS * D into scratch (nfs x ne, column-major)
-__global__ void k_cb_w(const TileItem* items, const DFront* F, Arenas A) {
-  TileItem it = items[blockIdx.x];
+// W = L21_NFS * D into scratch (nfs x ne, column-major) for the fronts whose
+// contribution GEMM reads it (launch_syrk): 256 rows x CBW_COLS columns per
+// CTA, one row per thread, every load of the chunk before its first store.  (A
+// thread that walks all of a front's columns pays one memory round trip per
+// column: 339 us for 12,882 x 648.)  A 2x2 pair belongs to the chunk of its
+// first column.
+constexpr int CBW_COLS = 32;
+__global__ void __launch_bounds__(256) k_cb_w(const TileItem* items, const DFront* F, Arenas A) {
+  const TileItem it = items[blockIdx.x];
   const DFront fr = F[it.front];
-  const double* L = A.panel + fr.panel;
-  double* W = A.scratch + fr.scratch;
   const int8_t* dt = A.dtype + fr.dpos;
   const double* dd = A.ddiag + fr.dpos;
   const double* dof = A.doff + fr.dpos;
-  int64_t i = (int64_t)it.ti * 256 + threadIdx.x;
-  if (i >= fr.nfs) return;
-  const double* l = L + fr.k + i;
-  int c = 0;
-  while (c < fr.ne) {
-    if (dt[c] == PT_1X1) { W[i + (int64_t)c * fr.nfs] = __dmul_rn(l[(int64_t)c * fr.m], dd[c]); c += 1; }
-    else {
-      double l1 = l[(int64_t)c * fr.m], l2 = l[(int64_t)(c + 1) * fr.m];
-      W[i + (int64_t)c * fr.nfs] = __dadd_rn(__dmul_rn(l1, dd[c]), __dmul_rn(l2, dof[c]));
-      W[i + (int64_t)(c + 1) * fr.nfs] = __dadd_rn(__dmul_rn(l1, dof[c]), __dmul_rn(l2, dd[c + 1]));
-      c += 2;
+  const int64_t i = (int64_t)it.ti * 256 + threadIdx.x;
+  const int c0 = it.tj * CBW_COLS, n = fr.ne - c0;
+  if (i >= fr.nfs || n <= 0) return;
+  const double* l = A.panel + fr.panel + fr.k + i + (int64_t)c0 * fr.m;
+  double* W = A.scratch + fr.scratch + i + (int64_t)c0 * fr.nfs;
+  dt += c0;
+  dd += c0;
+  dof += c0;
+  double lv[CBW_COLS + 1];
+#pragma unroll
+  for (int c = 0; c <= CBW_COLS; ++c) lv[c] = c < n ? l[(int64_t)c * fr.m] : 0.0;
+#pragma unroll
+  for (int c = 0; c < CBW_COLS; ++c) {
+    if (c >= n) break;
+    const int8_t t = dt[c];
+    if (t == PT_1X1) {
+      W[(int64_t)c * fr.nfs] = __dmul_rn(lv[c], dd[c]);
+    } else if (t == PT_2X2) {
+      W[(int64_t)c * fr.nfs] = __dadd_rn(__dmul_rn(lv[c], dd[c]), __dmul_rn(lv[c + 1], dof[c]));
+      W[(int64_t)(c + 1) * fr.nfs] = __dadd_rn(__dmul_rn(lv[c], dof[c]), __dmul_rn(lv[c + 1], dd[c + 1]));
     }
   }
 }
 
-constexpr int GT = 64;  // output tile
-constexpr int GK = 16;  // reduction chunk
+constexpr int GT = 64;  // output tile of k_cb_gemm
 
+// Contribution blocks of the small and medium fronts:
 // C[i,j] = fma(-W[i,c], L[j,c], C[i,j]) for c ascending (each output entry an
-// fma chain in the oracle's order); 256 threads, 4x4 outputs per thread.
-__global__ void __launch_bounds__(256) k_cb_gemm(const TileItem* items, const DFront* F, Arenas A) {
-  TileItem it = items[blockIdx.x];
+// fma chain in the oracle's order), W = L D formed as it is loaded: a W entry is
+// one or two products, so it costs less than a pass that writes W and a second
+// one that reads it.  64 x 64 outputs per CTA, 32 x 32 per warp on the FP64
+// tensor pipe (as warp_tile_update); the next step's operands load while this
+// one's 16 DMMAs run.
+__global__ void __launch_bounds__(128) k_cb_gemm(const TileItem* items, const DFront* F, Arenas A) {
+  const TileItem it = items[blockIdx.x];
   const DFront fr = F[it.front];
-  const int64_t nfs = fr.nfs, ne = fr.ne, ldl = fr.m;
-  const double* L = A.panel + fr.panel + fr.k;  // L21_NFS(j, c) = L[j + c*ldl]
-  const double* W = A.scratch + fr.scratch;     // W(i, c) = W[i + c*nfs]
-  double* C = A.cbase + fr.cb;
-  __shared__ double sW[GK][GT + 1];
-  __shared__ double sL[GK][GT + 1];
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const int64_t i0 = (int64_t)it.ti * GT, j0 = (int64_t)it.tj * GT;
-  double acc[4][4];
+  const int nfs = fr.nfs, ne = fr.ne, m = fr.m;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int fr_ = lane >> 2, fk = lane & 3, fc = fk * 2;
+  const int i0 = it.ti * GT + (warp & 1) * 32, j0 = it.tj * GT + (warp >> 1) * 32;
+  if (ne <= 0 || i0 >= nfs || j0 >= nfs || i0 + 31 < j0) return;
+  const double* L = A.panel + fr.panel + fr.k;  // L21_NFS(j, c) = L[j + c m]
+  const int8_t* dt = A.dtype + fr.dpos;
+  const double* dd = A.ddiag + fr.dpos;
+  const double* dof = A.doff + fr.dpos;
+  double* C = A.cbase + fr.cb + i0 + fr_ + (int64_t)(j0 + fc) * nfs;
+  const double* la = L + i0 + fr_;
+  const double* lb = L + j0 + fr_;
+  const int ni = nfs - i0 - fr_, njc = nfs - j0 - fc, njl = nfs - j0 - fr_;
+  const int dij = i0 + fr_ - j0 - fc;
+  double acc[4][4][2];
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int y = 0; y < 4; ++y)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      int64_t i = i0 + ty + 16 * a, j = j0 + tx + 16 * b;
-      acc[a][b] = (i < nfs && j < nfs && i >= j) ? C[i + j * nfs] : 0.0;
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        acc[x][y][q] = (8 * x < ni && 8 * y + q < njc && dij + 8 * (x - y) - q >= 0)
+                           ? C[8 * x + (int64_t)(8 * y + q) * nfs]
+                           : 0.0;
+  auto load = [&](int kk, double* a, double* b) {
+    const int c = kk + fk;
+    const bool in = c < ne;
+    const int8_t t = in ? dt[c] : (int8_t)PT_DELAYED;
+    // W(., c): the pair's first column times e0, its second times e1 (1x1: one product)
+    const int cf = t == PT_2X2B ? c - 1 : c;
+    const double e0 = !in ? 0.0 : (t == PT_2X2B ? dof[cf] : dd[c]);
+    const double e1 = t == PT_2X2 ? dof[c] : (t == PT_2X2B ? dd[c] : 0.0);
+    const bool pair = t == PT_2X2 || t == PT_2X2B;
+    const double* l0 = la + (int64_t)cf * m;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const bool row = in && 8 * q < ni;
+      const double v0 = row ? l0[8 * q] : 0.0;
+      const double v1 = row && pair ? l0[8 * q + m] : 0.0;
+      const double w = __dmul_rn(v0, e0);
+      a[q] = -(pair ? __dadd_rn(w, __dmul_rn(v1, e1)) : w);
+      b[q] = in && 8 * q < njl ? lb[8 * q + (int64_t)c * m] : 0.0;
     }
-  for (int64_t c0 = 0; c0 < ne; c0 += GK) {
-    for (int t = threadIdx.x; t < GK * GT; t += 256) {
-      int r = t % GT, c = t / GT;
-      int64_t cc = c0 + c;
-      sW[c][r] = (i0 + r < nfs && cc < ne) ? W[i0 + r + cc * nfs] : 0.0;
-      sL[c][r] = (j0 + r < nfs && cc < ne) ? L[j0 + r + cc * ldl] : 0.0;
-    }
-    __syncthreads();
-    int kc = (int)(ne - c0 < GK ? ne - c0 : GK);
-    for (int c = 0; c < kc; ++c) {
-      double wv[4], lv[4];
+  };
+  auto mma = [&](const double* a, const double* b) {
 #pragma unroll
-      for (int a = 0; a < 4; ++a) wv[a] = sW[c][ty + 16 * a];
+    for (int x = 0; x < 4; ++x)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) lv[b] = sL[c][tx + 16 * b];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = __fma_rn(-wv[a], lv[b], acc[a][b]);
-    }
-    __syncthreads();
+      for (int y = 0; y < 4; ++y)
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                     : "+d"(acc[x][y][0]), "+d"(acc[x][y][1])
+                     : "d"(a[x]), "d"(b[y]));
+  };
+  double af[2][4], bf[2][4];
+  load(0, af[0], bf[0]);
+  for (int kk = 0; kk < ne; kk += 8) {  // columns past ne are zeros: they add exact zeros
+    load(kk + 4, af[1], bf[1]);
+    mma(af[0], bf[0]);
+    if (kk + 8 < ne) load(kk + 8, af[0], bf[0]);
+    if (kk + 4 < ne) mma(af[1], bf[1]);
   }
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int y = 0; y < 4; ++y)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      int64_t i = i0 + ty + 16 * a, j = j0 + tx + 16 * b;
-      if (i < nfs && j < nfs && i >= j) C[i + j * nfs] = acc[a][b];
-    }
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        if (8 * x < ni && 8 * y + q < njc && dij + 8 * (x - y) - q >= 0)
+          C[8 * x + (int64_t)(8 * y + q) * nfs] = acc[x][y][q];
 }
 
 // ---------------------------------------------------------------------------
@@ -1693,7 +1734,7 @@ int presize_arenas(rvg_handle* h) {
       bool large = front_is_large(m, tpp, T, mid);
       int64_t sc = tpp ? 0 : (2 * IBMAX * m + nb);
       if (large) sc = m * (2 * IBMAX + lf_window_blocks(h) * nb) + nb;
-      if (has_cb) sc = std::max<int64_t>(sc, nfs * k);
+      if (has_cb && large) sc = std::max<int64_t>(sc, nfs * k);  // k_cb_w
       sc_w += sc;
       if (x.parent >= 0) rel[w] = std::max<int64_t>(rel[w], P.height[x.parent]);
     }
@@ -2340,6 +2381,12 @@ int factor_large_fronts(rvg_handle* h, const std::vector<int32_t>& ids, const Ar
 
 int finish_factor(rvg_handle* h, int64_t d_used);
 
+// k_cb_w's items of front s (columns that were delayed are found on the device)
+void add_cb_w(std::vector<TileItem>& items, int32_t s, const DFront& f) {
+  for (int tj = 0; tj * CBW_COLS < f.k; ++tj)
+    for (int ti = 0; ti * 256 < f.nfs; ++ti) items.push_back(TileItem{s, ti, tj, 0});
+}
+
 // Learned precision: large fronts of the wave just factored whose mixed-form
 // D grew past the bound (k_front_growth) are factored again in FP64, alone.
 // Each is assembled again from scratch -- original entries and its children's
@@ -2382,8 +2429,11 @@ int refactor_fp64(rvg_handle* h, const std::vector<int32_t>& redo, const Arenas&
   for (int32_t s : redo) {
     const DFront& f = h->h_fronts[s];
     if (!(f.flags & FF_HAS_CB) || f.k == 0) continue;
-    for (int ti = 0; ti * 256 < f.nfs; ++ti) witems.push_back(TileItem{s, ti, 0, 0});
-    if (f.nfs >= 256) { big_cb.push_back(s); continue; }  // GEMM by launch_syrk
+    if (f.nfs >= 256) {  // GEMM by launch_syrk
+      add_cb_w(witems, s, f);
+      big_cb.push_back(s);
+      continue;
+    }
     const int nt = (f.nfs + GT - 1) / GT;
     for (int tj = 0; tj < nt; ++tj)
       for (int ti = tj; ti < nt; ++ti) gitems.push_back(TileItem{s, ti, tj, 0});
@@ -2412,7 +2462,7 @@ int refactor_fp64(rvg_handle* h, const std::vector<int32_t>& redo, const Arenas&
   if (!witems.empty())
     k_cb_w<<<(unsigned)witems.size(), 256, 0, st>>>((const TileItem*)(D + o_w), h->d_fronts, A);
   if (!gitems.empty())
-    k_cb_gemm<<<(unsigned)gitems.size(), 256, 0, st>>>((const TileItem*)(D + o_g), h->d_fronts, A);
+    k_cb_gemm<<<(unsigned)gitems.size(), 128, 0, st>>>((const TileItem*)(D + o_g), h->d_fronts, A);
   for (int32_t s : big_cb) {
     const DFront& f = h->h_fronts[s];
     SyrkArgs ga{A.cbase + f.cb, f.nfs, A.scratch + f.scratch, f.nfs, A.panel + f.panel + f.k, f.m,
@@ -2565,7 +2615,7 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
         if (large) f.flags |= FF_LARGE;
         int64_t sc = tpp ? 0 : (2 * IBMAX * m + h->opt.outer_block_size);
         if (large) sc = m * (2 * IBMAX + lf_window_blocks(h) * h->opt.outer_block_size) + h->opt.outer_block_size;
-        if (f.flags & FF_HAS_CB) sc = std::max<int64_t>(sc, nfs * k);
+        if ((f.flags & FF_HAS_CB) && large) sc = std::max<int64_t>(sc, nfs * k);  // k_cb_w
         f.scratch = scratch_need; scratch_need += sc;
       }
     }
@@ -2642,8 +2692,10 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
     for (int64_t s : wave) {
       const DFront& f = h->h_fronts[s];
       if (!(f.flags & FF_HAS_CB) || f.k == 0) continue;
-      for (int ti = 0; ti * 256 < f.nfs; ++ti) witems.push_back(TileItem{(int32_t)s, ti, 0, 0});
-      if ((f.flags & FF_LARGE) && f.nfs >= 256) continue;  // GEMM by launch_syrk
+      if ((f.flags & FF_LARGE) && f.nfs >= 256) {  // GEMM by launch_syrk
+        add_cb_w(witems, (int32_t)s, f);
+        continue;
+      }
       int nt = (f.nfs + GT - 1) / GT;
       for (int tj = 0; tj < nt; ++tj)
         for (int ti = tj; ti < nt; ++ti) gitems.push_back(TileItem{(int32_t)s, ti, tj, 0});
@@ -2760,7 +2812,7 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
       k_cb_w<<<(unsigned)witems.size(), 256, 0, st>>>((const TileItem*)(D + o_w), h->d_fronts, A);
     mark(h, RVG_PART_CB_W);
     if (!gitems.empty())
-      k_cb_gemm<<<(unsigned)gitems.size(), 256, 0, st>>>((const TileItem*)(D + o_g), h->d_fronts, A);
+      k_cb_gemm<<<(unsigned)gitems.size(), 128, 0, st>>>((const TileItem*)(D + o_g), h->d_fronts, A);
     mark(h, RVG_PART_CB_GEMM);
     for (int64_t s : wave) {
       const DFront& f = h->h_fronts[s];

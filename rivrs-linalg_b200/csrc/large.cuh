@@ -13,12 +13,12 @@
 //                         panel row; the block's row permutation of the outer
 //                         block's earlier columns
 //     lf_update  grid     CTA 0: the NEXT inner block's 32 x 32 diagonal block
-//                         takes this block's update and is factored at once,
-//                         then this block's D entries; the other CTAs: the
-//                         rank-32 update of the outer block's trailing columns
+//                         takes this block's update and is factored at once; the
+//                         other CTAs: the rank-32 update of the outer block's trailing columns
 //                         on the FP64 tensor pipe.  The block is 32 dependent
 //                         pivot steps on one SM, so it runs beside the update
-//                         instead of after it.  When columns failed their
+//                         instead of after it (the block's own D entries are
+//                         written by the last CTA).  When columns failed their
 //                         threshold test, nothing is known of the next block
 //                         yet: CTA 0 does the post-processing, the others also
 //                         restore the failed panel columns and form their
@@ -202,6 +202,45 @@ __global__ void __launch_bounds__(NT) k_lf_begin_outer(LFArgs A) {
 // are a prefix, and the columns after them are written again by later blocks.
 // Rows below the outer block also leave it in the window of pending columns.
 constexpr int LF_PANEL_T = 64;
+
+// One panel row; FULL: a 32-column block all of whose pivots were found, the
+// usual one (nothing is tested against the block's width).  Returns the first
+// failing pivot.
+template <bool FULL>
+__device__ __forceinline__ int lf_panel_row(const LFArgs& A, const PanelView& V, const double (*TT)[IBMAX + 2],
+                                            const int* bperm, const double* bdd, const double* bdo,
+                                            const double* dinv, unsigned two, int64_t r, int k, int bs, int bnelim,
+                                            double bound) {
+  const int64_t bm = A.m - A.cs;
+  // every load of the row before the first store: the backup may alias the
+  // panel as far as the compiler knows, so a load placed after a store
+  // would wait for it (one memory round trip per column)
+  double x[IBMAX];
+  double* l = &V(r, k);
+#pragma unroll
+  for (int i = 0; i < IBMAX; ++i) x[i] = l[(int64_t)bperm[FULL ? i : min(i, bs - 1)] * A.m];
+  double* pb = A.pb + r;  // the backup, in the block's column order
+#pragma unroll
+  for (int i = 0; i < IBMAX; ++i)
+    if (FULL || i < bs) pb[i * bm] = x[i];
+  const int fail = panel_row_t<FULL>(x, TT, two, bdd, bdo, dinv, bnelim, bound);
+#pragma unroll
+  for (int i = 0; i < IBMAX; ++i)
+    if (FULL || i < bs) l[i * A.m] = x[i];
+  panel_row_w(x, two, bdd, bdo, bnelim);
+  double* w = A.w + r;
+#pragma unroll
+  for (int i = 0; i < IBMAX; ++i)
+    if (FULL || i < bnelim) w[i * bm] = x[i];
+  if (A.win && r >= A.bcols) {
+    w = A.wo + (A.cs + r - A.wrow0) + (A.wcol0 + k) * A.wld;
+#pragma unroll
+    for (int i = 0; i < IBMAX; ++i)
+      if (FULL || i < bnelim) w[i * A.wld] = x[i];
+  }
+  return fail;
+}
+
 __global__ void __launch_bounds__(LF_PANEL_T) k_lf_panel(LFArgs A) {
   chain_enter();
   __shared__ alignas(16) double TT[IBMAX][IBMAX + 2];  // TT[l][j] = L11(j, l)
@@ -246,32 +285,9 @@ __global__ void __launch_bounds__(LF_PANEL_T) k_lf_panel(LFArgs A) {
       if (i < bs) V(k + i, r) = buf[i];
   }
   if (r >= be && r < bm) {
-    // every load of the row before the first store: the backup may alias the
-    // panel as far as the compiler knows, so a load placed after a store
-    // would wait for it (one memory round trip per column)
-    double x[IBMAX];
-#pragma unroll
-    for (int i = 0; i < IBMAX; ++i) x[i] = i < bs ? V(r, k + bperm[i]) : 0.0;
-    double* pb = A.pb + r;  // the backup, in the block's column order
-#pragma unroll
-    for (int i = 0; i < IBMAX; ++i)
-      if (i < bs) pb[i * bm] = x[i];
-    const int fail = panel_row(x, TT, two, bdd, bdo, dinv, bnelim, bound);
-    double* l = &V(r, k);
-#pragma unroll
-    for (int i = 0; i < IBMAX; ++i)
-      if (i < bs) l[i * A.m] = x[i];
-    panel_row_w(x, two, bdd, bdo, bnelim);
-    double* w = A.w + r;
-#pragma unroll
-    for (int i = 0; i < IBMAX; ++i)
-      if (i < bnelim) w[i * bm] = x[i];
-    if (A.win && r >= A.bcols) {
-      w = A.wo + (A.cs + r - A.wrow0) + (A.wcol0 + k) * A.wld;
-#pragma unroll
-      for (int i = 0; i < IBMAX; ++i)
-        if (i < bnelim) w[i * A.wld] = x[i];
-    }
+    const int fail = (bs == IBMAX && bnelim == IBMAX)
+                         ? lf_panel_row<true>(A, V, TT, bperm, bdd, bdo, dinv, two, r, k, bs, bnelim, bound)
+                         : lf_panel_row<false>(A, V, TT, bperm, bdd, bdo, dinv, two, r, k, bs, bnelim, bound);
     if (fail < bnelim) atomicMin(&s_fail, fail);
   }
   __syncthreads();
@@ -396,9 +412,8 @@ __global__ void __launch_bounds__(NT, 2) k_lf_update(LFArgs A, int next) {
       return;
     }
     if (!fail) {
-      if (next) lf_block_cta(A, sh, A.par ^ 1, ts, end_pos, k, nelim);
-      lf_post_cta(A, b, nelim);
       if (tid == 0) st->bne = ts;
+      if (next) lf_block_cta(A, sh, A.par ^ 1, ts, end_pos, k, nelim);
       return;
     }
     if (bnelim > 0) lf_post_cta(A, b, nelim);
@@ -420,6 +435,7 @@ __global__ void __launch_bounds__(NT, 2) k_lf_update(LFArgs A, int next) {
                          nelim, skip);
       }
     }
+    if (!fail && blockIdx.x == gridDim.x - 1) lf_post_cta(A, b, nelim);  // (off CTA 0's path)
     if (fail) {
       // rows below the block: restore of the failed panel columns, the trailing x failed cross term
       const int nf = bs - nelim;

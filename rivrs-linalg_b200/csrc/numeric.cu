@@ -269,64 +269,83 @@ __device__ __forceinline__ void warp_tile_update(double* V, int64_t ld, int i0, 
                                                  int skip) {
   const int lane = threadIdx.x & 31;
   const int fr = lane >> 2, fk = lane & 3, fc = fk * 2;
-  // offsets from the tile's corner: 32 columns stay far below 2^31
-  double* vt = V + i0 + (int64_t)j0 * ld + fr;
-  const double* wt = W + i0 + fr;
-  const double* lt = L + j0 + fr;
+  // Offsets from the tile's corner (32 columns stay far below 2^31).  Rows and
+  // columns past the region are clamped to its last one and dropped later, so
+  // that every load is unconditional: a guarded load is a branch, and the
+  // loads of a step then wait for one another.
+  double* vt = V + i0 + (int64_t)j0 * ld;
+  const double* wt = W + i0;
+  const double* lt = L + j0;
   const int lv = (int)ld, lw = (int)ldw, ll = (int)ldl;
-  const int ni_ = bm - i0 - fr, nj_ = cmax - j0 - fc;  // rows 8 mi < ni_ and columns 8 ni + q < nj_ exist
-  const int dij = i0 + fr - j0 - fc;                   // i - j = dij + 8 (mi - ni) - q
+  const int ri = bm - 1 - i0, rj = cmax - 1 - j0;  // the last row and column
+  int oi[4], oj[4];                                 // the lane's operand rows
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    oi[q] = min(8 * q + fr, ri);
+    oj[q] = min(8 * q + fr, rj);
+  }
   double acc[4][4][2];
 #pragma unroll
   for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
-    for (int q = 0; q < 2; ++q)
+    for (int q = 0; q < 2; ++q) {
+      const double* col = vt + min(8 * ni + fc + q, rj) * lv;
 #pragma unroll
-      for (int mi = 0; mi < 4; ++mi)
-        acc[mi][ni][q] = (8 * mi < ni_ && 8 * ni + q < nj_ && dij + 8 * (mi - ni) - q >= 0)
-                             ? vt[8 * mi + (8 * ni + fc + q) * lv]
-                             : 0.0;
+      for (int mi = 0; mi < 4; ++mi) acc[mi][ni][q] = col[oi[mi]];
+    }
   double af[2][4], bf[2][4];
-  const int njl = cmax - j0 - fr;
   auto load = [&](int kk, double* x, double* y) {
-    const int c = kk + fk;
+    const int c = min(kk + fk, n - 1);
+    const double* w = wt + c * lw;
+    const double* l = lt + c * ll;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      x[q] = (c < n && 8 * q < ni_) ? -wt[8 * q + c * lw] : 0.0;
-      y[q] = (c < n && 8 * q < njl) ? lt[8 * q + c * ll] : 0.0;
+      x[q] = w[oi[q]];
+      y[q] = l[oj[q]];
     }
   };
-  auto mma = [&](const double* x, const double* y) {
+  auto mma = [&](int kk, const double* x, const double* y) {
+    const bool in = kk + fk < n;  // columns past n: zeros, which add exact zeros
+    double xn[4], yn[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      xn[q] = in ? -x[q] : 0.0;
+      yn[q] = in ? y[q] : 0.0;
+    }
 #pragma unroll
     for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
       for (int ni = 0; ni < 4; ++ni)
         asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                      : "+d"(acc[mi][ni][0]), "+d"(acc[mi][ni][1])
-                     : "d"(x[mi]), "d"(y[ni]));
+                     : "d"(xn[mi]), "d"(yn[ni]));
   };
   load(0, af[0], bf[0]);
-  for (int kk = 0; kk < n; kk += 8) {  // columns past n are zeros: they add exact zeros
+#pragma unroll 1
+  for (int kk = 0; kk < n; kk += 8) {
     load(kk + 4, af[1], bf[1]);
-    mma(af[0], bf[0]);
-    if (kk + 8 < n) load(kk + 8, af[0], bf[0]);
-    if (kk + 4 < n) mma(af[1], bf[1]);
+    mma(kk, af[0], bf[0]);
+    load(kk + 8, af[0], bf[0]);
+    if (kk + 4 < n) mma(kk + 4, af[1], bf[1]);
   }
 #pragma unroll
   for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
-    for (int q = 0; q < 2; ++q)
+    for (int q = 0; q < 2; ++q) {
+      const int dj = 8 * ni + fc + q;
+      double* col = vt + dj * lv;
 #pragma unroll
-      for (int mi = 0; mi < 4; ++mi)
-        if (8 * mi < ni_ && 8 * ni + q < nj_ && dij + 8 * (mi - ni) - q >= 0 &&
-            (i0 + 8 * mi + fr >= skip || j0 + 8 * ni + fc + q >= skip))
-          vt[8 * mi + (8 * ni + fc + q) * lv] = acc[mi][ni][q];
+      for (int mi = 0; mi < 4; ++mi) {
+        const int di = 8 * mi + fr;
+        if (di <= ri && dj <= rj && i0 + di >= j0 + dj && (i0 + di >= skip || j0 + dj >= skip)) col[di] = acc[mi][ni][q];
+      }
+    }
 }
 
 // The trailing update of one inner block inside a view, by the whole CTA
 // (update_trailing, factor.rs:1418-1526): columns [ts, nfsb), rows [ts, bm),
 // lower, W(i, c) = W[(i - ts) + c ldw], L = the view's columns k .. k + n - 1.
-__device__ __noinline__ void cta_trailing_update(PanelView V, int k, int ts, int bm, int nfsb, int n, const double* W, int ldw) {
+__device__ void cta_trailing_update(PanelView V, int k, int ts, int bm, int nfsb, int n, const double* W, int ldw) {
   const int nrt = (bm - ts + 31) / 32, nct = (nfsb - ts + 31) / 32;
   int ct = 0, rt = threadIdx.x >> 5;  // the warp's tile: column tile ct, the rt-th row tile from the diagonal down
   for (;; rt += NT / 32) {
@@ -347,7 +366,7 @@ __device__ __noinline__ void cta_trailing_update(PanelView V, int k, int ts, int
 // trailing update (FP64 tensor pipe).  A 368 x 368 front took 500 us per 32
 // columns when the panel row lived in local memory (its loops had run-time
 // bounds) and the update re-read W and L from global memory for every entry.
-__device__ __noinline__ int cta_factor_inner(CtaShared& sh, PanelView V, int bm, int pl, int nfsb, DRec VD, int32_t* lp,
+__device__ int cta_factor_inner(CtaShared& sh, PanelView V, int bm, int pl, int nfsb, DRec VD, int32_t* lp,
                                 double* bk, int64_t ldb, double* W, const DevOpts& o) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ib = o.ib;
@@ -741,42 +760,55 @@ __global__ void __launch_bounds__(128) k_cb_gemm(const TileItem* items, const DF
   const int8_t* dt = A.dtype + fr.dpos;
   const double* dd = A.ddiag + fr.dpos;
   const double* dof = A.doff + fr.dpos;
-  double* C = A.cbase + fr.cb + i0 + fr_ + (int64_t)(j0 + fc) * nfs;
-  const double* la = L + i0 + fr_;
-  const double* lb = L + j0 + fr_;
-  const int ni = nfs - i0 - fr_, njc = nfs - j0 - fc, njl = nfs - j0 - fr_;
-  const int dij = i0 + fr_ - j0 - fc;
+  double* C = A.cbase + fr.cb + i0 + (int64_t)j0 * nfs;
+  const double* la = L + i0;
+  const double* lb = L + j0;
+  const int ri = nfs - 1 - i0, rj = nfs - 1 - j0;  // loads clamped to the last row and column (warp_tile_update)
+  int oi[4], oj[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    oi[q] = min(8 * q + fr_, ri);
+    oj[q] = min(8 * q + fr_, rj);
+  }
   double acc[4][4][2];
 #pragma unroll
   for (int y = 0; y < 4; ++y)
 #pragma unroll
-    for (int q = 0; q < 2; ++q)
+    for (int q = 0; q < 2; ++q) {
+      const double* col = C + min(8 * y + fc + q, rj) * nfs;
 #pragma unroll
-      for (int x = 0; x < 4; ++x)
-        acc[x][y][q] = (8 * x < ni && 8 * y + q < njc && dij + 8 * (x - y) - q >= 0)
-                           ? C[8 * x + (int64_t)(8 * y + q) * nfs]
-                           : 0.0;
-  auto load = [&](int kk, double* a, double* b) {
-    const int c = kk + fk;
-    const bool in = c < ne;
-    const int8_t t = in ? dt[c] : (int8_t)PT_DELAYED;
-    // W(., c): the pair's first column times e0, its second times e1 (1x1: one product)
-    const int cf = t == PT_2X2B ? c - 1 : c;
-    const double e0 = !in ? 0.0 : (t == PT_2X2B ? dof[cf] : dd[c]);
-    const double e1 = t == PT_2X2 ? dof[c] : (t == PT_2X2B ? dd[c] : 0.0);
-    const bool pair = t == PT_2X2 || t == PT_2X2B;
+      for (int x = 0; x < 4; ++x) acc[x][y][q] = col[oi[x]];
+    }
+  // a step's operands: the lane's column of L for its W entries (the pair's first column and its second;
+  // equal ones for a 1x1), their coefficients, the column of L for the other side
+  struct Op { double v0[4], v1[4], b[4], e0, e1; int kind; };
+  auto load = [&](int kk, Op& o) {
+    const int c = min(kk + fk, ne - 1);
+    const int8_t t = dt[c];
+    const int cf = t == PT_2X2B ? c - 1 : c, cs = t == PT_2X2 ? c + 1 : c;
+    o.kind = kk + fk >= ne ? 0 : (t == PT_1X1 ? 1 : 2);
+    const double d = dd[c], off = dof[cf];
+    o.e0 = t == PT_2X2B ? off : d;
+    o.e1 = t == PT_2X2B ? d : off;
     const double* l0 = la + (int64_t)cf * m;
+    const double* l1 = la + (int64_t)cs * m;
+    const double* l2 = lb + (int64_t)c * m;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const bool row = in && 8 * q < ni;
-      const double v0 = row ? l0[8 * q] : 0.0;
-      const double v1 = row && pair ? l0[8 * q + m] : 0.0;
-      const double w = __dmul_rn(v0, e0);
-      a[q] = -(pair ? __dadd_rn(w, __dmul_rn(v1, e1)) : w);
-      b[q] = in && 8 * q < njl ? lb[8 * q + (int64_t)c * m] : 0.0;
+      o.v0[q] = l0[oi[q]];
+      o.v1[q] = l1[oi[q]];
+      o.b[q] = l2[oj[q]];
     }
   };
-  auto mma = [&](const double* a, const double* b) {
+  auto mma = [&](const Op& o) {
+    double a[4], b[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const double w0 = __dmul_rn(o.v0[q], o.e0);
+      const double w = o.kind == 2 ? __dadd_rn(w0, __dmul_rn(o.v1[q], o.e1)) : w0;
+      a[q] = o.kind ? -w : 0.0;
+      b[q] = o.kind ? o.b[q] : 0.0;
+    }
 #pragma unroll
     for (int x = 0; x < 4; ++x)
 #pragma unroll
@@ -785,22 +817,27 @@ __global__ void __launch_bounds__(128) k_cb_gemm(const TileItem* items, const DF
                      : "+d"(acc[x][y][0]), "+d"(acc[x][y][1])
                      : "d"(a[x]), "d"(b[y]));
   };
-  double af[2][4], bf[2][4];
-  load(0, af[0], bf[0]);
+  Op p0, p1;
+  load(0, p0);
+#pragma unroll 1
   for (int kk = 0; kk < ne; kk += 8) {  // columns past ne are zeros: they add exact zeros
-    load(kk + 4, af[1], bf[1]);
-    mma(af[0], bf[0]);
-    if (kk + 8 < ne) load(kk + 8, af[0], bf[0]);
-    if (kk + 4 < ne) mma(af[1], bf[1]);
+    load(kk + 4, p1);
+    mma(p0);
+    load(kk + 8, p0);
+    if (kk + 4 < ne) mma(p1);
   }
 #pragma unroll
   for (int y = 0; y < 4; ++y)
 #pragma unroll
-    for (int q = 0; q < 2; ++q)
+    for (int q = 0; q < 2; ++q) {
+      const int dj = 8 * y + fc + q;
+      double* col = C + (int64_t)dj * nfs;
 #pragma unroll
-      for (int x = 0; x < 4; ++x)
-        if (8 * x < ni && 8 * y + q < njc && dij + 8 * (x - y) - q >= 0)
-          C[8 * x + (int64_t)(8 * y + q) * nfs] = acc[x][y][q];
+      for (int x = 0; x < 4; ++x) {
+        const int di = 8 * x + fr_;
+        if (di <= ri && dj <= rj && i0 + di >= j0 + dj) col[di] = acc[x][y][q];
+      }
+    }
 }
 
 // ---------------------------------------------------------------------------

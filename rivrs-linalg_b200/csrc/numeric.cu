@@ -75,12 +75,9 @@ void set_error(const std::string& s) { g_err = s; }
 
 // Row list of each front: owned ++ delayed-from-children ++ pattern
 // (numeric.rs:1239-1262), and the identity pivot order.
-__global__ void k_front_rows(const int32_t* ids, int n, DFront* F, Statics S, Arenas A) {
-  int f = blockIdx.x;
-  if (f >= n) return;
-  int s = ids[f];
-  const DFront fr = F[s];
-  int32_t* rows = A.idx + fr.idx;
+// dly: the children's delay offsets, in order (nullptr: those of their descriptors).
+__device__ __forceinline__ void front_rows_cta(int s, const DFront& fr, const Statics& S, const Arenas& A,
+                                               const DFront* F, const int32_t* dly, int32_t* rows) {
   int32_t* perm = rows + fr.m;
   int64_t o0 = S.own_ptr[s];
   for (int i = threadIdx.x; i < fr.nown; i += blockDim.x) rows[i] = S.own_idx[o0 + i];
@@ -88,12 +85,20 @@ __global__ void k_front_rows(const int32_t* ids, int n, DFront* F, Statics S, Ar
   for (int i = threadIdx.x; i < fr.nfs; i += blockDim.x) rows[fr.k + i] = S.pat_idx[p0 + i];
   for (int i = threadIdx.x; i < fr.k; i += blockDim.x) perm[i] = i;
   for (int64_t q = S.ch_ptr[s]; q < S.ch_ptr[s + 1]; ++q) {
-    const DFront c = F[S.ch_idx[q]];
-    int nd = c.k - c.ne;
+    const DFront& c = F[S.ch_idx[q]];
+    const int ne = c.ne, nd = c.k - ne;
+    if (nd == 0) continue;
     const int32_t* crow = A.idx + c.idx;
     const int32_t* cperm = crow + c.m;
-    for (int i = threadIdx.x; i < nd; i += blockDim.x) rows[fr.nown + c.dly_off + i] = crow[cperm[c.ne + i]];
+    const int off = fr.nown + (dly ? dly[q - S.ch_ptr[s]] : c.dly_off);
+    for (int i = threadIdx.x; i < nd; i += blockDim.x) rows[off + i] = crow[cperm[ne + i]];
   }
+}
+__global__ void k_front_rows(const int32_t* ids, int n, DFront* F, Statics S, Arenas A) {
+  if ((int)blockIdx.x >= n) return;
+  const int s = ids[blockIdx.x];
+  const DFront fr = F[s];
+  front_rows_cta(s, fr, S, A, F, nullptr, A.idx + fr.idx);
 }
 
 struct ScatterItem { int32_t front; int32_t pad; int64_t e0; };
@@ -897,10 +902,22 @@ __global__ void k_norms3(const double* r, const double* x, const double* b, int6
   }
   if ((threadIdx.x & 31) == 0) { atomicAdd(out, s0); atomicAdd(out + 1, s1); atomicAdd(out + 2, s2); }
 }
-// Raises *flag when any of the n values is NaN or infinite.
-__global__ void k_nonfinite(const double* v, int64_t n, int32_t* flag) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    if (!isfinite(v[i])) { atomicExch(flag, 1); return; }
+// One read of the n values before a factorization: *flag is raised when any of
+// them is NaN or infinite, and their sum of squares (||A||_F^2 for the
+// refinement) is added to *sum when given.
+struct ScanOut { double sum; int32_t bad, pad; };
+__global__ void k_scan_values(const double* v, int64_t n, ScanOut* out, int want_sum) {
+  double s = 0;
+  bool bad = false;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const double x = v[i];
+    bad |= !isfinite(x);
+    s += x * x;
+  }
+  if (bad) atomicExch(&out->bad, 1);
+  if (!want_sum) return;
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) atomicAdd(&out->sum, s);
 }
 
 __global__ void k_sumsq(const double* v, int64_t n, double* out) {
@@ -960,19 +977,71 @@ __global__ void k_axpy1(double* x, const double* d, int64_t n, int64_t ldx, int6
 // ===========================================================================
 namespace rvg {
 
-// publish a wave's descriptors / pick up the children's delay offsets
-__global__ void k_put_fronts(const DFront* staged, const int32_t* ids, int n, DFront* F) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) F[ids[i]] = staged[i];
+// Start of a wave, one CTA per front: its descriptor, its children's delay
+// offsets (dly_vals: the wave's children in order, front i's from dly0[i] on),
+// its row list (k_front_rows) and, for blocks of order <= WB_ZERO, the zeroed
+// lower triangle of its contribution block (larger ones: k_zero_cb_lower).  Four
+// kernels of a few microseconds each otherwise, and as many launches, in every
+// wave.
+constexpr int WB_ZERO = 256;
+__global__ void __launch_bounds__(128) k_wave_begin(const DFront* staged, const int32_t* ids, const int32_t* dly0,
+                                                    const int32_t* dly_vals, DFront* F, Statics S, Arenas A) {
+  const int i = blockIdx.x, s = ids[i];
+  const DFront fr = staged[i];
+  if (threadIdx.x == 0) F[s] = fr;
+  int32_t* rows = A.idx + fr.idx;
+  front_rows_cta(s, fr, S, A, F, dly_vals + dly0[i], rows);
+  const int64_t q0 = S.ch_ptr[s], nq = S.ch_ptr[s + 1] - q0;
+  __syncthreads();  // (the children's descriptors have been read)
+  for (int64_t q = threadIdx.x; q < nq; q += blockDim.x) F[S.ch_idx[q0 + q]].dly_off = dly_vals[dly0[i] + q];
+  if ((fr.flags & FF_HAS_CB) && fr.nfs <= WB_ZERO) {
+    double* c = A.cbase + fr.cb;
+    for (int j = threadIdx.x >> 5; j < fr.nfs; j += (int)(blockDim.x >> 5))
+      for (int r = j + (threadIdx.x & 31); r < fr.nfs; r += 32) c[r + (int64_t)j * fr.nfs] = 0.0;
+  }
 }
-__global__ void k_put_dly(const int32_t* ids, const int32_t* vals, int n, DFront* F) {
+// eliminated counts of a wave's fronts, and behind them the device error word
+__global__ void k_get_counts(const int32_t* ids, int n, const DFront* F, int32_t* out, const int32_t* err) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) F[ids[i]].dly_off = vals[i];
-}
-__global__ void k_get_counts(const int32_t* ids, int n, const DFront* F, int32_t* out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (err && i == 0) out[3 * n] = *err;
   if (i < n) { const DFront& f = F[ids[i]]; out[3 * i] = f.ne; out[3 * i + 1] = f.n1; out[3 * i + 2] = f.n2; }
 }
+// The factorization's D by sign (MixedDiagonal::compute_inertia,
+// diagonal.rs:391-461), out[0..2] = positive, negative, zero eigenvalues, and
+// out[3] = its zero pivots (numeric.rs:987-1009).  One warp per front at a
+// time; counting here leaves four numbers to copy instead of the D arrays.
+__global__ void __launch_bounds__(256) k_d_counts(const DFront* F, int64_t ns, Arenas A, unsigned long long* out) {
+  const int lane = threadIdx.x & 31;
+  int64_t c[4] = {0, 0, 0, 0};
+  for (int64_t s = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); s < ns; s += (int64_t)gridDim.x * 8) {
+    const DFront f = F[s];
+    for (int i = lane; i < f.ne; i += 32) {
+      const int64_t q = f.dpos + i;
+      const int8_t t = A.dtype[q];
+      const double a = A.ddiag[q];
+      if (t == PT_1X1) {
+        c[a > 0 ? 0 : (a < 0 ? 1 : 2)]++;
+        if (a == 0.0) c[3]++;
+      } else if (t == PT_2X2) {
+        const double b = A.doff[q], cc = A.ddiag[q + 1];
+        const double det = a * cc - b * b, tr = a + cc;
+        if (det > 0) c[tr > 0 ? 0 : 1] += 2;
+        else if (det < 0) { c[0]++; c[1]++; }
+        else if (tr > 0) { c[0]++; c[2]++; }
+        else if (tr < 0) { c[1]++; c[2]++; }
+        else c[2] += 2;
+      }
+    }
+    if (lane == 0 && f.parent < 0 && f.ne < f.m) c[3] += f.k - f.ne;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    int64_t v = c[q];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0 && v) atomicAdd(out + q, (unsigned long long)v);
+  }
+}
+
 // Refactorization replay checks: the counts (and a large front's progress)
 // the captured schedule assumed.  On a difference the flag is raised and the
 // recorded value put in place of the computed one, so that every later launch
@@ -1239,7 +1308,9 @@ struct rvg_handle {
   std::vector<int32_t> sel_large;                    // the large fronts of the last factorization
   bool sel_force_fp64 = false;                       // the FP64 refactorization after a growth flag
   int aptp_ctas = 0;                                 // resident CTAs of the medium fronts' queue kernel
-  int32_t* d_nonfinite = nullptr;                    // set when the values or the scaling hold NaN or Inf
+  ScanOut* d_scan = nullptr;                         // the scan of the values and the scaling before a factorization
+  unsigned long long* d_dcount = nullptr;            // k_d_counts: D entries by sign, zero pivots
+  int64_t inertia[3] = {0, 0, 0};                    // of the last factorization
   int64_t sel_routed = 0, sel_flagged = 0, sel_fallback = 0;
   // measurement
   bool profiling = false;
@@ -2506,7 +2577,7 @@ int refactor_fp64(rvg_handle* h, const std::vector<int32_t>& redo, const Arenas&
                 0, f.nfs, 0, f.nfs, 0, &h->d_fronts[s].ne};
     if ((rc = launch_syrk(h, ga, f.k, false))) return rc;
   }
-  k_get_counts<<<blocks_for(n, 128), 128, 0, st>>>(d_ids, n, h->d_fronts, (int32_t*)(D + o_cnt));
+  k_get_counts<<<blocks_for(n, 128), 128, 0, st>>>(d_ids, n, h->d_fronts, (int32_t*)(D + o_cnt), nullptr);
   int32_t* hc = (int32_t*)h->h_stage2;
   CK(cudaMemcpyAsync(hc, D + o_cnt, (size_t)3 * n * 4, cudaMemcpyDeviceToHost, st));
   const double ts0 = now_ms();
@@ -2615,14 +2686,14 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
     const int nw = (int)wave.size();
     // ---- sizes from the children's eliminated counts (numeric.rs:1239-1262)
     int64_t panel_need = 0, idx_need = 0, d_need = 0, cb_need = 0, scratch_need = 0;
-    std::vector<int32_t> dly_ids, dly_vals;
+    std::vector<int32_t> dly0, dly_vals;  // the children's delay offsets, and each front's first
     for (int64_t s : wave) {
       DFront& f = h->h_fronts[s];
+      dly0.push_back((int32_t)dly_vals.size());
       int64_t nown = P.sn[s].n_owned(), ndin = 0;
       for (int64_t c : P.children[s]) {
         DFront& cf = h->h_fronts[c];
         cf.dly_off = (int32_t)ndin;
-        dly_ids.push_back((int32_t)c);
         dly_vals.push_back((int32_t)ndin);
         ndin += cf.k - cf.ne;
       }
@@ -2721,7 +2792,7 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
     std::vector<CbZeroItem> zitems;
     for (int64_t s : wave) {
       const DFront& f = h->h_fronts[s];
-      if (f.flags & FF_HAS_CB)
+      if ((f.flags & FF_HAS_CB) && f.nfs > WB_ZERO)
         for (int j0 = 0; j0 < f.nfs; j0 += 32) zitems.push_back(CbZeroItem{(int32_t)s, j0});
     }
     std::vector<TileItem> witems, gitems;
@@ -2738,7 +2809,7 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
         for (int ti = tj; ti < nt; ++ti) gitems.push_back(TileItem{(int32_t)s, ti, tj, 0});
     }
     Packer pk;
-    size_t o_staged = pk.add(staged), o_ids = pk.add(ids), o_dly_ids = pk.add(dly_ids), o_dly_vals = pk.add(dly_vals);
+    size_t o_staged = pk.add(staged), o_ids = pk.add(ids), o_dly0 = pk.add(dly0), o_dly_vals = pk.add(dly_vals);
     size_t o_tpp = pk.add(tpp_ids), o_aptp = pk.add(aptp_ids), o_s = pk.add(sitems);
     std::vector<size_t> o_e(maxch);
     for (size_t q = 0; q < maxch; ++q) o_e[q] = pk.add(eitems[q]);
@@ -2765,18 +2836,14 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
     CK(cudaMemcpyAsync(h->d_stage, hs, pk.buf.size(), cudaMemcpyHostToDevice, st));
     char* D = h->d_stage;
     const int32_t* d_ids = (const int32_t*)(D + o_ids);
-    // ---- descriptors
-    k_put_fronts<<<blocks_for(nw, 128), 128, 0, st>>>((const DFront*)(D + o_staged), d_ids, nw, h->d_fronts);
-    if (!dly_ids.empty())
-      k_put_dly<<<blocks_for(dly_ids.size(), 128), 128, 0, st>>>((const int32_t*)(D + o_dly_ids),
-                                                                 (const int32_t*)(D + o_dly_vals), (int)dly_ids.size(),
-                                                                 h->d_fronts);
-    // contribution blocks of this wave: zero lower triangles (the extend-add adds into them)
+    // ---- descriptors, row lists, small contribution blocks
+    k_wave_begin<<<nw, 128, 0, st>>>((const DFront*)(D + o_staged), d_ids, (const int32_t*)(D + o_dly0),
+                                     (const int32_t*)(D + o_dly_vals), h->d_fronts, statics(h), A);
+    // the larger contribution blocks of this wave: zero lower triangles (the extend-add adds into them)
     if (!zitems.empty())
       k_zero_cb_lower<<<(unsigned)zitems.size(), 256, 0, st>>>((const CbZeroItem*)(D + o_z), h->d_fronts, A);
     CK(cudaEventRecord(h->ev[1], st));
     // ---- assembly
-    k_front_rows<<<nw, 128, 0, st>>>(d_ids, nw, h->d_fronts, statics(h), A);
     if (!sitems.empty())
       k_scatter<<<(unsigned)sitems.size(), 256, 0, st>>>((const ScatterItem*)(D + o_s), h->d_fronts, statics(h), A,
                                                          d_vals, d_scal);
@@ -2887,11 +2954,10 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
       panel_used += panel_need; idx_used += idx_need; d_used += d_need;
       continue;
     }
-    k_get_counts<<<blocks_for(nw, 128), 128, 0, st>>>(d_ids, nw, h->d_fronts, (int32_t*)(D + o_cnt));
+    k_get_counts<<<blocks_for(nw, 128), 128, 0, st>>>(d_ids, nw, h->d_fronts, (int32_t*)(D + o_cnt), h->d_err);
     const size_t nlr = learned ? large_ids.size() : 0;  // the large fronts' routes after the growth check
     if ((rc = ensure_host((char*&)h->h_counts, h->h_counts_cap, (size_t)(3 * nw + 4 + nlr) * 4))) return rc;
-    CK(cudaMemcpyAsync(h->h_counts, D + o_cnt, (size_t)3 * nw * 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(h->h_counts + 3 * nw, h->d_err, 4, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(h->h_counts, D + o_cnt, (size_t)(3 * nw + 1) * 4, cudaMemcpyDeviceToHost, st));
     if (nlr) CK(cudaMemcpyAsync(h->h_counts + 3 * nw + 4, D + o_rt, nlr * 4, cudaMemcpyDeviceToHost, st));
     {
       double ts0 = now_ms();
@@ -2921,7 +2987,7 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
     }
     h->launches += 1 + (int64_t)eitems.size() * 0 + (sitems.empty() ? 0 : 1) +
                    n_small_launches + (witems.empty() ? 0 : 1) + (gitems.empty() ? 0 : 1) + 2 +
-                   (dly_ids.empty() ? 0 : 1) + (zitems.empty() ? 0 : 1);
+                   (zitems.empty() ? 0 : 1);
     for (size_t q = 0; q < maxch; ++q) h->launches += eitems[q].empty() ? 0 : 1;
     if (h->profiling) {  // the device memory in use (profiling runs only: the query costs host time)
       size_t fb = 0, tb = 0;
@@ -2965,7 +3031,23 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
 int finish_factor(rvg_handle* h, int64_t d_used) {
   cudaStream_t st = h->st;
   const int64_t ns = (int64_t)h->P.sn.size();
+  // aggregate stats (numeric.rs:929-1009)
+  h->tot1 = h->tot2 = h->totdel = h->zero_piv = h->max_front = 0;
+  h->inertia[0] = h->inertia[1] = h->inertia[2] = 0;
+  unsigned long long* hc = (unsigned long long*)h->h_norms;
+  if (d_used) {
+    if (!h->d_dcount) CK(cudaMalloc((void**)&h->d_dcount, 4 * sizeof(unsigned long long)));
+    CK(cudaMemsetAsync(h->d_dcount, 0, 4 * sizeof(unsigned long long), st));
+    const Arenas A{h->panel, h->idx, h->dtype, h->ddiag, h->doff, nullptr, h->cb_arena};
+    k_d_counts<<<(unsigned)std::min<int64_t>((ns + 7) / 8, 4 * h->nsm), 256, 0, st>>>(h->d_fronts, ns, A, h->d_dcount);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(hc, h->d_dcount, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+  }
   CK(cudaStreamSynchronize(st));
+  if (d_used) {
+    for (int q = 0; q < 3; ++q) h->inertia[q] = (int64_t)hc[q];
+    h->zero_piv = (int64_t)hc[3];
+  }
   float tot = 0;
   cudaEventElapsedTime(&tot, h->ev[0], h->ev[5]);
   h->t_factor = tot;
@@ -2975,21 +3057,10 @@ int finish_factor(rvg_handle* h, int64_t d_used) {
       cudaEventElapsedTime(&ms, h->ev_pool[e], h->ev_pool[e + 1]);
       h->syrk_ms += ms;
     }
-  // aggregate stats (numeric.rs:929-1009)
-  h->tot1 = h->tot2 = h->totdel = h->zero_piv = h->max_front = 0;
-  std::vector<int8_t> dt(d_used);
-  std::vector<double> dd(d_used);
-  if (d_used) {
-    CK(cudaMemcpy(dt.data(), h->dtype, d_used, cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(dd.data(), h->ddiag, d_used * 8, cudaMemcpyDeviceToHost));
-  }
   for (int64_t s = 0; s < ns; ++s) {
     const DFront& f = h->h_fronts[s];
     h->tot1 += f.n1; h->tot2 += f.n2; h->totdel += f.k - f.ne;
     h->max_front = std::max<int64_t>(h->max_front, f.m);
-    for (int c = 0; c < f.ne; ++c)
-      if (dt[f.dpos + c] == PT_1X1 && dd[f.dpos + c] == 0.0) h->zero_piv++;
-    if (f.parent < 0 && f.ne < f.m) h->zero_piv += f.k - f.ne;
   }
   h->factored = true;
   return RVG_OK;
@@ -3244,20 +3315,23 @@ static int factor_common(rvg_handle* h, const double* dv, const double* ds) {
   if (dv != h->d_vals && h->nnz) CK(cudaMemcpyAsync(h->d_vals, dv, h->nnz * 8, cudaMemcpyDeviceToDevice, h->st));
   // NaN or Inf in the values or the scaling: a clean InvalidInput before any factor kernel runs (the
   // reference rejects them in its MC64 scaling, ordering/matching.rs:143-157)
+  // (and ||A||_F from the same read)
+  h->a_fro = 0;
   if (h->nnz || (ds && h->P.n)) {
-    if (!h->d_nonfinite) CK(cudaMalloc((void**)&h->d_nonfinite, sizeof(int32_t)));
-    CK(cudaMemsetAsync(h->d_nonfinite, 0, sizeof(int32_t), h->st));
-    if (h->nnz) k_nonfinite<<<296, 256, 0, h->st>>>(h->d_vals, h->nnz, h->d_nonfinite);
-    if (ds && h->P.n) k_nonfinite<<<296, 256, 0, h->st>>>(ds, h->P.n, h->d_nonfinite);
+    if (!h->d_scan) CK(cudaMalloc((void**)&h->d_scan, sizeof(ScanOut)));
+    CK(cudaMemsetAsync(h->d_scan, 0, sizeof(ScanOut), h->st));
+    if (h->nnz) k_scan_values<<<296, 256, 0, h->st>>>(h->d_vals, h->nnz, h->d_scan, 1);
+    if (ds && h->P.n) k_scan_values<<<296, 256, 0, h->st>>>(ds, h->P.n, h->d_scan, 0);
     CK(cudaGetLastError());
-    int32_t bad = 0;
-    CK(cudaMemcpyAsync(&bad, h->d_nonfinite, 4, cudaMemcpyDeviceToHost, h->st));
+    const ScanOut* sc = (const ScanOut*)h->h_norms;
+    CK(cudaMemcpyAsync(h->h_norms, h->d_scan, sizeof(ScanOut), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
-    if (bad) {
+    if (sc->bad) {
       h->factored = false;
       set_error("the matrix values or the scaling contain NaN or Inf");
       return RVG_ERR_INVALID_INPUT;
     }
+    h->a_fro = std::sqrt(sc->sum);
   }
   bool done = false;
   if (h->opt.graph_refactor && h->rec_ok && h->opt.precision != 2) {
@@ -3277,14 +3351,6 @@ static int factor_common(rvg_handle* h, const double* dv, const double* ds) {
     h->sel_flagged = flagged;
     h->sel_fallback = h->sel_refactored;
   }
-  double* d_acc = nullptr;
-  CK(cudaMallocAsync((void**)&d_acc, 8, h->st));
-  CK(cudaMemsetAsync(d_acc, 0, 8, h->st));
-  if (h->nnz) k_sumsq<<<296, 256, 0, h->st>>>(h->d_vals, h->nnz, d_acc);
-  CK(cudaMemcpyAsync(h->h_norms, d_acc, 8, cudaMemcpyDeviceToHost, h->st));
-  CK(cudaFreeAsync(d_acc, h->st));
-  CK(cudaStreamSynchronize(h->st));
-  h->a_fro = std::sqrt(h->h_norms[0]);
   return RVG_OK;
 }
 
@@ -3805,36 +3871,7 @@ rvg_status rvg_solve_refine_nrhs(rvg_handle* h, const double* rhs, double* x, in
 rvg_status rvg_inertia(rvg_handle* h, int64_t out3[3]) {
   if (!h) { set_error("null handle"); return RVG_ERR_INVALID_INPUT; }
   if (!h->factored) { set_error("factor() must be called first"); return RVG_ERR_SOLVE_BEFORE_FACTOR; }
-  int64_t pos = 0, neg = 0, zer = 0;
-  int64_t tot = 0;
-  for (auto& f : h->h_fronts) tot = std::max<int64_t>(tot, f.dpos + f.k);
-  std::vector<int8_t> dt(tot);
-  std::vector<double> dd(tot), dof(tot);
-  if (tot) {
-    CK(cudaMemcpy(dt.data(), h->dtype, tot, cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(dd.data(), h->ddiag, tot * 8, cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(dof.data(), h->doff, tot * 8, cudaMemcpyDeviceToHost));
-  }
-  // MixedDiagonal::compute_inertia (diagonal.rs:391-461) per front
-  for (auto& f : h->h_fronts) {
-    int c = 0;
-    while (c < f.ne) {
-      int64_t q = f.dpos + c;
-      if (dt[q] == PT_1X1) {
-        double d = dd[q];
-        if (d > 0) pos++; else if (d < 0) neg++; else zer++;
-        c += 1;
-      } else {
-        double a = dd[q], b = dof[q], cc = dd[q + 1];
-        double det = a * cc - b * b, tr = a + cc;
-        if (det > 0) { if (tr > 0) pos += 2; else neg += 2; }
-        else if (det < 0) { pos++; neg++; }
-        else { if (tr > 0) { pos++; zer++; } else if (tr < 0) { neg++; zer++; } else zer += 2; }
-        c += 2;
-      }
-    }
-  }
-  out3[0] = pos; out3[1] = neg; out3[2] = zer;
+  for (int q = 0; q < 3; ++q) out3[q] = h->inertia[q];
   return RVG_OK;
 }
 
@@ -4140,7 +4177,8 @@ void rvg_destroy(rvg_handle* h) {
   if (h->d_sel) cudaFree(h->d_sel);
   fr(h->d_feat);
   if (h->d_sel_flag) cudaFree(h->d_sel_flag);
-  if (h->d_nonfinite) cudaFree(h->d_nonfinite);
+  if (h->d_scan) cudaFree(h->d_scan);
+  if (h->d_dcount) cudaFree(h->d_dcount);
   if (h->d_mismatch) cudaFree(h->d_mismatch);
   if (h->h_stage_all) cudaFreeHost(h->h_stage_all);
   for (size_t t = 0; t < h->lfx.size(); ++t) {

@@ -53,8 +53,9 @@ typedef struct {
   /* B200 scheduling, no reference counterpart: fronts of order >= this use
    * the multi-kernel path (whole GPU per front), and so do fronts of at least
    * half this order in a wave that holds at most 16 of them; the others are
-   * batched one CTA or warp per front.  Results do not depend on it.
-   * Default 2048. */
+   * batched one CTA or warp per front, except the few (of order >= a 16th of
+   * this) whose single CTA would hold the wave up: those take the multi-kernel
+   * path too, in FP64.  Results do not depend on it.  Default 2048. */
   int64_t large_front_threshold;
   /* Arithmetic of the large Schur-complement updates, no reference
    * counterpart: 0 = plain FP64 (tensor-core DMMA, bit-identical to the CPU

@@ -98,10 +98,10 @@ struct WarpTpp {
   int64_t m, nc;
   int lane;
 
-  __device__ double sym(int64_t row, int64_t col) const {  // factor.rs:2597-2606
+  __device__ __forceinline__ double sym(int64_t row, int64_t col) const {  // factor.rs:2597-2606
     return (col < nc && row >= col) ? a(row, col) : a(col, row);
   }
-  __device__ bool col_small(int64_t idx, int64_t from, int64_t to, double small) const {  // 2674-2690
+  __device__ __forceinline__ bool col_small(int64_t idx, int64_t from, int64_t to, double small) const {  // 2674-2690
     bool big = false;
     int64_t ce = idx < nc ? idx : nc;
     for (int64_t c = from + lane; c < ce; c += 32) big |= fabs(a(idx, c)) >= small;
@@ -109,7 +109,7 @@ struct WarpTpp {
       for (int64_t r = idx + lane; r < to; r += 32) big |= fabs(a(r, idx)) >= small;
     return !__any_sync(0xffffffffu, big);
   }
-  __device__ int64_t row_abs_max(int64_t p, int64_t from, int64_t to) const {  // 2695-2710
+  __device__ __forceinline__ int64_t row_abs_max(int64_t p, int64_t from, int64_t to) const {  // 2695-2710
     if (from >= to) return from;
     double bv = -1.0;
     int64_t bk = INT64_MAX;
@@ -120,7 +120,7 @@ struct WarpTpp {
     warp_argmax(bv, bk);
     return bk;
   }
-  __device__ double rc_abs_max_excl(int64_t col, int64_t nelim, int64_t excl) const {  // 2715-2737
+  __device__ __forceinline__ double rc_abs_max_excl(int64_t col, int64_t nelim, int64_t excl) const {  // 2715-2737
     double best = 0.0;
     int64_t ce = col < nc ? col : nc;
     for (int64_t c = nelim + lane; c < ce; c += 32) if (c != excl) best = fmax(best, fabs(a(col, c)));
@@ -128,7 +128,7 @@ struct WarpTpp {
       for (int64_t r = col + 1 + lane; r < m; r += 32) if (r != excl) best = fmax(best, fabs(a(r, col)));
     return warp_max(best);
   }
-  __device__ bool test_2x2(int64_t t, int64_t p, double maxt, double maxp, double u, double small) const {
+  __device__ __forceinline__ bool test_2x2(int64_t t, int64_t p, double maxt, double maxp, double u, double small) const {
     double a11 = a(t, t), a21 = a(p, t), a22 = a(p, p);  // factor.rs:2268-2315
     double maxpiv = fmax(fmax(fabs(a11), fabs(a21)), fabs(a22));
     if (maxpiv < small) return false;

@@ -7,7 +7,8 @@
 
 namespace rvg {
 
-enum : int32_t { FF_SMALL_LEAF = 1, FF_HAS_CB = 2, FF_HAS_PARENT = 4, FF_LARGE = 8 };
+enum : int32_t { FF_SMALL_LEAF = 1, FF_HAS_CB = 2, FF_HAS_PARENT = 4, FF_LARGE = 8,
+                FF_ROUTED = 16 };  // a medium front on the large fronts' path (always in FP64)
 
 struct DFront {
   int64_t panel;    // offset (doubles) in the panel arena, ld = m

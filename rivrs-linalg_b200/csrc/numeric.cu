@@ -1246,6 +1246,7 @@ struct rvg_handle {
   int device = 0;
   cudaStream_t st = nullptr;
   cudaEvent_t ev[8] = {};
+  cudaEvent_t ev_large = nullptr, ev_beside = nullptr;  // forks and joins of the large fronts' streams
   int64_t nnz = 0;
   // static device data
   int64_t *d_own_ptr = nullptr, *d_pat_ptr = nullptr, *d_amap_ptr = nullptr, *d_ea_ptr = nullptr, *d_ch_ptr = nullptr;
@@ -1815,6 +1816,54 @@ inline bool front_is_large(int64_t m, bool tpp, int64_t T, int64_t mid) {
   return !tpp && (m >= T || (m >= T / 2 && mid <= LF_FEW));
 }
 
+// Medium fronts that would hold a wave up on one CTA go to the large fronts'
+// path (results do not depend on it).  One CTA's time grows with the front's
+// trailing tiles, the whole GPU's hardly: measured for one dense front of order
+// n (B200), 128: 130 / 103 us, 256: 366 / 253, 512: 1525 / 630, 1000: 7300 /
+// 1540, which the two models below follow.  The queue runs all its fronts at
+// once, the large path up to `ctx` at a time beside it, each further one with a
+// host thread to start: the j longest fronts move where that makes the longer of
+// the two shortest, and only if it saves a tenth.  Only fronts of order >= T / 16
+// (128 at the default threshold) count, so the threshold still turns the path
+// off; they keep the FP64 updates in every precision.
+constexpr int LF_ROUTED_MAX = 16;
+double cta_front_us(double m, double k) {
+  double t = 0;
+  for (double c = 32; c < k + 32; c += 32) {
+    const double cols = std::max(0.0, k - c), rows = std::max(0.0, m - c);
+    t += 28 + rows / 40 + 1.2 * cols * (rows - cols / 2) / 1024;
+  }
+  return t;
+}
+double lf_front_us(double m, double k, double nb) {
+  return std::ceil(k / 32) * (24 + m / 60) + 60 * std::ceil(k / nb) + 20;
+}
+// the positions in mk (order, fully-summed columns) of the fronts to move
+std::vector<int> route_medium(const std::vector<std::pair<int64_t, int64_t>>& mk, int64_t T, int64_t nb) {
+  std::vector<std::pair<double, int>> c;
+  for (int i = 0; i < (int)mk.size(); ++i) c.emplace_back(cta_front_us((double)mk[i].first, (double)mk[i].second), i);
+  const int top = (int)std::min<size_t>(c.size(), LF_ROUTED_MAX + 1);
+  std::partial_sort(c.begin(), c.begin() + top, c.end(), [](const auto& a, const auto& b) {
+    return a.first > b.first || (a.first == b.first && a.second < b.second);
+  });
+  const int ctx = LF_CONCURRENT - 1;
+  int best = 0;
+  double best_t = c.empty() ? 0 : 0.9 * c[0].first, sum = 0, longest = 0;
+  for (int j = 1; j <= (int)std::min<size_t>(c.size(), LF_ROUTED_MAX); ++j) {
+    const auto& f = mk[c[j - 1].second];
+    if (f.first < T / 16) break;
+    const double l = lf_front_us((double)f.first, (double)f.second, (double)nb);
+    sum += l;
+    longest = std::max(longest, l);
+    const double lf = std::max(longest, sum / std::min(j, ctx)) + 15 + 25 * (std::min(j, ctx) - 1);
+    const double t = std::max(lf, j < (int)c.size() ? c[j].first : 0.0);
+    if (t < best_t) { best_t = t; best = j; }
+  }
+  std::vector<int> out;
+  for (int j = 0; j < best; ++j) out.push_back(c[j].second);
+  return out;
+}
+
 // Arena sizes of the delay-free schedule, computed from the pattern alone
 // (delays can only add to them; the arenas grow in that case).
 int presize_arenas(rvg_handle* h) {
@@ -1830,6 +1879,16 @@ int presize_arenas(rvg_handle* h) {
       const int64_t k = x.n_owned(), m = k + (int64_t)x.pattern.size();
       if (!(x.in_small_leaf || k < ib) && m >= T / 2 && m < T) ++mid;
     }
+    std::vector<std::pair<int64_t, int64_t>> med;
+    std::vector<int64_t> med_s;
+    for (int64_t s : P.waves[w]) {
+      const Snode& x = P.sn[s];
+      const int64_t k = x.n_owned(), m = k + (int64_t)x.pattern.size();
+      const bool tpp = x.in_small_leaf || k < ib;
+      if (!tpp && !front_is_large(m, tpp, T, mid)) { med.emplace_back(m, k); med_s.push_back(s); }
+    }
+    std::vector<int64_t> routed;
+    for (int i : route_medium(med, T, nb)) routed.push_back(med_s[i]);
     for (int64_t s : P.waves[w]) {
       const Snode& x = P.sn[s];
       int64_t k = x.n_owned(), nfs = (int64_t)x.pattern.size(), m = k + nfs;
@@ -1841,7 +1900,8 @@ int presize_arenas(rvg_handle* h) {
       bool tpp = x.in_small_leaf || k < ib;
       bool large = front_is_large(m, tpp, T, mid);
       int64_t sc = tpp ? 0 : (2 * IBMAX * m + nb);
-      if (large) sc = m * (2 * IBMAX + lf_window_blocks(h) * nb) + nb;
+      if (large || std::find(routed.begin(), routed.end(), s) != routed.end())
+        sc = m * (2 * IBMAX + lf_window_blocks(h) * nb) + nb;
       if (has_cb && large) sc = std::max<int64_t>(sc, nfs * k);  // k_cb_w
       sc_w += sc;
       if (x.parent >= 0) rel[w] = std::max<int64_t>(rel[w], P.height[x.parent]);
@@ -1972,6 +2032,7 @@ static void launch_pack(rvg_handle* h, cudaStream_t st, dim3 grid, const PackArg
 // Whether front s takes the mixed form's tensor-core updates: every large
 // front with precision = 1, the selector's choice with precision = 2.
 bool front_mixed(const rvg_handle* h, int64_t s) {
+  if (h->h_fronts[s].flags & FF_ROUTED) return false;
   if (h->opt.precision == 1) return true;
   if (h->opt.precision != 2 || h->sel_force_fp64) return false;
   return s >= 0 && s < (int64_t)h->route.size() && h->route[s] != 0;
@@ -2411,8 +2472,12 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
 // The large fronts of one wave: one after another on the handle's stream when
 // there is one (profiling marks on), otherwise up to LF_CONCURRENT at a time,
 // each context's fronts in turn on its own host thread and stream, ordered
-// after the wave's assembly and before what follows by events.
-int factor_large_fronts(rvg_handle* h, const std::vector<int32_t>& ids, const Arenas& A, const DevOpts& dop) {
+// after the wave's assembly and before what follows by events.  beside: the
+// event behind the assembly when the wave's small and medium fronts are queued
+// on the handle's stream meanwhile; the large ones then use the other
+// contexts' streams only and run beside them.
+int factor_large_fronts(rvg_handle* h, const std::vector<int32_t>& ids, const Arenas& A, const DevOpts& dop,
+                        cudaEvent_t beside = nullptr) {
   if (ids.empty()) return RVG_OK;
   if (h->lfx.empty()) {
     h->lfx.resize(1);
@@ -2430,7 +2495,8 @@ int factor_large_fronts(rvg_handle* h, const std::vector<int32_t>& ids, const Ar
   };
   // (a capture forks into the same contexts with the fronts dealt the same way:
   // the replayed graph runs them concurrently on the buffers the dynamic run sized)
-  const int nc = (int)std::min<size_t>(ids.size(), LF_CONCURRENT);
+  const int first = beside ? 1 : 0;  // the first context used
+  const int nc = (int)std::min<size_t>(ids.size() + first, LF_CONCURRENT);
   while ((int)h->lfx.size() < nc) {  // grown before any reference into lfx is taken
     if (tl_no_alloc) return no_alloc_fail();
     LfCtx c;
@@ -2443,7 +2509,7 @@ int factor_large_fronts(rvg_handle* h, const std::vector<int32_t>& ids, const Ar
   LfCtx& c0 = h->lfx[0];
   c0.wpack = h->wpack; c0.wpack_cap = h->wpack_cap;
   int rc = RVG_OK;
-  if (nc == 1) {
+  if (nc == 1 && !beside) {
     c0.marks = true;
     for (int32_t s : ids)
       if ((rc = factor_large_front(h, c0, s, A, dop))) break;
@@ -2452,10 +2518,13 @@ int factor_large_fronts(rvg_handle* h, const std::vector<int32_t>& ids, const Ar
     return rc;
   }
   mark(h, -1);
-  cudaEvent_t ready;
-  CK(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
-  CK(cudaEventRecord(ready, h->st));
-  for (int t = 1; t < nc; ++t) CK(cudaStreamWaitEvent(h->lfx[t].st, ready, 0));
+  cudaEvent_t ready = h->ev_large;
+  if (!ready) {
+    CK(cudaEventCreateWithFlags(&h->ev_large, cudaEventDisableTiming));
+    ready = h->ev_large;
+  }
+  if (!beside) CK(cudaEventRecord(ready, h->st));
+  for (int t = 1; t < nc; ++t) CK(cudaStreamWaitEvent(h->lfx[t].st, beside ? beside : ready, 0));
   std::vector<int> rcs(nc, RVG_OK);
   std::vector<std::string> errs(nc);
   const bool no_alloc = tl_no_alloc;
@@ -2465,22 +2534,21 @@ int factor_large_fronts(rvg_handle* h, const std::vector<int32_t>& ids, const Ar
     tl_no_alloc = no_alloc;
     LfCtx& c = h->lfx[t];
     c.marks = false;
-    for (size_t i = t; i < ids.size(); i += nc)
+    for (size_t i = t - first; i < ids.size(); i += nc - first)
       if ((rcs[t] = factor_large_front(h, c, ids[i], A, dop))) { errs[t] = g_err; break; }
     tl_no_alloc = was;
   };
   std::vector<std::thread> th;
-  for (int t = 1; t < nc; ++t) th.emplace_back(work, t);
-  work(0);
+  for (int t = first + 1; t < nc; ++t) th.emplace_back(work, t);
+  work(first);
   for (auto& x : th) x.join();
   h->wpack = c0.wpack; h->wpack_cap = c0.wpack_cap;
   for (int t = 1; t < nc; ++t) {
     CK(cudaEventRecord(ready, h->lfx[t].st));
     CK(cudaStreamWaitEvent(h->st, ready, 0));
   }
-  CK(cudaEventDestroy(ready));
   mark(h, RVG_PART_OTHER);
-  for (int t = 0; t < nc; ++t) {
+  for (int t = first; t < nc; ++t) {
     fold(h->lfx[t]);
     if (rcs[t] && !rc) { rc = rcs[t]; set_error(errs[t]); }
   }
@@ -2715,14 +2783,23 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
         const DFront& f = h->h_fronts[s];
         if (!((f.flags & FF_SMALL_LEAF) || f.k < ib) && f.m >= T / 2 && f.m < T) ++mid;
       }
+      std::vector<std::pair<int64_t, int64_t>> med;
+      std::vector<int64_t> med_s;
+      for (int64_t s : wave) {
+        DFront& f = h->h_fronts[s];
+        const bool tpp = (f.flags & FF_SMALL_LEAF) || f.k < ib;
+        if (front_is_large(f.m, tpp, T, mid)) f.flags |= FF_LARGE;
+        else if (!tpp) { med.emplace_back(f.m, f.k); med_s.push_back(s); }
+      }
+      for (int i : route_medium(med, T, h->opt.outer_block_size)) h->h_fronts[med_s[i]].flags |= FF_ROUTED;
       for (int64_t s : wave) {
         DFront& f = h->h_fronts[s];
         const int64_t m = f.m, k = f.k, nfs = f.nfs;
         const bool tpp = (f.flags & FF_SMALL_LEAF) || k < ib;
-        const bool large = front_is_large(m, tpp, T, mid);
-        if (large) f.flags |= FF_LARGE;
+        const bool large = (f.flags & FF_LARGE) != 0;
         int64_t sc = tpp ? 0 : (2 * IBMAX * m + h->opt.outer_block_size);
-        if (large) sc = m * (2 * IBMAX + lf_window_blocks(h) * h->opt.outer_block_size) + h->opt.outer_block_size;
+        if (large || (f.flags & FF_ROUTED))
+          sc = m * (2 * IBMAX + lf_window_blocks(h) * h->opt.outer_block_size) + h->opt.outer_block_size;
         if ((f.flags & FF_HAS_CB) && large) sc = std::max<int64_t>(sc, nfs * k);  // k_cb_w
         f.scratch = scratch_need; scratch_need += sc;
       }
@@ -2756,7 +2833,7 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
     if (panel_need) CK(cudaMemsetAsync(h->panel + panel_used, 0, (size_t)panel_need * 8, st));
     const Arenas A{h->panel, h->idx, h->dtype, h->ddiag, h->doff, scratch, h->cb_arena};
     // ---- launch data of the whole wave, packed into one upload
-    std::vector<int32_t> ids(wave.begin(), wave.end()), tpp_ids, aptp_ids, large_ids;
+    std::vector<int32_t> ids(wave.begin(), wave.end()), tpp_ids, aptp_ids, large_ids, routed_ids;
     std::vector<DFront> staged;
     staged.reserve(nw);
     for (int64_t s : wave) {
@@ -2764,6 +2841,7 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
       const DFront& f = h->h_fronts[s];
       if ((f.flags & FF_SMALL_LEAF) || f.k < ib) tpp_ids.push_back((int32_t)s);
       else if (f.flags & FF_LARGE) large_ids.push_back((int32_t)s);
+      else if (f.flags & FF_ROUTED) routed_ids.push_back((int32_t)s);
       else aptp_ids.push_back((int32_t)s);
     }
     // medium fronts largest first (dense work ~ k m^2): the persistent launch starts the long ones early
@@ -2876,6 +2954,14 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
     }
     // ---- dense factorization
     mark(h, -1);
+    // large fronts beside the small and medium ones (one after the other while the profiling marks are on)
+    std::vector<int32_t> lf_ids(large_ids);
+    lf_ids.insert(lf_ids.end(), routed_ids.begin(), routed_ids.end());
+    const bool beside = !lf_ids.empty() && !(aptp_ids.empty() && tpp_ids.empty()) && !h->profiling;
+    if (beside) {
+      if (!h->ev_beside) CK(cudaEventCreateWithFlags(&h->ev_beside, cudaEventDisableTiming));
+      CK(cudaEventRecord(h->ev_beside, st));
+    }
     // the wave's small and medium fronts (profiling: part "aptp")
     bool group = false;  // a launch of the group has gone out: the next ones may start beside it
     if (!aptp_ids.empty()) {
@@ -2908,7 +2994,7 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
       }
       h->sel_large.insert(h->sel_large.end(), large_ids.begin(), large_ids.end());
     }
-    if ((rc = factor_large_fronts(h, large_ids, A, dop))) return rc;
+    if ((rc = factor_large_fronts(h, lf_ids, A, dop, beside ? h->ev_beside : nullptr))) return rc;
     CK(cudaEventRecord(h->ev[3], st));
     // ---- contribution GEMM (fronts with nothing eliminated skip inside)
     mark(h, -1);
@@ -4205,6 +4291,8 @@ void rvg_destroy(rvg_handle* h) {
   for (auto e : h->ev_pool) cudaEventDestroy(e);
   for (auto e : h->mk_pool) cudaEventDestroy(e);
   for (auto& e : h->ev) if (e) cudaEventDestroy(e);
+  if (h->ev_large) cudaEventDestroy(h->ev_large);
+  if (h->ev_beside) cudaEventDestroy(h->ev_beside);
   delete h;
   cudaGetLastError();  // nothing of this handle's teardown is left for the caller's next call to report
 }

@@ -53,8 +53,23 @@ def test_small_leaf_fronts(rv, orc, k, kind):
 # 32-column blocks with and without a remainder, panels and tiles of 32 rows and one more or less
 @pytest.mark.parametrize("k,r", [(32, 1), (33, 31), (63, 32), (64, 33), (65, 100), (97, 64), (300, 37)])
 @pytest.mark.parametrize("kind", ["plain", "delay", "zero"])
-def test_medium_fronts(rv, orc, k, r, kind):
-    check(rv, orc, k, r, kind, small_leaf_threshold=0)
+@pytest.mark.parametrize("threshold", [2048, 10 ** 6])  # the second keeps every front on its own CTA
+def test_medium_fronts(rv, orc, k, r, kind, threshold):
+    check(rv, orc, k, r, kind, small_leaf_threshold=0, large_front_threshold=threshold)
+
+
+# the medium fronts that take the large fronts' path keep FP64 updates in the mixed form
+def test_routed_fronts_stay_fp64(rv):
+    s = arrow_system(rv, 450, 60, 3, "plain")
+    order = np.arange(s.n, dtype=np.int64)
+    rec = []
+    for precision in ("fp64", "mixed"):
+        solver = rv.SparseLDLT.analyze(s, rv.AnalyzeOptions(rv.OrderingStrategy.USER_SUPPLIED, order))
+        solver.factor(None, rv.FactorOptions(precision=precision))
+        rec.append(solver.pivot_record())
+        solver.close()
+    for a, b in zip(*rec):
+        assert np.array_equal(a, b)
 
 
 @pytest.mark.parametrize("ib,nb", [(8, 32), (17, 64), (32, 96)])

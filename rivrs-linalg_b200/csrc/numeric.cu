@@ -1278,7 +1278,15 @@ struct rvg_handle {
   float* pack = nullptr; size_t pack_cap = 0;        // TF32 hi/lo operand tiles of the mixed-form updates
   float* wpack = nullptr; size_t wpack_cap = 0;      // the same for a large front's window of pending columns
   int32_t* d_err = nullptr;                          // set by a device wait that timed out
-  int32_t* sf_sync = nullptr; size_t sf_sync_cap = 0; // solve: ticket counter and block flags of one wave
+  int32_t* sf_sync = nullptr; size_t sf_sync_cap = 0; // solve: ticket counters and block flags of all waves
+  // solve: block layout of the factored fronts, made by the first solve after a factorization
+  struct SfLayout {
+    bool ok = false;
+    struct Wave { size_t fwd, bwd, mfwd, mbwd; int32_t nbf, nbb; int64_t tf, tb; };  // offsets in the buffer and sf_sync
+    std::vector<Wave> w;
+    int64_t nsync = 0, slots = 1, rows = 0;  // sf_sync words, partial-sum slots, rows of all fronts
+  } sf;
+  char* sf_lay = nullptr; size_t sf_lay_cap = 0;
   double* sf_part = nullptr; size_t sf_part_cap = 0;   // backward solve: partial sums of one wave
   int nsm = 0;                                       // SMs of the device (persistent grids)
   bool chain_pdl = true;                             // large-front chain kernels by programmatic dependent launch
@@ -3392,6 +3400,7 @@ static int replay_factor(rvg_handle* h, const double* ds, bool* done) {
 
 static int factor_common(rvg_handle* h, const double* dv, const double* ds) {
   int rc;
+  h->sf.ok = false;  // the solve's layout is the last factorization's
   if (h->need_presize) {  // after rvg_trim: the arenas at their delay-free size again
     if ((rc = presize_arenas(h))) return rc;
     if (h->vm && (rc = vm_restore(h))) return rc;  // (address-stable: up to their largest size, all of them)
@@ -3473,12 +3482,70 @@ static int device_wait_status(rvg_handle* h) {
   return RVG_OK;
 }
 
+// The block layout of the factored fronts for the solve kernels: per wave, the
+// forward blocks (diagonal, then L21, per front) and the backward tickets
+// (gathers, partial sums, column blocks), the front of every ticket, and the
+// fronts' offsets in the solve workspace (DFront::scratch: rows before it).
+// Valid until the next factorization or rvg_trim.
+static int sf_make_layout(rvg_handle* h) {
+  const Plan& P = h->P;
+  cudaStream_t st = h->st;
+  rvg_handle::SfLayout& Y = h->sf;
+  Y = rvg_handle::SfLayout();
+  std::vector<DFront> fr = h->h_fronts;
+  for (auto& f : fr) { f.scratch = Y.rows; Y.rows += f.m; }
+  Packer pk;
+  const size_t o_fr = pk.add(fr);
+  for (size_t w = 0; w < P.waves.size(); ++w) {
+    std::vector<SfFront> vf, vb;
+    std::vector<int32_t> mf, mb;
+    int32_t slots = 0;
+    rvg_handle::SfLayout::Wave v{};
+    for (int64_t s : P.waves[w]) {
+      const DFront& f = fr[s];
+      if (f.ne == 0) continue;
+      const int32_t nbd = (f.ne + SF_B - 1) / SF_B, nbr = (f.m - f.ne + SF_B - 1) / SF_B;
+      const int32_t ngrp = (nbr + SF_PG - 1) / SF_PG;
+      const int32_t at = (int32_t)vf.size();
+      vf.push_back(SfFront{(int32_t)s, v.nbf, nbd, nbr, 0, 0});
+      vb.push_back(SfFront{(int32_t)s, v.nbb, nbd, nbr, ngrp, slots});
+      v.nbf += nbd + nbr;
+      v.nbb += nbr + nbd * ngrp + nbd;  // gathers, partial sums, column blocks
+      mf.resize(v.nbf, at);
+      mb.resize(v.nbb, at);
+      slots += nbd * ngrp;
+    }
+    Y.slots = std::max<int64_t>(Y.slots, slots);
+    v.fwd = pk.add(vf);
+    v.bwd = pk.add(vb);
+    v.mfwd = pk.add(mf);
+    v.mbwd = pk.add(mb);
+    v.tf = Y.nsync;
+    Y.nsync += 1;  // the forward blocks need a ticket counter only
+    v.tb = Y.nsync;
+    Y.nsync += 1 + v.nbb;
+    Y.w.push_back(v);
+  }
+  int rc;
+  if ((rc = ensure_nocopy(h->sf_lay, h->sf_lay_cap, pk.buf.size() + 16, st))) return rc;
+  // through the pinned buffer when it is large enough as it is: growing it would cost more than the copy
+  const char* src = pk.buf.data();
+  if (pk.buf.size() <= h->h_stage_cap && h->h_stage) {
+    std::memcpy(h->h_stage, src, pk.buf.size());
+    src = h->h_stage;
+  }
+  CK(cudaMemcpyAsync(h->sf_lay, src, pk.buf.size(), cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(h->d_fronts, h->sf_lay + o_fr, fr.size() * sizeof(DFront), cudaMemcpyDeviceToDevice, st));
+  CK(cudaStreamSynchronize(st));  // the source is free again
+  Y.ok = true;
+  return RVG_OK;
+}
+
 // aptp_solve (solve.rs:57-326) with the permutation and scaling of
 // SparseLDLT::solve_in_place (solver.rs:396-425): per wave one forward launch
 // (leaves first) and, in reverse, one backward launch of solve_sf.cuh.
 static int solve_common(rvg_handle* h, double* d_rhs, int64_t nrhs, int64_t ldb) {
-  Plan& P = h->P;
-  const int64_t n = P.n;
+  const int64_t n = h->P.n;
   cudaStream_t st = h->st;
   if (n == 0 || nrhs == 0) return RVG_OK;
   // right-hand sides per pass: 8, 4, 2 or 1.  A pass costs the factor's read
@@ -3490,12 +3557,14 @@ static int solve_common(rvg_handle* h, double* d_rhs, int64_t nrhs, int64_t ldb)
   const int64_t npad = nrhs / 8 * 8 + pass(nrhs % 8);
   int rc = ensure(h->d_x, h->x_cap, (size_t)(n * npad), st);
   if (rc) return rc;
+  if (!h->sf.ok && (rc = sf_make_layout(h))) return rc;
+  const rvg_handle::SfLayout& Y = h->sf;
+  const size_t nw = Y.w.size();
   // the per-front solve workspace: forward results, then final values (R x m each)
-  int64_t wneed = 0;
-  std::vector<DFront> fr = h->h_fronts;
-  for (auto& f : fr) { f.scratch = wneed; wneed += 2 * (int64_t)rmax * f.m; }
+  const int64_t wneed = 2 * (int64_t)rmax * Y.rows;
   if ((rc = ensure(h->solve_work, h->solve_work_cap, (size_t)std::max<int64_t>(wneed, 1), st))) return rc;
-  CK(cudaMemcpyAsync(h->d_fronts, fr.data(), fr.size() * sizeof(DFront), cudaMemcpyHostToDevice, st));
+  if ((rc = ensure(h->sf_sync, h->sf_sync_cap, (size_t)std::max<int64_t>(Y.nsync, 1), st))) return rc;
+  if ((rc = ensure_nocopy(h->sf_part, h->sf_part_cap, (size_t)Y.slots * 8 * SF_B, st))) return rc;
   Arenas A{h->panel, h->idx, h->dtype, h->ddiag, h->doff, nullptr, h->cb_arena};
   CK(cudaEventRecord(h->ev[6], st));
   int64_t launches = 0;
@@ -3504,60 +3573,28 @@ static int solve_common(rvg_handle* h, double* d_rhs, int64_t nrhs, int64_t ldb)
                                                                  h->has_scaling ? h->d_scal : nullptr);
   launches++;
   if (npad > nrhs) CK(cudaMemsetAsync(h->d_x + n * nrhs, 0, (size_t)(n * (npad - nrhs)) * 8, st));
-  // block layout of every wave: forward (diagonal then L21 blocks per front) and backward (diagonal blocks)
-  const size_t nw = P.waves.size();
-  Packer pk;
-  std::vector<size_t> offf(nw), offb(nw);
-  std::vector<int32_t> nfr(nw, 0), nbf(nw, 0), nbb(nw, 0);
-  int32_t maxblk = 1;
-  int64_t maxslots = 1;
-  for (size_t w = 0; w < nw; ++w) {
-    std::vector<SfFront> vf, vb;
-    int32_t slots = 0;
-    for (int64_t s : P.waves[w]) {
-      const DFront& f = fr[s];
-      if (f.ne == 0) continue;
-      const int32_t nbd = (f.ne + SF_B - 1) / SF_B, nbr = (f.m - f.ne + SF_B - 1) / SF_B;
-      const int32_t ngrp = (nbr + SF_PG - 1) / SF_PG;
-      vf.push_back(SfFront{(int32_t)s, nbf[w], nbd, nbr, 0, 0});
-      vb.push_back(SfFront{(int32_t)s, nbb[w], nbd, nbr, ngrp, slots});
-      nbf[w] += nbd + nbr;
-      nbb[w] += nbr + nbd * ngrp + nbd;  // gathers, partial sums, column blocks
-      slots += nbd * ngrp;
-    }
-    maxslots = std::max<int64_t>(maxslots, slots);
-    nfr[w] = (int32_t)vf.size();
-    offf[w] = pk.add(vf);
-    offb[w] = pk.add(vb);
-    maxblk = std::max(maxblk, std::max(nbf[w], nbb[w]));
-  }
-  if ((rc = arena_ensure(h, VM_STAGE, h->d_stage, h->stage_cap, pk.buf.size() + 16, st, true))) return rc;
-  if ((rc = ensure_host(h->h_stage, h->h_stage_cap, pk.buf.size() + 16))) return rc;
-  std::memcpy(h->h_stage, pk.buf.data(), pk.buf.size());
-  CK(cudaMemcpyAsync(h->d_stage, h->h_stage, pk.buf.size(), cudaMemcpyHostToDevice, st));
-  if ((rc = ensure(h->sf_sync, h->sf_sync_cap, (size_t)maxblk + 1, st))) return rc;
-  if ((rc = ensure_nocopy(h->sf_part, h->sf_part_cap, (size_t)maxslots * 8 * SF_B, st))) return rc;
   auto wave = [&](size_t w, bool fwd, int64_t rh) {
+    const rvg_handle::SfLayout::Wave& v = Y.w[w];
     SfWave sw;
     sw.part = h->sf_part;
-    sw.fr = (const SfFront*)(h->d_stage + (fwd ? offf[w] : offb[w]));
-    sw.nfr = nfr[w];
-    sw.nblk = fwd ? nbf[w] : nbb[w];
-    sw.ticket = h->sf_sync;
-    sw.flags = h->sf_sync + 1;
+    sw.fr = (const SfFront*)(h->sf_lay + (fwd ? v.fwd : v.bwd));
+    sw.fmap = (const int32_t*)(h->sf_lay + (fwd ? v.mfwd : v.mbwd));
+    sw.nblk = fwd ? v.nbf : v.nbb;
+    sw.ticket = h->sf_sync + (fwd ? v.tf : v.tb);
+    sw.flags = sw.ticket + 1;
     sw.x = h->d_x + rh * n;
     sw.ldx = n;
     sw.work = h->solve_work;
     sw.err = h->d_err;
     return sw;
   };
-  auto fwd = [&](int r, size_t w, const SfWave& sw) {
-    const unsigned g = (unsigned)std::min<int64_t>(nbf[w], 16LL * h->nsm);
+  auto fwd = [&](int r, const SfWave& sw) {
+    const dim3 g((unsigned)std::min<int64_t>(sw.nblk, 16LL * h->nsm));
     switch (r) {
-      case 8: k_sf_fwd<8><<<g, SF_B, 0, st>>>(sw, h->d_fronts, A); break;
-      case 4: k_sf_fwd<4><<<g, SF_B, 0, st>>>(sw, h->d_fronts, A); break;
-      case 2: k_sf_fwd<2><<<g, SF_B, 0, st>>>(sw, h->d_fronts, A); break;
-      default: k_sf_fwd<1><<<g, SF_B, 0, st>>>(sw, h->d_fronts, A); break;
+      case 8: launch_chain(h, k_sf_fwd<8>, g, SF_B, 0, st, sw, (const DFront*)h->d_fronts, A); break;
+      case 4: launch_chain(h, k_sf_fwd<4>, g, SF_B, 0, st, sw, (const DFront*)h->d_fronts, A); break;
+      case 2: launch_chain(h, k_sf_fwd<2>, g, SF_B, 0, st, sw, (const DFront*)h->d_fronts, A); break;
+      default: launch_chain(h, k_sf_fwd<1>, g, SF_B, 0, st, sw, (const DFront*)h->d_fronts, A); break;
     }
   };
   if (!h->sf_attr) {  // the backward kernels' static + dynamic shared memory exceeds the default 48 KB
@@ -3567,29 +3604,27 @@ static int solve_common(rvg_handle* h, double* d_rhs, int64_t nrhs, int64_t ldb)
     CK(cudaFuncSetAttribute(k_sf_bwd<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, SF_BWD_DYN));
     h->sf_attr = true;
   }
-  auto bwd = [&](int r, size_t w, const SfWave& sw) {
-    const unsigned g = (unsigned)std::min<int64_t>(nbb[w], 6LL * h->nsm);
+  auto bwd = [&](int r, const SfWave& sw) {
+    const dim3 g((unsigned)std::min<int64_t>(sw.nblk, 6LL * h->nsm));
     switch (r) {
-      case 8: k_sf_bwd<8><<<g, SF_B, SF_BWD_DYN, st>>>(sw, h->d_fronts, A); break;
-      case 4: k_sf_bwd<4><<<g, SF_B, SF_BWD_DYN, st>>>(sw, h->d_fronts, A); break;
-      case 2: k_sf_bwd<2><<<g, SF_B, SF_BWD_DYN, st>>>(sw, h->d_fronts, A); break;
-      default: k_sf_bwd<1><<<g, SF_B, SF_BWD_DYN, st>>>(sw, h->d_fronts, A); break;
+      case 8: launch_chain(h, k_sf_bwd<8>, g, SF_B, SF_BWD_DYN, st, sw, (const DFront*)h->d_fronts, A); break;
+      case 4: launch_chain(h, k_sf_bwd<4>, g, SF_B, SF_BWD_DYN, st, sw, (const DFront*)h->d_fronts, A); break;
+      case 2: launch_chain(h, k_sf_bwd<2>, g, SF_B, SF_BWD_DYN, st, sw, (const DFront*)h->d_fronts, A); break;
+      default: launch_chain(h, k_sf_bwd<1>, g, SF_B, SF_BWD_DYN, st, sw, (const DFront*)h->d_fronts, A); break;
     }
   };
   for (int64_t rh = 0; rh < nrhs;) {
-    const int64_t left = nrhs - rh;
-    const int r = pass(left);
-    CK(cudaMemsetAsync(h->solve_work, 0xff, (size_t)wneed * 8, st));  // SF_EMPTY
+    const int r = pass(nrhs - rh);
+    CK(cudaMemsetAsync(h->solve_work, 0xff, (size_t)(2 * (int64_t)r * Y.rows) * 8, st));  // SF_EMPTY
+    CK(cudaMemsetAsync(h->sf_sync, 0, (size_t)Y.nsync * 4, st));
     for (size_t w = 0; w < nw; ++w) {
-      if (!nbf[w]) continue;
-      CK(cudaMemsetAsync(h->sf_sync, 0, (size_t)(nbf[w] + 1) * 4, st));
-      fwd(r, w, wave(w, true, rh));
+      if (!Y.w[w].nbf) continue;
+      fwd(r, wave(w, true, rh));
       launches++;
     }
     for (size_t w = nw; w-- > 0;) {
-      if (!nbb[w]) continue;
-      CK(cudaMemsetAsync(h->sf_sync, 0, (size_t)(nbb[w] + 1) * 4, st));
-      bwd(r, w, wave(w, false, rh));
+      if (!Y.w[w].nbb) continue;
+      bwd(r, wave(w, false, rh));
       launches++;
     }
     rh += r;
@@ -4199,6 +4234,8 @@ rvg_status rvg_trim(rvg_handle* h, int32_t what) {
   if (what & 1) {
     RVG_TRIM(h->solve_work, h->solve_work_cap);
     RVG_TRIM(h->sf_part, h->sf_part_cap);
+    RVG_TRIM(h->sf_lay, h->sf_lay_cap);
+    h->sf.ok = false;
     RVG_TRIM(h->d_x, h->x_cap);
     RVG_TRIM(h->d_ref, h->ref_cap);
     RVG_TRIM(h->d_gm, h->gm_cap);
@@ -4257,7 +4294,7 @@ void rvg_destroy(rvg_handle* h) {
     fr(h->d_stage); fr(h->scratch); fr(h->cb_arena); fr(h->pack); fr(h->wpack);
   }
   fr(h->d_vals); fr(h->d_scal);
-  fr(h->d_x); fr(h->solve_work); fr(h->d_stage2); fr(h->d_lf); fr(h->sf_sync); fr(h->sf_part); fr(h->d_gm);
+  fr(h->d_x); fr(h->solve_work); fr(h->d_stage2); fr(h->d_lf); fr(h->sf_sync); fr(h->sf_part); fr(h->sf_lay); fr(h->d_gm);
   drop_graph(h);
   fr(h->d_rec);
   if (h->d_sel) cudaFree(h->d_sel);

@@ -42,9 +42,11 @@
 //     further away watch one value with one thread, to keep the traffic on
 //     those lines low;
 //   * the sums over 64 columns run as four interleaved chains;
-//   * the diagonal block is solved by eights: one thread per right-hand side
-//     solves 8 unknowns, then every row takes their update (16 short barriers
-//     instead of 64 warp-serial steps), with all right-hand sides side by side.
+//   * the diagonal block is solved by eights (sf_diag): 8 or 16 short barriers
+//     instead of 64 warp-serial steps, all right-hand sides side by side.
+// What a solve needs to know of the factor (block layout, the front of each
+// ticket) is uploaded once per factorization; ticket counters and flags of all
+// waves are cleared together.
 // Up to 8 right-hand sides go through one launch (template R), each L value
 // read once for all of them.
 #pragma once
@@ -73,13 +75,14 @@ struct SfFront {
 
 struct SfWave {
   const SfFront* fr;
+  const int32_t* fmap;  // the position in fr of each ticket's front
   double* part;     // backward partial sums: slot q at part + q R 64
-  int32_t nfr, nblk;
+  int32_t nblk;
   int32_t* ticket;  // zeroed before the launch
   int32_t* flags;   // nblk entries, zeroed before the launch (backward: gathers and partial sums)
   double* x;        // solution vectors, permuted order: right-hand side r at x + r ldx
   int64_t ldx;
-  double* work;     // per-front work at DFront::scratch: y (R x m) then x_final (R x m); SF_EMPTY before the pass
+  double* work;     // per-front work at 2 R DFront::scratch: y (R x m) then x_final (R x m); SF_EMPTY before the pass
   int32_t* err;
 };
 
@@ -150,17 +153,6 @@ __device__ __forceinline__ void sf_wait(const int32_t* flag, int32_t* err) {
   }
 }
 
-// the wave's front holding ticket blk (last front with blk0 <= blk)
-__device__ __forceinline__ int sf_front(const SfWave& w, int blk) {
-  int lo = 0, hi = w.nfr - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (w.fr[mid].blk0 <= blk) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
-}
-
 __device__ __forceinline__ int32_t sf_col(const int32_t* rows, const int32_t* perm, int64_t i) { return rows[perm[i]]; }
 __device__ __forceinline__ int32_t sf_row(const int32_t* rows, const int32_t* perm, int64_t ne, int64_t k,
                                           int64_t t) {
@@ -203,12 +195,65 @@ __device__ __forceinline__ void sf_strip(const double (&l)[SF_B], int n, const d
 // Unit triangular solve of a diagonal block of n <= 64 rows held in shared
 // memory, row t of the R right-hand sides in acc of thread t; y is scratch.
 // Lower: L(t, j) = Ld[t][j], from the top; upper (the transpose): Ld[j][t],
-// from the bottom.  By eights: thread r solves the 8 unknowns of right-hand
-// side r, then every remaining row takes their update.
+// from the bottom.  By eights: the 8 unknowns are solved (by thread r for
+// right-hand side r, or by every thread for itself), then every remaining row
+// takes their update.
 template <int R, bool UPPER>
 __device__ __forceinline__ void sf_diag(const double (*Ld)[SF_B + 1], int n, double (*y)[SF_B], double (&acc)[R]) {
   const int t = threadIdx.x;
   const int nb = (n + 7) / 8;
+  if constexpr (R <= 2) {
+    // few right-hand sides: every thread solves the 8 unknowns itself, from coefficients read before the
+    // barrier, so a step is one barrier and one shared-memory trip
+    for (int q = 0; q < nb; ++q) {
+      const int j0 = (UPPER ? nb - 1 - q : q) * 8;
+      const bool own = t >= j0 && t < j0 + 8;
+      const bool later = UPPER ? t < j0 : (t >= j0 + 8 && t < n);
+      if (own) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) y[r][t] = t < n ? acc[r] : 0.0;
+      }
+      double cf[8][8], l[8];
+#pragma unroll
+      for (int a = 1; a < 8; ++a)
+#pragma unroll
+        for (int b = 0; b < a; ++b) cf[a][b] = j0 + a < n ? Ld[j0 + a][j0 + b] : 0.0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) l[j] = later && j0 + j < n ? (UPPER ? Ld[j0 + j][t] : Ld[t][j0 + j]) : 0.0;
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        double v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = y[r][j0 + i];
+        if (!UPPER) {
+#pragma unroll
+          for (int j = 0; j < 7; ++j)
+#pragma unroll
+            for (int i = j + 1; i < 8; ++i) v[i] = __fma_rn(-cf[i][j], v[j], v[i]);
+        } else {
+#pragma unroll
+          for (int j = 7; j > 0; --j)
+#pragma unroll
+            for (int i = 0; i < j; ++i) v[i] = __fma_rn(-cf[j][i], v[j], v[i]);
+        }
+        if (own) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (t == j0 + i) acc[r] = v[i];
+        } else {
+          double e = 0.0, o = 0.0;
+#pragma unroll
+          for (int j = 0; j < 8; j += 2) {
+            e = __fma_rn(-l[j], v[j], e);
+            o = __fma_rn(-l[j + 1], v[j + 1], o);
+          }
+          if (later) acc[r] += e + o;
+        }
+      }
+    }
+    return;
+  }
   for (int q = 0; q < nb; ++q) {
     const int j0 = (UPPER ? nb - 1 - q : q) * 8, j1 = j0 + 8 < n ? j0 + 8 : n;
     if (t >= j0 && t < j0 + 8) {
@@ -260,19 +305,20 @@ __global__ void __launch_bounds__(SF_B) k_sf_fwd(SfWave w, const DFront* F, Aren
   __shared__ double yb[R][SF_B];
   __shared__ double Ls[SF_B][SF_B + 1];
   const int t = threadIdx.x;
+  chain_enter();  // (launched while the wave before still runs)
   for (;;) {
     if (t == 0) s_blk = atomicAdd(w.ticket, 1);
     __syncthreads();
     const int blk = s_blk;
     __syncthreads();
     if (blk >= w.nblk) break;
-    const SfFront sf = w.fr[sf_front(w, blk)];
+    const SfFront sf = w.fr[w.fmap[blk]];
     const DFront fr = F[sf.s];
     const int64_t m = fr.m, ne = fr.ne;
     const double* L = A.panel + fr.panel;
     const int32_t* rows = A.idx + fr.idx;
     const int32_t* perm = rows + m;
-    double* v = w.work + fr.scratch;  // y of right-hand side r at v + r m
+    double* v = w.work + 2 * R * fr.scratch;  // y of right-hand side r at v + r m
     const int b = blk - sf.blk0;
     const bool diag = b < sf.nbd;
     const int64_t r0 = diag ? (int64_t)b * SF_B : ne + (int64_t)(b - sf.nbd) * SF_B;
@@ -346,20 +392,21 @@ __global__ void __launch_bounds__(SF_B) k_sf_bwd(SfWave w, const DFront* F, Aren
   double(*Ld)[SF_B + 1] = reinterpret_cast<double(*)[SF_B + 1]>(sf_dyn);
   __shared__ double xs[R][SF_B];
   const int t = threadIdx.x;
+  chain_enter();  // (launched while the wave before still runs)
   for (;;) {
     if (t == 0) s_blk = atomicAdd(w.ticket, 1);
     __syncthreads();
     const int blk = s_blk;
     __syncthreads();
     if (blk >= w.nblk) break;
-    const SfFront sf = w.fr[sf_front(w, blk)];
+    const SfFront sf = w.fr[w.fmap[blk]];
     const DFront fr = F[sf.s];
     const int64_t m = fr.m, ne = fr.ne;
     const double* L = A.panel + fr.panel;
     const int32_t* rows = A.idx + fr.idx;
     const int32_t* perm = rows + m;
-    const double* y = w.work + fr.scratch;      // forward results of right-hand side r at y + r m
-    double* xf = w.work + fr.scratch + R * m;   // final values of this front's columns, at xf + r m
+    const double* y = w.work + 2 * R * fr.scratch;  // forward results of right-hand side r at y + r m
+    double* xf = w.work + 2 * R * fr.scratch + R * m;  // final values of this front's columns, at xf + r m
     int32_t* flags = w.flags + sf.blk0;
     const int nbr = sf.nbr, ngrp = sf.ngrp;
     const int lt = blk - sf.blk0;  // ticket within the front

@@ -68,6 +68,7 @@ struct LFState {
   // later launch of the front returns at once until the host clears it
   int32_t spec_bad;
   int32_t done;  // CTAs of a k_lf_update with failed columns that have finished
+  int32_t valid[2];  // the outer block (its number + 1) that began last with each parity
   LFBlk b[2];    // inner block i is b[i & 1]: the update of block i factors block i + 1
 };
 
@@ -85,12 +86,14 @@ struct LFArgs {
   int64_t cs, bcols, nfsb;  // outer block start, width, NFS boundary (global p)
   int par;          // which of the state's two blocks is the current inner block
   int win;          // the rows below the outer block keep their W (the outer block joins the window)
+  int outer;        // the outer block's number (lp is one of two arrays, by its parity)
   DevOpts o;
 };
 
 __global__ void k_lf_init(LFState* st, int32_t* perm, int64_t p) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     st->gne = 0; st->n1 = 0; st->n2 = 0; st->spec_bad = 0; st->done = 0;
+    st->valid[0] = st->valid[1] = 0;
   }
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < p; i += (int64_t)gridDim.x * blockDim.x)
     perm[i] = (int32_t)i;
@@ -189,7 +192,7 @@ __global__ void __launch_bounds__(NT) k_lf_begin_outer(LFArgs A) {
     if (threadIdx.x == 0) st->spec_bad = 1;
     return;
   }
-  if (threadIdx.x == 0) { st->end_pos = (int32_t)A.bcols; st->bne = 0; }
+  if (threadIdx.x == 0) { st->end_pos = (int32_t)A.bcols; st->bne = 0; st->valid[A.outer & 1] = A.outer + 1; }
   for (int i = threadIdx.x; i < A.bcols; i += blockDim.x) A.lp[i] = i;
   __syncthreads();
   lf_block_cta(A, sh, 0, 0, (int)A.bcols, 0, 0);
@@ -466,11 +469,14 @@ __global__ void __launch_bounds__(NT, 2) k_lf_update(LFArgs A, int next) {
 }
 
 // row permutation of the outer block applied to the front's earlier columns
-// 0..cs (two_level_factor, factor.rs:2165-2181): 16 columns per CTA
+// 0..cs (two_level_factor, factor.rs:2165-2181): 16 columns per CTA.  Nothing
+// on the front's path reads those rows again, so it runs on a stream of its own
+// beside the blocks that follow (12 to 17 us of ~290 per outer block of a
+// 13,572 front); it acts if its outer block really began, whatever a later,
+// mispredicted one has flagged meanwhile.
 constexpr int LF_PROP_COLS = 16;
 __global__ void __launch_bounds__(256) k_lf_prop(LFArgs A) {
-  chain_enter();
-  if (A.st->spec_bad) return;  // a block issued past a mispredicted start column
+  if (A.st->valid[A.outer & 1] != A.outer + 1) return;
   extern __shared__ double buf[];  // bcols x LF_PROP_COLS
   const int64_t c0 = (int64_t)blockIdx.x * LF_PROP_COLS;
   const int nc = (int)((A.cs - c0) < LF_PROP_COLS ? (A.cs - c0) : LF_PROP_COLS);
@@ -507,14 +513,18 @@ __device__ __forceinline__ void lf_swap_delayed(const LFArgs& A, int64_t cs, int
 }
 
 // End of an outer block: its column order into the front's pivot order, the
-// delay swap (unless `swap` is 0: a far-field update may still be running on
-// another stream, and the host issues the swap itself, k_lf_swap, once it has
-// seen the delay), the eliminated total.
-__global__ void __launch_bounds__(NT) k_lf_outer(LFArgs A, int64_t rem, int two_level, int swap) {
+// delay swap (unless `swap` is 0: a far-field update or the row permutation may
+// still be running on another stream, and the host issues the swap itself,
+// k_lf_swap, once it has seen the delay), the eliminated total, also into the
+// host's (pinned) slot for this block when given.
+__global__ void __launch_bounds__(NT) k_lf_outer(LFArgs A, int64_t rem, int two_level, int swap, int32_t* host_gne) {
   chain_enter();
-  if (A.st->spec_bad) return;  // a block issued past a mispredicted start column
   LFState* st = A.st;
   const int tid = threadIdx.x;
+  if (st->spec_bad) {  // a block issued past a mispredicted start column
+    if (tid == 0 && host_gne) *host_gne = st->gne;
+    return;
+  }
   const int bne = st->bne;
   const int64_t cs = A.cs, bcols = A.bcols;
   // perm[cs + i] = orig[lp[i]], via the inner W scratch as the copy buffer
@@ -525,7 +535,11 @@ __global__ void __launch_bounds__(NT) k_lf_outer(LFArgs A, int64_t rem, int two_
   __syncthreads();
   if (swap && two_level && bne < bcols) lf_swap_delayed(A, cs, bcols, rem, bne);
   __syncthreads();
-  if (tid == 0) st->gne += bne;
+  if (tid == 0) {
+    const int32_t g = st->gne + bne;
+    st->gne = g;
+    if (host_gne) *host_gne = g;
+  }
 }
 
 // The delay swap of an outer block issued without it (k_lf_outer with swap =

@@ -1228,6 +1228,9 @@ struct LfCtx {
   // far-field part of a full window's update, beside the next outer blocks (mixed form)
   cudaStream_t far_st = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_far = nullptr;
+  // row permutations of the outer blocks, beside the blocks that follow (one event per parity)
+  cudaStream_t prop_st = nullptr;
+  cudaEvent_t ev_prop_fork = nullptr, ev_prop[2] = {};
   int64_t far_launches = 0;
   int id = 0;  // position in the handle's contexts (its window buffer's address-stable arena)
 };
@@ -2189,7 +2192,7 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
   a.wo = sc + 2 * m * IBMAX;
   const bool mixed = front_mixed(h, s);
   const int64_t F = lf_window_cols(h, nb, mixed);
-  a.lp = (int32_t*)(sc + m * (2 * IBMAX + lf_window_blocks(h) * nb));
+  int32_t* const lp2 = (int32_t*)(sc + m * (2 * IBMAX + lf_window_blocks(h) * nb));  // two arrays of nb
   a.nfsb = p;
   a.o = dop;
   const int two_level = p > nb;
@@ -2223,6 +2226,17 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
     CK(cudaEventCreateWithFlags(&cx.ev_fork, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&cx.ev_far, cudaEventDisableTiming));
   }
+  // The row permutations on their own stream, and the delay swap (which touches the same rows) left to the
+  // host, in the dynamic schedule; in order on the front's stream in a captured graph or with the marks on.
+  const bool side_prop = two_level && !profiling_marks && !h->replay;
+  if (side_prop && !cx.prop_st) {
+    if (tl_no_alloc) return no_alloc_fail();
+    CK(cudaStreamCreateWithFlags(&cx.prop_st, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&cx.ev_prop_fork, cudaEventDisableTiming));
+    for (auto& e : cx.ev_prop) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  }
+  bool prop_due[2] = {false, false};  // a permutation of that parity's lp may still run
+  const bool host_swap = async_far || side_prop;
   mk(-1);
   k_lf_init<<<blocks_for(p, 256), 256, 0, st>>>(a.st, a.perm, p);
   cx.launches++;
@@ -2259,6 +2273,13 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
     I.cs = cs; I.bcols = bcols; I.oe = oe;
     a.cs = cs;
     a.bcols = bcols;
+    a.outer = (int)S.outer;
+    const int opar = a.outer & 1;
+    a.lp = lp2 + opar * nb;
+    if (prop_due[opar]) {
+      ck(cudaStreamWaitEvent(st, cx.ev_prop[opar], 0), "cudaStreamWaitEvent (row permutation)");
+      prop_due[opar] = false;
+    }
     I.window = two_level && oe < p;
     a.win = I.window;
     if (I.window) {  // this block's W joins the window [wd, gne + bne)
@@ -2286,8 +2307,16 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
     cx.launches += 1 + 2 * ninner;
     if (two_level) {
       if (cs > 0) {
-        launch_chain(h, k_lf_prop, (unsigned)((cs + LF_PROP_COLS - 1) / LF_PROP_COLS), 256,
-                     (size_t)bcols * LF_PROP_COLS * 8, st, a);
+        const cudaStream_t ps = side_prop ? cx.prop_st : st;
+        if (side_prop) {
+          ck(cudaEventRecord(cx.ev_prop_fork, st), "cudaEventRecord (row permutation fork)");
+          ck(cudaStreamWaitEvent(ps, cx.ev_prop_fork, 0), "cudaStreamWaitEvent (row permutation fork)");
+        }
+        k_lf_prop<<<(unsigned)((cs + LF_PROP_COLS - 1) / LF_PROP_COLS), 256, (size_t)bcols * LF_PROP_COLS * 8, ps>>>(a);
+        if (side_prop) {
+          ck(cudaEventRecord(cx.ev_prop[opar], ps), "cudaEventRecord (row permutation)");
+          prop_due[opar] = true;
+        }
         cx.launches++;
         mk(RVG_PART_LF_PROP);
       }
@@ -2347,7 +2376,8 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
         mk(RVG_PART_LF_SYRK);
       }
     }
-    launch_chain(h, k_lf_outer, 1, NT, 0, st, a, rem, (int)two_level, async_far ? 0 : 1);
+    launch_chain(h, k_lf_outer, 1, NT, 0, st, a, rem, (int)two_level, host_swap ? 0 : 1,
+                 h->replay ? (int32_t*)nullptr : cx.h_gne + slot);
     cx.launches++;
     mk(RVG_PART_LF_OUTER);
     return I;
@@ -2418,7 +2448,6 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
         next_slot = (next_slot + 1) % LF_AHEAD;
         Issued I = issue(S, slot);
         if (irc) return irc;
-        CK(cudaMemcpyAsync(cx.h_gne + slot, &a.st->gne, 4, cudaMemcpyDeviceToHost, st));
         CK(cudaEventRecord(cx.ring_ev[slot], st));
         CK(cudaGetLastError());
         q.push_back(I);
@@ -2430,7 +2459,7 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
       const double t0 = now_ms();
       CK(cudaEventSynchronize(cx.ring_ev[I.slot]));
       const double waited = now_ms() - t0;
-      const int32_t g = cx.h_gne[I.slot];
+      const int32_t g = *(volatile int32_t*)(cx.h_gne + I.slot);  // written by the block's k_lf_outer
       h->rec_g[s].push_back(g);
       if (profiling_marks) {
         mark_flush(h);
@@ -2445,16 +2474,18 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
       const double t1 = now_ms();
       CK(cudaStreamSynchronize(st));
       if (cx.far_st) CK(cudaStreamSynchronize(cx.far_st));
+      if (cx.prop_st) CK(cudaStreamSynchronize(cx.prop_st));
+      prop_due[0] = prop_due[1] = false;
       cx.sync_ms += now_ms() - t1;
       cx.misses += (int64_t)q.size();
       q.clear();
       HostLF T = next_state(I, g);
       T.far_due = -1;  // nothing runs on the far stream any more
-      if (async_far) {
+      if (host_swap) {
         const int64_t bne = g - I.cs;
         a.cs = I.cs;
         a.bcols = I.bcols;
-        if (two_level && I.window && !I.flush && I.oe + nb < p) {
+        if (async_far && I.window && !I.flush && I.oe + nb < p) {
           // the far field takes the window, this block's eliminated columns included
           irc = launch_window_gemm(h, cx, a, m, I.oe + nb, p, I.before.wd, I.before.wrow, F, pk_wb[I.before.par],
                                    pk_lb[I.before.par], I.kadd + bne, nullptr, nullptr, 0, mixed);
@@ -2470,6 +2501,8 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
     }
   }
   if (S.far_due >= 0) CK(cudaStreamWaitEvent(st, cx.ev_far, 0));  // a far-field update still running
+  for (int q = 0; q < 2; ++q)
+    if (prop_due[q]) CK(cudaStreamWaitEvent(st, cx.ev_prop[q], 0));
   k_lf_finish<<<1, 32, 0, st>>>(a, h->d_fronts, s);
   cx.launches++;
   mk(RVG_PART_LF_SETUP);
@@ -4311,6 +4344,9 @@ void rvg_destroy(rvg_handle* h) {
     if (c.far_st) { cudaStreamSynchronize(c.far_st); cudaStreamDestroy(c.far_st); }
     if (c.ev_fork) cudaEventDestroy(c.ev_fork);
     if (c.ev_far) cudaEventDestroy(c.ev_far);
+    if (c.prop_st) { cudaStreamSynchronize(c.prop_st); cudaStreamDestroy(c.prop_st); }
+    if (c.ev_prop_fork) cudaEventDestroy(c.ev_prop_fork);
+    for (auto& e : c.ev_prop) if (e) cudaEventDestroy(e);
     if (t == 0) continue;  // the handle's own stream, state and window buffer
     if (!h->vm) fr(c.wpack);
     if (c.lf) cudaFree(c.lf);

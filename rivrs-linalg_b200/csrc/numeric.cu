@@ -132,8 +132,11 @@ __global__ void k_scatter(const ScatterItem* items, const DFront* F, Statics S, 
 // (numeric.rs:2445-2559).  The child block is [delayed; NFS] x [delayed;
 // NFS]: its delayed columns live in the child's panel (rows ne..k and k..m
 // of columns ne..k), its NFS x NFS part in the child's contribution buffer.
-// An item is a 32-column group [j0, j0+32) of one child's block and a
-// segment of its rows [i0, i0 + EA_ROWS), i >= j only.  Each CTA stages the group's 32 destination
+// An item is a group of `width` columns [j0, j0 + width) of one child's block and
+// a segment of its rows [i0, i0 + EA_ROWS), i >= j only: 32 columns where the
+// items fill the GPU (a row's map is looked up once for all of them), 8 where
+// they do not (a batch of 8 columns is two memory round trips, and four batches
+// one after another are most of a small launch's 8.5 us).  Each CTA stages the group's destination
 // columns in shared memory, then walks its rows in tiles of 256, one row per
 // thread: the thread maps its row once, then handles the 32 columns in
 // batches of 8 with all eight source loads, then all eight destination
@@ -145,7 +148,9 @@ __global__ void k_scatter(const ScatterItem* items, const DFront* F, Statics S, 
 constexpr int EA_ROWS = 4096;  // rows per item
 struct EaTile { int32_t parent; int32_t child; int32_t j0; int32_t i0; };
 
-__global__ void __launch_bounds__(256, 3) k_extend_add_tiled(const EaTile* items, const DFront* F, Statics S, Arenas A) {
+constexpr int EA_WIDE = 32, EA_NARROW = 8;
+__global__ void __launch_bounds__(256, 3) k_extend_add_tiled(const EaTile* items, const DFront* F, Statics S, Arenas A,
+                                                             int width) {
   const EaTile it = items[blockIdx.x];
   const DFront P = F[it.parent];
   const DFront C = F[it.child];
@@ -163,7 +168,7 @@ __global__ void __launch_bounds__(256, 3) k_extend_add_tiled(const EaTile* items
     return l < P.nown ? l : l + P.ndin;
   };
   __shared__ int s_lj[32];
-  const int jn = min(32, sz - it.j0);
+  const int jn = min(width, sz - it.j0);
   if (threadIdx.x < 32) s_lj[threadIdx.x] = threadIdx.x < jn ? map(it.j0 + threadIdx.x) : 0;
   __syncthreads();
   const int i1 = min(sz, it.i0 + EA_ROWS);
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(256, 3) k_extend_add_tiled(const EaTile* items
     // rows of the child block: delayed rows live in the child's panel rows ne.., NFS rows at k..
     const int64_t prow = i < nd ? (int64_t)(C.ne + i) : (int64_t)(C.k + (i - nd));
 #pragma unroll 1
-    for (int jb = 0; jb < 32; jb += 8) {
+    for (int jb = 0; jb < width; jb += 8) {
       double v[8];
       double* dst[8];
 #pragma unroll
@@ -2673,7 +2678,7 @@ int refactor_fp64(rvg_handle* h, const std::vector<int32_t>& redo, const Arenas&
   for (size_t q = 0; q < maxch; ++q)
     if (!eitems[q].empty())
       k_extend_add_tiled<<<(unsigned)eitems[q].size(), 256, 0, st>>>((const EaTile*)(D + o_e[q]), h->d_fronts,
-                                                                      statics(h), A);
+                                                                      statics(h), A, EA_WIDE);
   CK(cudaGetLastError());
   if ((rc = factor_large_fronts(h, redo, A, dop))) return rc;
   if (!witems.empty())
@@ -2898,16 +2903,23 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
     size_t maxch = 0;
     for (int64_t s : wave) maxch = std::max(maxch, P.children[s].size());
     std::vector<std::vector<EaTile>> eitems(maxch);
-    for (size_t q = 0; q < maxch; ++q)
+    std::vector<int> ewidth(maxch, EA_WIDE);
+    auto ea_items = [&](size_t q, int width) {
+      eitems[q].clear();
       for (int64_t s : wave) {
         if (q >= P.children[s].size()) continue;
         int64_t c = P.children[s][q];
         const DFront& cf = h->h_fronts[c];
         if (!(cf.flags & FF_HAS_PARENT) || cf.ne >= cf.m) continue;
         int sz = cf.m - cf.ne;
-        for (int j0 = 0; j0 < sz; j0 += 32)
+        for (int j0 = 0; j0 < sz; j0 += width)
           for (int i0 = j0; i0 < sz; i0 += EA_ROWS) eitems[q].push_back(EaTile{(int32_t)s, (int32_t)c, j0, i0});
       }
+    };
+    for (size_t q = 0; q < maxch; ++q) {
+      ea_items(q, EA_WIDE);
+      if (eitems[q].size() < (size_t)h->nsm) ea_items(q, ewidth[q] = EA_NARROW);  // (up to 4 times as many: 4 per SM)
+    }
     std::vector<CbZeroItem> zitems;
     for (int64_t s : wave) {
       const DFront& f = h->h_fronts[s];
@@ -2969,7 +2981,7 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
     for (size_t q = 0; q < maxch; ++q)
       if (!eitems[q].empty())
         k_extend_add_tiled<<<(unsigned)eitems[q].size(), 256, 0, st>>>((const EaTile*)(D + o_e[q]), h->d_fronts,
-                                                                        statics(h), A);
+                                                                        statics(h), A, ewidth[q]);
     CK(cudaEventRecord(h->ev[2], st));
     // contribution blocks whose parents are now all assembled
     for (size_t w2 = 0; w2 < w; ++w2)

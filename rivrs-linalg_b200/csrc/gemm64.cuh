@@ -184,26 +184,36 @@ __global__ void __launch_bounds__(32 * WR * WC, MINB) k_syrk_dmma(SyrkArgs a) {
   extern __shared__ double gsm[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wr = (warp % WR) * 32, wc = (warp / WR) * 32;
-  const int64_t nchunk = (K + G_BK - 1) / G_BK;
-  auto issue = [&](int64_t ch) {
+  const int nchunk = (int)((K + G_BK - 1) / G_BK);
+  // A thread copies one row of W and one of L, every NT / BM-th (NT / BN-th)
+  // column: its addresses advance by a constant.  (Indexed per element, the 64-bit
+  // products and bounds were most of the instructions of a chunk: 27.2 -> 31.3
+  // TFLOP/s on a 9600^2 rank-1024 update.)
+  static_assert(NT % BM == 0 && NT % BN == 0, "a thread keeps its row");
+  constexpr int SW = NT / BM, SL = NT / BN;  // columns between a thread's copies
+  const int rw = tid % BM, kw = tid / BM, rl = tid % BN, kl = tid / BN;
+  const bool okw = i0 + rw < a.r1, okl = j0 + rl < a.c1;
+  const double* pw = a.W + (okw ? i0 + rw - a.r0 : 0) + (int64_t)kw * a.ldw;
+  const double* pl = a.L + (okl ? j0 + rl : a.c0) + (int64_t)kl * a.ldl;
+  const int64_t stw = SW * a.ldw, stl = SL * a.ldl;
+  auto issue = [&](int ch) {
     double* sw = gsm + (ch % G_STAGES) * G_BK * (LDW + LDL);
     double* sl = sw + G_BK * LDW;
-    const int64_t k0 = ch * G_BK;
+    const int64_t k0 = (int64_t)ch * G_BK;
+    const bool full = k0 + G_BK <= K;
+    const double* p = pw + k0 * a.ldw;
+    const double* q = pl + k0 * a.ldl;
 #pragma unroll
-    for (int e = 0; e < (G_BK * BM) / NT; ++e) {
-      const int idx = tid + NT * e;
-      const int r = idx % BM, k = idx / BM;
-      const int64_t kk = k0 + k, i = i0 + r;
-      const bool v = kk < K && i < a.r1;
-      cp_async8(sw + k * LDW + r, v ? a.W + (i - a.r0) + kk * a.ldw : a.W, v);
+    for (int e = 0; e < G_BK / SW; ++e) {
+      const bool v = okw && (full || k0 + kw + SW * e < K);
+      cp_async8(sw + (kw + SW * e) * LDW + rw, v ? p : a.W, v);
+      p += stw;
     }
 #pragma unroll
-    for (int e = 0; e < (G_BK * BN) / NT; ++e) {
-      const int idx = tid + NT * e;
-      const int r = idx % BN, k = idx / BN;
-      const int64_t kk = k0 + k, j = j0 + r;
-      const bool v = kk < K && j < a.c1;
-      cp_async8(sl + k * LDL + r, v ? a.L + j + kk * a.ldl : a.L, v);
+    for (int e = 0; e < G_BK / SL; ++e) {
+      const bool v = okl && (full || k0 + kl + SL * e < K);
+      cp_async8(sl + (kl + SL * e) * LDL + rl, v ? q : a.L, v);
+      q += stl;
     }
   };
 #pragma unroll
@@ -219,10 +229,11 @@ __global__ void __launch_bounds__(32 * WR * WC, MINB) k_syrk_dmma(SyrkArgs a) {
     for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
+        // (clamped to the last row and column; what lies past them is not stored)
         const int64_t i = i0 + wr + mi * 8 + fr, j = j0 + wc + ni * 8 + fc + q;
-        acc[mi][ni][q] = (i < a.r1 && j < a.c1 && i >= j) ? a.C[i + j * a.ldc] : 0.0;
+        acc[mi][ni][q] = a.C[(i < a.r1 ? i : a.r1 - 1) + (j < a.c1 ? j : a.c1 - 1) * a.ldc];
       }
-  for (int64_t ch = 0; ch < nchunk; ++ch) {
+  for (int ch = 0; ch < nchunk; ++ch) {
     cp_async_wait<G_STAGES - 2>();
     __syncthreads();
     if (ch + G_STAGES - 1 < nchunk) issue(ch + G_STAGES - 1);
@@ -261,8 +272,9 @@ __global__ void __launch_bounds__(32 * WR * WC, MINB) k_syrk_dmma(SyrkArgs a) {
 
 
 // the configuration used by the library: DMMA, 2 x 2 warps (64 x 64 tile),
-// four CTAs per SM (the fastest of the measured shapes: 25-28 TFLOP/s on a
-// 16384^2 rank-256 / rank-1024 update)
+// four CTAs per SM (the fastest of the measured shapes on a 9600^2 rank-1024
+// update: 31.3 TFLOP/s; 128 x 64 with 4 or 8 warps 30.3 and 30.8, 64 x 128 29.4,
+// 128 x 128 26.8; a fourth stage or tiles walked in groups of rows change nothing)
 #ifndef RVG_SYRK_WR
 #define RVG_SYRK_WR 2
 #define RVG_SYRK_WC 2

@@ -135,8 +135,12 @@ __device__ __forceinline__ void sf_take_block(const double* src, int64_t m, int 
     __syncthreads();
   }
   if (t < n) {
+    unsigned long long v[R];  // every right-hand side's value in flight before the first is looked at
 #pragma unroll
-    for (int r = 0; r < R; ++r) dst[r][t] = sf_take(src + r * m + t, err);
+    for (int r = 0; r < R; ++r) v[r] = sf_peek(src + r * m + t);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      dst[r][t] = v[r] != SF_EMPTY ? __longlong_as_double((long long)v[r]) : sf_take(src + r * m + t, err);
   }
   __syncthreads();
 }

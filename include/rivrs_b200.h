@@ -53,7 +53,7 @@ typedef struct {
   /* B200 scheduling, no reference counterpart: fronts of order >= this use
    * the multi-kernel path (whole GPU per front), and so do fronts of at least
    * half this order in a wave that holds at most 16 of them; the others are
-   * batched one CTA or warp per front, except the few (of order >= a 16th of
+   * batched one CTA per front, except the few (of order >= a 16th of
    * this) whose single CTA would hold the wave up: those take the multi-kernel
    * path too, in FP64.  Results do not depend on it.  Default 2048. */
   int64_t large_front_threshold;
@@ -275,20 +275,20 @@ typedef struct {
 
 /* Indices of rvg_profile.part_ms.  Large fronts (whole GPU per front): */
 enum {
-  RVG_PART_LF_SETUP = 0,   /* per-front and per-outer-block bookkeeping */
-  RVG_PART_LF_BLOCK = 1,   /* 32x32 diagonal block, complete pivoting */
-  RVG_PART_LF_PANEL = 2,   /* TRSM + D^-1 of the rows below, threshold test */
+  RVG_PART_LF_SETUP = 0,   /* per-front bookkeeping */
+  RVG_PART_LF_BLOCK = 1,   /* an outer block's first 32x32 diagonal block, complete pivoting */
+  RVG_PART_LF_PANEL = 2,   /* TRSM + D^-1 of the rows below, threshold test, W = L D */
   RVG_PART_LF_POST = 3,    /* (unused: the first failing column is handled inside LF_UPDATE) */
-  RVG_PART_LF_UPDATE = 4,  /* rank-32 update inside the outer block */
-  RVG_PART_LF_DELAY = 5,   /* delayed columns to the end */
+  RVG_PART_LF_UPDATE = 4,  /* rank-32 update inside the outer block, the next diagonal block beside it */
+  RVG_PART_LF_DELAY = 5,   /* (unused: delayed columns are moved inside LF_UPDATE) */
   RVG_PART_LF_PROP = 6,    /* row order propagated to earlier columns */
-  RVG_PART_LF_W = 7,       /* W = L D of the outer block */
+  RVG_PART_LF_W = 7,       /* (unused: W = L D is formed inside LF_PANEL) */
   RVG_PART_LF_SYRK = 8,    /* deferred trailing Schur update */
   RVG_PART_LF_OUTER = 9,   /* end of outer block */
   /* batched fronts and contribution blocks: */
-  RVG_PART_TPP = 10,       /* warp-per-front TPP fronts */
-  RVG_PART_APTP = 11,      /* CTA-per-front APTP fronts */
-  RVG_PART_CB_W = 12,      /* W = L21 D of contribution blocks */
+  RVG_PART_TPP = 10,       /* (unused: counted in APTP) */
+  RVG_PART_APTP = 11,      /* small (TPP) and medium (APTP) fronts, one CTA each */
+  RVG_PART_CB_W = 12,      /* W = L21 D of large contribution blocks */
   RVG_PART_CB_GEMM = 13,   /* small contribution GEMMs (batched) */
   RVG_PART_CB_SYRK = 14,   /* large contribution GEMMs */
   RVG_PART_OTHER = 15,

@@ -2,7 +2,7 @@
 
 Two options only schedule the work: the large-front cutoff
 (`large_front_threshold`: fronts at or above it take the whole GPU one after
-another, the others are batched one CTA or warp per front) and, in the mixed
+another, the others are batched one CTA per front) and, in the mixed
 form without flushing, the Schur GEMM's tile width (`mixed_tile_cols`: 128, or
 256 = two 128-column tiles sharing one W tile).  In the plain form neither
 changes a result; the tile width changes none in the mixed form either, but

@@ -6,7 +6,7 @@ level-set schedule of the numeric phase (factor_tree_levelset,
 sparse/src/symmetric/numeric.rs:1957-2163) puts the fronts of every system
 that sit at the same height into the same wave, and each wave's small and
 medium fronts, across all the union's systems, go through the same batched
-launches (one CTA or warp per front); large fronts take the whole GPU one
+launches (one CTA per front); large fronts take the whole GPU one
 after another.  Each system's fronts, pivots and factors are exactly the ones
 a separate factorization of that system with the same ordering and scaling
 produces (its tree is untouched by the others).

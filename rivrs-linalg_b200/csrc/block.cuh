@@ -20,14 +20,15 @@
 //     swaps do not move them; they are put in position order once at the end.
 // Every entry gets the operations of the reference's loops, in their order.
 //
-// Measured (clock64, one CTA, 32 columns): 55.5k -> 36.8k cycles where every
-// pivot is 1x1 (a stencil's block), 41.3k -> 25.7k with mostly 2x2 pivots,
+// Measured (clock64, one CTA, 32 columns): 55.5k -> 34.7k cycles where every
+// pivot is 1x1 (a stencil's block), 41.3k -> 25.1k with mostly 2x2 pivots,
 // against the version in which warp 0 searched, swapped and scaled while the
-// others waited (three barrier-separated phases a step).  A step is ~1150
+// others waited (three barrier-separated phases a step).  A step is ~1100
 // cycles: barrier and candidate reduction ~300, decoding ~150, reciprocal ~90,
 // update ~350, own reduction ~90.  Four warps (the repeated work issued once per
-// scheduler), 16 warps, and rows and columns kept in place with a position
-// table instead of moved entries were all slower or equal.
+// scheduler: 41k / 29k), 16 warps with rows and columns kept in place and a
+// position table (37k / 27k), and integer instead of FP64 compares (32.7k /
+// 28.9k, slower over mixed pivots) were not better.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>

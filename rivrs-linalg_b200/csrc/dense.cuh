@@ -8,14 +8,14 @@
 // contribution buffer.
 //
 // Two executors:
-//   * warp_tpp_*  : one warp runs threshold partial pivoting
-//                   (factor.rs:2335-2506, 2761-2947); used for small-leaf
-//                   fronts, fronts with k < ib, and the TPP fallback.
+//   * WarpTpp     : one warp runs threshold partial pivoting
+//                   (factor.rs:2335-2506, 2761-2947): the TPP fallback and
+//                   the allocation-free entry point; its scans also serve
+//                   the CTA version of the small fronts (tpp.cuh).
 //   * cta_aptp_*  : one CTA runs the blocked APTP (factor_inner,
 //                   factor.rs:1811-2095, and two_level_factor,
 //                   factor.rs:2108-2252), with the 32x32 complete-pivoting
-//                   block (factor.rs:891-1153) done by one warp in shared
-//                   memory with warp-shuffle arg-max reductions.
+//                   block (factor.rs:891-1153) of block.cuh.
 // Per-entry arithmetic follows the oracle's operation order, so the values a
 // front produces match the oracle's bit for bit wherever no cross-thread
 // reduction order is involved.

@@ -204,6 +204,8 @@ __global__ void __launch_bounds__(NT) k_lf_begin_outer(LFArgs A) {
 // found, before the scan's result over all rows is known: the pivots that pass
 // are a prefix, and the columns after them are written again by later blocks.
 // Rows below the outer block also leave it in the window of pending columns.
+// 8.5 us on a front of order 13,572, most of it latency: the launch, two trips
+// to memory, the 31 dependent steps of the triangular solve.
 constexpr int LF_PANEL_T = 64;
 
 // One panel row; FULL: a 32-column block all of whose pivots were found, the

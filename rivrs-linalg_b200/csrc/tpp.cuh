@@ -29,9 +29,13 @@ namespace rvg {
 constexpr int TPP_MAX_T = 256;               // threads of a CTA at most
 constexpr size_t TPP_SMEM_MAX = 226 * 1024;  // dynamic shared memory of a CTA at most
 
+// Off: int where the front is in shared memory, int64_t where it is in global
+// memory (with a raised small_leaf_threshold, m k is not bounded by 2^31 there).
+template <class Off>
 struct CtaTpp {
   double* a;
-  int ld, m, n;  // n = k: all stored columns are candidates
+  Off ld;
+  int m, n;  // n = k: all stored columns are candidates
   int32_t* perm;
   DRec d;
   double* mx;  // [0] max |a(r, ne)| over r > ne, r != ne + 1; [1] max |a(r, ne + 1)| over r > ne + 1
@@ -257,7 +261,7 @@ __global__ void __launch_bounds__(TPP_MAX_T) k_tpp_cta(const int32_t* ids, DFron
     }
     for (int i = tid; i < k; i += nt) perm[i] = i;
     __syncthreads();
-    const CtaTpp T{tsm, ld, m, k, perm, d, s_mx, tid, nt, lane, warp, nw};
+    const CtaTpp<int> T{tsm, ld, m, k, perm, d, s_mx, tid, nt, lane, warp, nw};
     ne = T.run(o, &n1, &n2);
     __syncthreads();
     for (int j = warp; j < k; j += nw) {
@@ -268,7 +272,7 @@ __global__ void __launch_bounds__(TPP_MAX_T) k_tpp_cta(const int32_t* ids, DFron
     }
     for (int i = tid; i < k; i += nt) gperm[i] = perm[i];
   } else {
-    const CtaTpp T{g, m, m, k, gperm, d, s_mx, tid, nt, lane, warp, nw};
+    const CtaTpp<int64_t> T{g, m, m, k, gperm, d, s_mx, tid, nt, lane, warp, nw};
     ne = T.run(o, &n1, &n2);
   }
   if (tid == 0) { F[s].ne = ne; F[s].n1 = n1; F[s].n2 = n2; }

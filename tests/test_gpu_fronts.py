@@ -2,6 +2,7 @@
 leaf fronts of k columns and k + r rows under one dense root of order r."""
 import numpy as np
 import pytest
+import scipy.sparse as sp
 
 from test_gpu_parity import assert_parity, run_both
 
@@ -42,6 +43,26 @@ def check(rv, orc, k, r, kind, **opts):
 @pytest.mark.parametrize("kind", ["plain", "delay", "zero"])
 def test_tpp_fronts(rv, orc, k, r, kind):
     check(rv, orc, k, r, kind, nemin=1)
+
+
+# a small-leaf front with more than 2^31 entries (the threshold is the caller's): its pivots are all zero but
+# the last, so that the factorization is a scan of 46,341 columns
+def test_small_leaf_front_past_32_bit_offsets(rv):
+    n = 46343
+    hub = np.concatenate([[0, 1], np.arange(3, n)])
+    row = np.concatenate([np.arange(n), hub, np.full(n - 1, 2)])
+    col = np.concatenate([np.arange(n), np.full(n - 1, 2), hub])
+    val = np.zeros(row.size)
+    val[n - 1] = -2.0
+    s = rv.problems.from_scipy("hub", sp.csc_matrix((val, (row, col)), shape=(n, n)))
+    solver = rv.SparseLDLT.analyze(s, rv.AnalyzeOptions(rv.OrderingStrategy.USER_SUPPLIED, np.arange(n)))
+    solver.factor(None, rv.FactorOptions(nemin=1, small_leaf_threshold=n))
+    assert solver.stats()["max_front_size"] ** 2 > 2 ** 31
+    assert solver.inertia() == (0, 1, n - 1)
+    col, code, dd, _ = solver.pivot_record()
+    assert np.array_equal(col, np.arange(n)) and np.all(code == 1)
+    assert np.all(dd[:-1] == 0.0) and dd[-1] == -2.0
+    solver.close()
 
 
 @pytest.mark.parametrize("k", [40, 77, 128])

@@ -310,11 +310,12 @@ rvg_status rvg_get_profile(rvg_handle* h, rvg_profile* out);
 rvg_status rvg_mc64(int64_t n, const int64_t* colptr, const int64_t* rowidx, const double* values,
                     int64_t* matching, double* scaling, int64_t* matched);
 
-/* Self-test of the bounded device waits (no reference counterpart): runs one
- * wait that nothing releases, on the handle's stream, and returns the status
+/* Self-test of the bounded device waits (no reference counterpart): runs
+ * waits that nothing releases, on the handle's stream, and returns the status
  * the host then reads: RVG_ERR_DEVICE_TIMEOUT when the wait ran out and was
- * reported (the handle stays usable).  which = 0: a solve block's flag wait
- * (1 s); which = 1: the mixed-form GEMM's pipeline wait (2 s). */
+ * reported (the handle stays usable).  which = 0: the solve's flag wait, then
+ * its wait for a block's values (1 s each; both have to run out); which = 1:
+ * the mixed-form GEMM's pipeline wait (2 s). */
 rvg_status rvg_selftest_waits(rvg_handle* h, int32_t which);
 /* Device memory release (no reference counterpart; the Rust numeric object
  * is dropped whole, solver.rs:312-315).  what: bit 0 = the workspace of

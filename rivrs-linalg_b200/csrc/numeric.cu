@@ -4130,12 +4130,16 @@ rvg_status rvg_set_profiling(rvg_handle* h, int32_t enable) {
   return RVG_OK;
 }
 
-// A one-thread wait on a flag that nothing raises (the solve's flag wait).
+// The solve's waits on what nothing delivers: a flag, and a block's values for 8 right-hand sides.
 __global__ void k_wait_probe(const int32_t* flag, int32_t* err) { sf_wait(flag, err); }
+__global__ void __launch_bounds__(SF_B) k_take_probe(const double* values, int32_t* err) {
+  __shared__ double dst[8][SF_B];
+  sf_take_block<8>(values, SF_B, SF_B, true, dst, err);
+}
 
 rvg_status rvg_selftest_waits(rvg_handle* h, int32_t which) {
   if (!h) { set_error("null handle"); return RVG_ERR_INVALID_INPUT; }
-  if (which != 0 && which != 1) { set_error("which must be 0 (solve flag) or 1 (tensor-core pipeline)"); return RVG_ERR_INVALID_INPUT; }
+  if (which != 0 && which != 1) { set_error("which must be 0 (solve waits) or 1 (tensor-core pipeline)"); return RVG_ERR_INVALID_INPUT; }
   CK(cudaSetDevice(h->device));
   cudaStream_t st = h->st;
   int rc = device_wait_status(h);  // start from a clean error word
@@ -4144,6 +4148,11 @@ rvg_status rvg_selftest_waits(rvg_handle* h, int32_t which) {
   CK(cudaMemsetAsync(h->sf_sync, 0, 2 * sizeof(int32_t), st));
   if (which == 0) {
     k_wait_probe<<<1, 1, 0, st>>>(h->sf_sync, h->d_err);
+    CK(cudaGetLastError());
+    if ((rc = device_wait_status(h)) != RVG_ERR_DEVICE_TIMEOUT) return (rvg_status)rc;
+    if ((rc = ensure(h->solve_work, h->solve_work_cap, 8 * SF_B, st))) return (rvg_status)rc;
+    CK(cudaMemsetAsync(h->solve_work, 0xff, 8 * SF_B * sizeof(double), st));  // SF_EMPTY
+    k_take_probe<<<1, SF_B, 0, st>>>(h->solve_work, h->d_err);
   } else {
     // one 128 x 128 tile, K = 32, operands never copied in: the MMA warp's wait runs out
     double* c = nullptr;

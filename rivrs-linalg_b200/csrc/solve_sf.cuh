@@ -59,12 +59,12 @@
 namespace rvg {
 
 constexpr int SF_B = 64;                            // block rows / columns
-constexpr uint64_t SF_TIMEOUT_NS = 1000000000ull;   // 1 s per wait
-
-// one front of a wave: its first ticket and its block counts
+constexpr uint64_t SF_TIMEOUT_NS = 1000000000ull;   // 1 s until the first wait gives up,
+constexpr uint64_t SF_GIVEN_UP_NS = 1000000ull;     // 1 ms for each wait after that
 constexpr int SF_PG = 8;  // backward: L21 row blocks per partial-sum ticket (512 rows)
 constexpr int SF_BWD_DYN = SF_B * (SF_B + 1) * 8;  // k_sf_bwd's dynamic shared memory
 
+// one front of a wave: its first ticket and its block counts
 struct SfFront {
   int32_t s;      // supernode
   int32_t blk0;   // first ticket of the front
@@ -111,17 +111,24 @@ __device__ __forceinline__ void sf_publish(double* p, double v) {
   const unsigned long long b = v != v ? 0x7ff8000000000000ull : (unsigned long long)__double_as_longlong(v);
   asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(b) : "memory");
 }
+// Whether a wait that began at t0 has run out: after SF_TIMEOUT_NS, or after SF_GIVEN_UP_NS when another one has
+// (a block may have to wait 1 + R times, and all that depends on it again: the limits must not add up).
+__device__ __forceinline__ bool sf_run_out(uint64_t t0, int32_t* err) {
+  const uint64_t dt = sf_timer() - t0;
+  if (dt <= SF_GIVEN_UP_NS) return false;
+  if (dt > SF_TIMEOUT_NS) {
+    atomicExch(err, 2);
+    return true;
+  }
+  return sf_ld_acquire(err) != 0;
+}
 // bounded wait for a published value
 __device__ __forceinline__ double sf_take(const double* p, int32_t* err) {
   unsigned long long v = sf_peek(p);
   if (v == SF_EMPTY) {
     const uint64_t t0 = sf_timer();
-    while ((v = sf_peek(p)) == SF_EMPTY) {
-      if (sf_timer() - t0 > SF_TIMEOUT_NS) {
-        atomicExch(err, 2);
-        return 0.0;
-      }
-    }
+    while ((v = sf_peek(p)) == SF_EMPTY)
+      if (sf_run_out(t0, err)) return 0.0;
   }
   return __longlong_as_double((long long)v);
 }
@@ -150,12 +157,8 @@ __device__ __forceinline__ void sf_take_block(const double* src, int64_t m, int 
 __device__ __forceinline__ void sf_wait(const int32_t* flag, int32_t* err) {
   if (sf_ld_acquire(flag)) return;
   const uint64_t t0 = sf_timer();
-  while (!sf_ld_acquire(flag)) {
-    if (sf_timer() - t0 > SF_TIMEOUT_NS) {
-      atomicExch(err, 2);
-      return;
-    }
-  }
+  while (!sf_ld_acquire(flag))
+    if (sf_run_out(t0, err)) return;
 }
 
 __device__ __forceinline__ int32_t sf_col(const int32_t* rows, const int32_t* perm, int64_t i) { return rows[perm[i]]; }

@@ -4,6 +4,8 @@ RVG_ERR_DEVICE_TIMEOUT, and the handle (and its CUDA context) stays usable.
 The waits are made to run out on purpose without faulting anything: a flag
 that is never raised (the solve's block dependencies) and a tensor-core GEMM
 whose producer issues no copies (the mixed-form pipeline)."""
+import time
+
 import numpy as np
 import pytest
 
@@ -25,6 +27,17 @@ def test_wait_runs_out_and_is_reported(rv, which):
     x, iters, err = solver.solve_refine(b, tol=1e-14, max_iter=10)
     assert err <= 1e-14
     assert solver.inertia() == s.inertia
+    solver.close()
+
+
+# which = 0 runs two waits of 1 s one after the other: a flag, and the values of a block for 8 right-hand sides,
+# whose 1 + 8 waits must not take 1 s each
+def test_limits_of_a_block_do_not_add_up(rv):
+    solver = rv.SparseLDLT.analyze(rv.problems.shifted_laplacian(4, 0.1))
+    solver.factor()
+    t0 = time.perf_counter()
+    assert rv._native.lib().rvg_selftest_waits(solver._handle, 0) == RVG_ERR_DEVICE_TIMEOUT
+    assert 1.9 < time.perf_counter() - t0 < 4.0
     solver.close()
 
 

@@ -41,20 +41,33 @@ def device_memory():
     return int(out[0]), int(out[1])
 
 
-def memory_estimate(sym, outer_block: int = 256, nrhs: int = 8) -> tuple:
+LF_FEW, LF_ROUTED_MAX = 16, 16  # numeric.cu: fronts of a wave that may take the large fronts' path below the threshold
+
+
+def memory_estimate(sym, outer_block: int = 256, nrhs: int = 8, large_front_threshold: int = 2048) -> tuple:
     """(factor bytes, workspace bytes) of one system's numeric phase, from its
     supernode structure and the delay-free level-set schedule: the factor is
-    every front's m x k panel (8 bytes) plus indices and D; the workspace is
-    the largest sum over a wave of the fronts' scratch plus the contribution
-    blocks alive across waves (nfs^2 doubles each, from the child's wave to
-    its parent's), and the solve vectors.  An upper bound of what the device
-    arenas take (they are sized the same way)."""
+    every front's m x k panel (8 bytes) plus indices and D, with the arenas'
+    margins; the workspace is the largest sum over a wave of the fronts'
+    scratch plus the contribution blocks alive across waves (nfs^2 doubles
+    each, from the child's wave to its parent's), and the solve vectors.
+
+    Scratch: 64 m doubles for a front on one CTA; a window of 4 outer blocks
+    more (and its packed operands, and nfs k doubles for the contribution
+    GEMM's W) for a large one, i.e. of order >= large_front_threshold, or >= half
+    of it where the wave holds at most LF_FEW such fronts.  Of the others, the
+    LF_ROUTED_MAX largest of a wave may take the large fronts' path (which ones
+    depends on the wave), so all of those are charged the window.  The sum of
+    several systems' estimates therefore covers their union, in whose waves the
+    same numbers hold once.  Delayed columns, nemin amalgamation and the
+    matrix itself are not counted."""
     k = (sym.sup_end - sym.sup_begin).astype(np.int64)
     r = np.diff(sym.pat_ptr).astype(np.int64)
     m = k + r
     par = sym.sup_parent
     ns = k.size
-    factor = float(np.sum(m * k)) * 8 * (1 + 1 / 16) + float(np.sum(m + k)) * 4 + float(np.sum(k)) * 17
+    factor = float(np.sum(m * k)) * 8 * (1 + 1 / 16) + float(np.sum(m + k)) * 4 * (1 + 1 / 16) + \
+        float(np.sum(k)) * 17 * (1 + 1 / 8)
     h = np.zeros(ns, np.int64)
     for s in range(ns):  # children precede their parents
         if par[s] >= 0 and h[par[s]] < h[s] + 1:
@@ -62,14 +75,23 @@ def memory_estimate(sym, outer_block: int = 256, nrhs: int = 8) -> tuple:
     nh = int(h.max()) + 2 if ns else 1
     cb = (r.astype(np.float64) ** 2) * 8
     live = np.zeros(nh + 1)
-    scr = np.zeros(nh + 1)
     for s in range(ns):
         if par[s] >= 0 and r[s] > 0:
             live[h[s]:h[par[s]] + 1] += cb[s]
-        sc = (2 * 32 * m[s] + outer_block) * 8
-        if m[s] >= 2048:
-            sc = (m[s] * (2 * 32 + 4 * outer_block) + outer_block) * 8 + 2 * m[s] * 4 * outer_block * 8
-        scr[h[s]] += max(sc, r[s] * k[s] * 8)
+    T = large_front_threshold
+    scratch = (2 * 32 * m + outer_block) * 8.0
+    window = m * (4.0 * outer_block) * 8
+    large = m >= T
+    mid = (m >= T // 2) & (m < T) & (k >= 32)
+    large |= mid & (np.bincount(h[mid], minlength=nh)[h] <= LF_FEW)
+    # rank of each remaining medium front within its wave, largest first
+    cand = np.nonzero(~large & (m >= T // 16) & (k >= 32))[0]
+    cand = cand[np.lexsort((-m[cand], h[cand]))]
+    hc = h[cand]
+    rank = np.arange(cand.size) - np.searchsorted(hc, hc)
+    scratch[cand[rank < LF_ROUTED_MAX]] += window[cand[rank < LF_ROUTED_MAX]]
+    scratch[large] = np.maximum(scratch[large] + window[large], 8.0 * r[large] * k[large]) + 2 * window[large]
+    scr = np.bincount(h, weights=scratch, minlength=nh + 1)
     work = float(np.max(live + scr)) + 2.0 * nrhs * float(np.sum(m)) * 8 + 16.0 * float(np.sum(m))
     return factor, work
 

@@ -4,6 +4,7 @@ same ordering and scaling, refactorization with new values matches too, and
 every system's solution meets the backward-error gate."""
 import numpy as np
 import pytest
+import scipy.sparse as sp
 
 pytestmark = pytest.mark.gpu
 
@@ -180,3 +181,36 @@ def test_refactorizations_replay_as_graphs_across_turns(rv, precision):
                     assert rv.problems.backward_error(sv, x[:, j], bb[:, j]) <= 1e-14
     dyn.close()
     rep.close()
+
+
+def hub_blocks(rv, order, count):
+    # `count` independent fronts of the given order: an arrow whose hub goes first fills completely
+    rng = np.random.default_rng(order)
+    n = order * count
+    hub = np.repeat(np.arange(count) * order, order - 1)
+    leaf = np.delete(np.arange(n), np.arange(count) * order)
+    row = np.concatenate([np.arange(n), leaf, hub])
+    col = np.concatenate([np.arange(n), hub, leaf])
+    off = rng.standard_normal(leaf.size)
+    val = np.concatenate([rng.uniform(50.0, 100.0, n), off, off])
+    return rv.problems.from_scipy(f"hub{order}x{count}", sp.csc_matrix((val, (row, col)), shape=(n, n)))
+
+
+# fronts below the large-front threshold that take the large fronts' path (order 1000) need its scratch: the
+# estimate covers what the arenas take.  Their memory is mapped on demand here, so the device's free memory
+# shows it.
+def test_memory_estimate_covers_routed_fronts(rv):
+    opts = rv.FactorOptions(graph_refactor=2)
+
+    def taken(s):
+        solver = rv.SparseLDLT.analyze(s, rv.AnalyzeOptions(rv.OrderingStrategy.USER_SUPPLIED, np.arange(s.n)))
+        before = rv.batch.device_memory()[0]
+        solver.factor(None, opts)
+        used = before - rv.batch.device_memory()[0]
+        est = sum(rv.batch.memory_estimate(solver.symbolic))
+        solver.close()
+        return used, est
+
+    taken(hub_blocks(rv, 1000, 4))  # modules, streams and pools
+    used, est = taken(hub_blocks(rv, 1000, 16))
+    assert 16 * 1000 * 1000 * 8 < used <= 1.1 * est

@@ -3030,8 +3030,8 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
       n_small_launches++;
     }
     for (const TppLaunch& t : tpp_launches) {
-      launch_beside(group, k_tpp_cta, (unsigned)t.count, (unsigned)t.threads, t.smem, st,
-                    (const int32_t*)(D + o_tpp) + t.first, h->d_fronts, A, dop, (int)(t.smem > 0));
+      launch_beside(group, t.smem ? k_tpp_cta<true> : k_tpp_cta<false>, (unsigned)t.count, (unsigned)t.threads, t.smem,
+                    st, (const int32_t*)(D + o_tpp) + t.first, h->d_fronts, A, dop);
       group = true;
       n_small_launches++;
     }
@@ -3327,7 +3327,7 @@ rvg_status rvg_create(int64_t n, int64_t nsup, const int64_t* sup_begin, const i
   CK(cudaMallocHost((void**)&h->h_norms, 4 * sizeof(double)));
   if (o.graph_refactor == 2 && (rc = vm_create(h.get()))) return (rvg_status)rc;  // address-stable arenas
   if ((rc = presize_arenas(h.get()))) return (rvg_status)rc;
-  CK(cudaFuncSetAttribute(k_tpp_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TPP_SMEM_MAX));
+  CK(cudaFuncSetAttribute(k_tpp_cta<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TPP_SMEM_MAX));
   CK(cudaFuncSetAttribute(k_syrk_lower, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G_SMEM));
   CK(cudaFuncSetAttribute(k_syrk_tc<1, TC_TF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
   CK(cudaFuncSetAttribute(k_syrk_tc<2, TC_TF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));

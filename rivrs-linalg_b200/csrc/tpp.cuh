@@ -233,12 +233,15 @@ struct CtaTpp {
   }
 };
 
-// One CTA per front.  smem = 1: the front (its lower trapezoid, leading
-// dimension m | 1: row scans hit different banks) and its pivot order live in
-// dynamic shared memory meanwhile; 0: it stays in global memory.
+// One CTA per front.  SMEM: the front (its lower trapezoid, leading dimension
+// m | 1: row scans hit different banks) and its pivot order live in dynamic
+// shared memory meanwhile; else it stays in global memory.  Two kernels of 64
+// registers: one that holds both kinds of offsets takes 78, with which 3 instead
+// of 4 CTAs of 256 threads fit on a multiprocessor.
 __host__ __device__ __forceinline__ int tpp_ld(int m) { return m | 1; }
 
-__global__ void __launch_bounds__(TPP_MAX_T) k_tpp_cta(const int32_t* ids, DFront* F, Arenas A, DevOpts o, int smem) {
+template <bool SMEM>
+__global__ void __launch_bounds__(TPP_MAX_T) k_tpp_cta(const int32_t* ids, DFront* F, Arenas A, DevOpts o) {
   extern __shared__ double tsm[];
   __shared__ double s_mx[2];
   wave_kernel_enter();
@@ -250,7 +253,7 @@ __global__ void __launch_bounds__(TPP_MAX_T) k_tpp_cta(const int32_t* ids, DFron
   int32_t* gperm = A.idx + fr.idx + m;
   const DRec d{A.dtype + fr.dpos, A.ddiag + fr.dpos, A.doff + fr.dpos};
   int n1 = 0, n2 = 0, ne;
-  if (smem) {
+  if constexpr (SMEM) {
     const int ld = tpp_ld(m);
     int32_t* perm = (int32_t*)(tsm + (size_t)ld * k);
     for (int j = warp; j < k; j += nw) {

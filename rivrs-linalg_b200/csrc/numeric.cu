@@ -1212,9 +1212,10 @@ __global__ void k_front_growth(const int32_t* ids, const DFront* F, Arenas A, do
 using namespace rvg;
 
 // One large front in flight: the stream its launches go to, its pivot state
-// on the device and the packed window of its mixed-form updates.  Context 0
-// is the handle's own stream; the others let the large fronts of one wave run
-// side by side (one host thread each).
+// on the device and the packed window of its mixed-form updates.  Context 0 is
+// on the handle's own stream, or on one of its own while the wave's other fronts
+// are queued there; the others let the large fronts of one wave run side by side
+// (one host thread each).
 constexpr int LF_AHEAD = 8;  // outer blocks of a large front issued ahead of the host's check of their start
 struct LfCtx {
   cudaStream_t st = nullptr;
@@ -1274,6 +1275,7 @@ struct rvg_handle {
   int32_t* h_counts = nullptr; size_t h_counts_cap = 0;
   LFState* d_lf = nullptr;                          // state of the large-front path
   std::vector<LfCtx> lfx;                            // concurrent large-front contexts 1.. (0 = the handle's)
+  cudaStream_t lf_st = nullptr;                      // context 0's stream beside the small and medium fronts
   int64_t* d_colptr = nullptr;                      // matrix pattern (full symmetric CSC = its own CSR)
   int32_t* d_rowidx = nullptr;
   double a_fro = 0;                                 // ||A||_F of the last factored values
@@ -1862,7 +1864,7 @@ std::vector<int> route_medium(const std::vector<std::pair<int64_t, int64_t>>& mk
   std::partial_sort(c.begin(), c.begin() + top, c.end(), [](const auto& a, const auto& b) {
     return a.first > b.first || (a.first == b.first && a.second < b.second);
   });
-  const int ctx = LF_CONCURRENT - 1;
+  const int ctx = LF_CONCURRENT;
   int best = 0;
   double best_t = c.empty() ? 0 : 0.9 * c[0].first, sum = 0, longest = 0;
   for (int j = 1; j <= (int)std::min<size_t>(c.size(), LF_ROUTED_MAX); ++j) {
@@ -2520,15 +2522,18 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
 // each context's fronts in turn on its own host thread and stream, ordered
 // after the wave's assembly and before what follows by events.  beside: the
 // event behind the assembly when the wave's small and medium fronts are queued
-// on the handle's stream meanwhile; the large ones then use the other
-// contexts' streams only and run beside them.
+// on the handle's stream meanwhile; context 0 then has a stream of its own too
+// and the large ones run beside them.
 int factor_large_fronts(rvg_handle* h, const std::vector<int32_t>& ids, const Arenas& A, const DevOpts& dop,
                         cudaEvent_t beside = nullptr) {
   if (ids.empty()) return RVG_OK;
   if (h->lfx.empty()) {
     h->lfx.resize(1);
-    h->lfx[0].st = h->st;
     h->lfx[0].lf = h->d_lf;
+  }
+  if (beside && !h->lf_st) {
+    if (tl_no_alloc) return no_alloc_fail();
+    CK(cudaStreamCreateWithFlags(&h->lf_st, cudaStreamNonBlocking));
   }
   auto fold = [&](LfCtx& c) {
     h->launches += c.launches;
@@ -2541,8 +2546,7 @@ int factor_large_fronts(rvg_handle* h, const std::vector<int32_t>& ids, const Ar
   };
   // (a capture forks into the same contexts with the fronts dealt the same way:
   // the replayed graph runs them concurrently on the buffers the dynamic run sized)
-  const int first = beside ? 1 : 0;  // the first context used
-  const int nc = (int)std::min<size_t>(ids.size() + first, LF_CONCURRENT);
+  const int nc = (int)std::min<size_t>(ids.size(), LF_CONCURRENT);
   while ((int)h->lfx.size() < nc) {  // grown before any reference into lfx is taken
     if (tl_no_alloc) return no_alloc_fail();
     LfCtx c;
@@ -2553,6 +2557,7 @@ int factor_large_fronts(rvg_handle* h, const std::vector<int32_t>& ids, const Ar
     h->lfx.push_back(c);
   }
   LfCtx& c0 = h->lfx[0];
+  c0.st = beside ? h->lf_st : h->st;
   c0.wpack = h->wpack; c0.wpack_cap = h->wpack_cap;
   int rc = RVG_OK;
   if (nc == 1 && !beside) {
@@ -2570,7 +2575,8 @@ int factor_large_fronts(rvg_handle* h, const std::vector<int32_t>& ids, const Ar
     ready = h->ev_large;
   }
   if (!beside) CK(cudaEventRecord(ready, h->st));
-  for (int t = 1; t < nc; ++t) CK(cudaStreamWaitEvent(h->lfx[t].st, beside ? beside : ready, 0));
+  const int first = beside ? 0 : 1;  // the first context not on the handle's stream
+  for (int t = first; t < nc; ++t) CK(cudaStreamWaitEvent(h->lfx[t].st, beside ? beside : ready, 0));
   std::vector<int> rcs(nc, RVG_OK);
   std::vector<std::string> errs(nc);
   const bool no_alloc = tl_no_alloc;
@@ -2580,21 +2586,21 @@ int factor_large_fronts(rvg_handle* h, const std::vector<int32_t>& ids, const Ar
     tl_no_alloc = no_alloc;
     LfCtx& c = h->lfx[t];
     c.marks = false;
-    for (size_t i = t - first; i < ids.size(); i += nc - first)
+    for (size_t i = t; i < ids.size(); i += nc)
       if ((rcs[t] = factor_large_front(h, c, ids[i], A, dop))) { errs[t] = g_err; break; }
     tl_no_alloc = was;
   };
   std::vector<std::thread> th;
-  for (int t = first + 1; t < nc; ++t) th.emplace_back(work, t);
-  work(first);
+  for (int t = 1; t < nc; ++t) th.emplace_back(work, t);
+  work(0);
   for (auto& x : th) x.join();
   h->wpack = c0.wpack; h->wpack_cap = c0.wpack_cap;
-  for (int t = 1; t < nc; ++t) {
+  for (int t = first; t < nc; ++t) {
     CK(cudaEventRecord(ready, h->lfx[t].st));
     CK(cudaStreamWaitEvent(h->st, ready, 0));
   }
   mark(h, RVG_PART_OTHER);
-  for (int t = first; t < nc; ++t) {
+  for (int t = 0; t < nc; ++t) {
     fold(h->lfx[t]);
     if (rcs[t] && !rc) { rc = rcs[t]; set_error(errs[t]); }
   }
@@ -4374,6 +4380,7 @@ void rvg_destroy(rvg_handle* h) {
     if (c.lf) cudaFree(c.lf);
     if (c.own && c.st) { cudaStreamSynchronize(c.st); cudaStreamDestroy(c.st); }
   }
+  if (h->lf_st) { cudaStreamSynchronize(h->lf_st); cudaStreamDestroy(h->lf_st); }
   fr(h->d_err);
   fr(h->d_colptr); fr(h->d_rowidx); fr(h->d_ref);
   if (st) { cudaStreamSynchronize(st); cudaStreamDestroy(st); }

@@ -79,6 +79,29 @@ def test_medium_fronts(rv, orc, k, r, kind, threshold):
     check(rv, orc, k, r, kind, small_leaf_threshold=0, large_front_threshold=threshold)
 
 
+# more large fronts than there are contexts for them, beside small and medium ones: the first context leaves the
+# handle's stream to those and comes back to it for the root
+@pytest.mark.parametrize("count", [1, 8, 9])
+def test_large_fronts_beside_small_ones(rv, orc, count):
+    sizes = np.array([300] * count + [70] * 6 + [20] * 6)
+    r = 260
+    first = np.cumsum(sizes) - sizes
+    n = int(sizes.sum()) + r
+    rng = np.random.default_rng(count)
+    a = np.zeros((n, n))
+    for f, k in zip(first, sizes):
+        a[f:f + k, f:f + k] = rng.standard_normal((k, k))
+        a[n - r:, f:f + k] = rng.standard_normal((r, k)) * (rng.random((r, 1)) < 0.3)
+    a[n - r:, n - r:] = rng.standard_normal((r, r))
+    a = a + a.T
+    s = rv.problems.from_scipy("beside", a)
+    solver, ref, b = run_both(rv, orc, s, order=np.arange(n, dtype=np.int64), nemin=1, small_leaf_threshold=0,
+                              large_front_threshold=310)
+    assert_parity(rv, s, solver, ref, b, bwd=1e-12)
+    solver.close()
+    ref.close()
+
+
 # the medium fronts that take the large fronts' path keep FP64 updates in the mixed form
 def test_routed_fronts_stay_fp64(rv):
     s = arrow_system(rv, 450, 60, 3, "plain")

@@ -2523,9 +2523,11 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
 // after the wave's assembly and before what follows by events.  beside: the
 // event behind the assembly when the wave's small and medium fronts are queued
 // on the handle's stream meanwhile; context 0 then has a stream of its own too
-// and the large ones run beside them.
+// and the large ones run beside them.  counted: ids[0] is the wave's only large
+// front, the others medium ones on its path: its GEMMs are counted as if it
+// were alone.
 int factor_large_fronts(rvg_handle* h, const std::vector<int32_t>& ids, const Arenas& A, const DevOpts& dop,
-                        cudaEvent_t beside = nullptr) {
+                        cudaEvent_t beside = nullptr, bool counted = false) {
   if (ids.empty()) return RVG_OK;
   if (h->lfx.empty()) {
     h->lfx.resize(1);
@@ -2585,9 +2587,10 @@ int factor_large_fronts(rvg_handle* h, const std::vector<int32_t>& ids, const Ar
     const bool was = tl_no_alloc;
     tl_no_alloc = no_alloc;
     LfCtx& c = h->lfx[t];
-    c.marks = false;
-    for (size_t i = t; i < ids.size(); i += nc)
+    for (size_t i = t; i < ids.size(); i += nc) {
+      c.marks = counted && i == 0;
       if ((rcs[t] = factor_large_front(h, c, ids[i], A, dop))) { errs[t] = g_err; break; }
+    }
     tl_no_alloc = was;
   };
   std::vector<std::thread> th;
@@ -3053,7 +3056,13 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
       }
       h->sel_large.insert(h->sel_large.end(), large_ids.begin(), large_ids.end());
     }
-    if ((rc = factor_large_fronts(h, lf_ids, A, dop, beside ? h->ev_beside : nullptr))) return rc;
+    const bool counted = large_ids.size() == 1;
+    if (counted && !routed_ids.empty() && h->profiling) {  // the large front alone: it carries the profiling marks
+      if ((rc = factor_large_fronts(h, large_ids, A, dop)) || (rc = factor_large_fronts(h, routed_ids, A, dop)))
+        return rc;
+    } else if ((rc = factor_large_fronts(h, lf_ids, A, dop, beside ? h->ev_beside : nullptr, counted))) {
+      return rc;
+    }
     CK(cudaEventRecord(h->ev[3], st));
     // ---- contribution GEMM (fronts with nothing eliminated skip inside)
     mark(h, -1);

@@ -2,6 +2,7 @@
 aggregate FactorizationStats and with the oracle's fronts."""
 import numpy as np
 import pytest
+import scipy.sparse as sp
 
 pytestmark = pytest.mark.gpu
 
@@ -23,3 +24,37 @@ def test_per_supernode_stats_sum_to_the_totals(rv, orc):
     assert np.array_equal(solver.front_info()[:, :5], ref.front_info()[:, :5])
     ref.close()
     solver.close()
+
+
+def dense_fronts(rv, orders):
+    # one front of each order: an arrow whose hub goes first fills completely
+    orders = np.asarray(orders)
+    first = np.cumsum(orders) - orders
+    n = int(orders.sum())
+    rng = np.random.default_rng(1)
+    hub, leaf = np.repeat(first, orders - 1), np.delete(np.arange(n), first)
+    off = rng.standard_normal(leaf.size)
+    row, col = np.concatenate([np.arange(n), leaf, hub]), np.concatenate([np.arange(n), hub, leaf])
+    val = np.concatenate([rng.uniform(50.0, 100.0, n), off, off])
+    return rv.problems.from_scipy("fronts", sp.csc_matrix((val, (row, col)), shape=(n, n)))
+
+
+# the Schur GEMMs of a wave's only large front (order 1100) are counted whatever runs beside it: small and medium
+# fronts, medium fronts (order 600) that take its path, or both
+@pytest.mark.parametrize("others", [[40] * 5, [600] * 3, [600] * 3 + [40] * 5])
+def test_schur_gemm_counters_of_a_lone_large_front(rv, others):
+    def counters(orders, profiling):
+        s = dense_fronts(rv, orders)
+        solver = rv.SparseLDLT.analyze(s, rv.AnalyzeOptions(rv.OrderingStrategy.USER_SUPPLIED, np.arange(s.n)))
+        solver.factor()
+        solver.set_profiling(profiling)
+        solver.factor()
+        p = solver.profile()
+        assert solver.inertia()[2] == 0 and (p["syrk_ms"] > 0) == profiling
+        solver.close()
+        return p["syrk_launches"], p["syrk_flops"]
+
+    alone = counters([1100], False)
+    assert alone[0] > 0 and alone[1] > 0
+    for profiling in (False, True):
+        assert counters([1100] + others, profiling) == alone

@@ -2717,13 +2717,31 @@ int refactor_fp64(rvg_handle* h, const std::vector<int32_t>& redo, const Arenas&
 // Launches of a wave's TPP fronts (one CTA each, k_tpp_cta), which sorts them
 // by size, largest first.  A launch's CTAs all reserve the shared memory of its
 // largest front, so the fronts are split where 8, 4, 2 or 1 of them fit on a
-// multiprocessor (28 / 56 / 112 / 226 KB; larger ones stay in global memory),
-// and a smaller class joins the launch above it while that still runs in one
-// go (fewer launches; the multiprocessors have room).  Threads: a front's steps
-// are latency bound, so 256 while every CTA is resident at that width; where a
-// class has several rounds of CTAs its fronts share the issue slots, and two
-// warps per front waste fewer of them on the decisions every warp repeats.
+// multiprocessor (larger ones stay in global memory), and a smaller class joins
+// the launch above it while that still runs in one go: a launch less, the same
+// device time (100 fronts of order 80 and 300 of order 24: 113 us together, 110
+// apart; 50 of 110 and 200 of 24: 171 and 171).
+//
+// Threads: 256.  A front's steps are latency bound, and where 4 CTAs or fewer
+// share a multiprocessor its issue slots are not (us, 256 / 128 / 64 threads: 600
+// fronts of order 80 236 / 281 / 419, 600 of 160 1449 / 2188 / 3843, in global
+// memory 600 of 200 1930 / 2409 / 4222).  Small fronts (27 KB) fit 8 to a
+// multiprocessor but their registers only at 128 threads, and fewer warps waste
+// fewer issue slots on the decisions every warp repeats: 128 above two CTAs a
+// multiprocessor (order 24: 296 fronts 40 / 42 / 50 and 600 64 / 46 / 52; order
+// 55: 296 81 / 91 / 124, 600 145 / 112 / 136), 64 where they come in several
+// rounds and are short (1800 of 40 212 / 149 / 130, of 55 306 / 224 / 261).
 struct TppLaunch { int first, count, threads; size_t smem; };
+
+// classes of at most `bytes` per front, of which `ctas` fit on a multiprocessor
+struct TppClass { size_t bytes; int ctas; };
+constexpr TppClass TPP_CLASS[4] = {{TPP_SMEM_MAX, 1}, {112 * 1024, 2}, {55 * 1024, 4}, {27 * 1024, 8}};
+constexpr bool tpp_class_fits(const TppClass& c, int threads) {  // 228 KB, of which 1 KB a CTA is the system's
+  return (c.bytes + 1024 + 128) * c.ctas <= 228 * 1024 && c.ctas * threads <= TPP_CTAS * TPP_MAX_T;
+}
+static_assert(tpp_class_fits(TPP_CLASS[0], 256) && tpp_class_fits(TPP_CLASS[1], 256) &&
+                  tpp_class_fits(TPP_CLASS[2], 256) && tpp_class_fits(TPP_CLASS[3], 128),
+              "TPP classes by the CTAs that fit");
 
 std::vector<TppLaunch> plan_tpp(const rvg_handle* h, std::vector<int32_t>& ids) {
   std::vector<TppLaunch> out;
@@ -2733,21 +2751,18 @@ std::vector<TppLaunch> plan_tpp(const rvg_handle* h, std::vector<int32_t>& ids) 
     return (size_t)tpp_ld(f.m) * f.k * 8 + (size_t)f.k * 4;
   };
   std::stable_sort(ids.begin(), ids.end(), [&](int32_t a, int32_t b) { return bytes(a) > bytes(b); });
-  constexpr size_t KB = 1024;
-  const size_t lim[5] = {SIZE_MAX, TPP_SMEM_MAX, 112 * KB, 56 * KB, 28 * KB};  // class c: at most lim[c] bytes
-  const int per_sm[5] = {8, 1, 2, 4, 8};
   const int n = (int)ids.size();
   int i = 0;
   while (i < n) {
     const size_t b = bytes(ids[i]);
-    int c = 4;
-    while (b > lim[c]) --c;
-    const int cap = per_sm[c] * h->nsm;
+    int c = 3;  // -1: global memory
+    while (c >= 0 && b > TPP_CLASS[c].bytes) --c;
     int e = i;
-    while (e < n && (c == 4 || bytes(ids[e]) > lim[c + 1])) ++e;
-    if (c > 0 && e - i < cap) e = std::min(n, i + cap) == n ? n : e;  // the rest fits beside it
-    TppLaunch t{i, e - i, 0, c == 0 ? 0 : b};
-    t.threads = t.count <= cap ? 256 : (c == 4 ? 64 : 128);
+    while (e < n && (c == 3 || bytes(ids[e]) > TPP_CLASS[c + 1].bytes)) ++e;
+    if (c >= 0 && n - i <= TPP_CLASS[c].ctas * h->nsm) e = n;  // the rest fits beside it
+    TppLaunch t{i, e - i, 256, c < 0 ? 0 : b};
+    if (c == 3 && t.count > 2 * h->nsm)
+      t.threads = t.count > TPP_CLASS[c].ctas * h->nsm && b <= 18 * 1024 ? 64 : 128;
     out.push_back(t);
     i = e;
   }

@@ -27,6 +27,7 @@
 namespace rvg {
 
 constexpr int TPP_MAX_T = 256;               // threads of a CTA at most
+constexpr int TPP_CTAS = 4;                  // such CTAs on a multiprocessor: 64 registers a thread
 constexpr size_t TPP_SMEM_MAX = 226 * 1024;  // dynamic shared memory of a CTA at most
 
 // Off: int where the front is in shared memory, int64_t where it is in global
@@ -241,7 +242,7 @@ struct CtaTpp {
 __host__ __device__ __forceinline__ int tpp_ld(int m) { return m | 1; }
 
 template <bool SMEM>
-__global__ void __launch_bounds__(TPP_MAX_T) k_tpp_cta(const int32_t* ids, DFront* F, Arenas A, DevOpts o) {
+__global__ void __launch_bounds__(TPP_MAX_T, TPP_CTAS) k_tpp_cta(const int32_t* ids, DFront* F, Arenas A, DevOpts o) {
   extern __shared__ double tsm[];
   __shared__ double s_mx[2];
   wave_kernel_enter();

@@ -36,13 +36,27 @@ def check(rv, orc, k, r, kind, **opts):
     ref.close()
 
 
-# (k, r): one column, odd sizes, warp remainders; then fronts on either side of the 28, 56, 112 and 226 KB of
+# (k, r): one column, odd sizes, warp remainders; then fronts on either side of the 27, 55, 112 and 226 KB of
 # shared memory at which the launch changes, the last one too large for it
 @pytest.mark.parametrize("k,r", [(1, 3), (2, 1), (5, 33), (31, 32), (31, 82), (31, 90), (31, 200), (31, 430),
                                  (31, 880), (31, 940)])
 @pytest.mark.parametrize("kind", ["plain", "delay", "zero"])
 def test_tpp_fronts(rv, orc, k, r, kind):
     check(rv, orc, k, r, kind, nemin=1)
+
+
+# as many fronts in a wave as change the width of their CTAs (148 multiprocessors: 128 threads above 296 fronts,
+# 64 above 1184)
+@pytest.mark.parametrize("count", [297, 1185])
+def test_many_tpp_fronts(rv, orc, count):
+    k = 13
+    rng = np.random.default_rng(count)
+    blocks = rng.standard_normal((count, k, k)) * (rng.random((count, 1, 1)) + 0.1)
+    s = rv.problems.from_scipy("many", sp.block_diag([b + b.T for b in blocks]))
+    solver, ref, b = run_both(rv, orc, s, order=np.arange(s.n, dtype=np.int64))
+    assert_parity(rv, s, solver, ref, b, bwd=1e-12)
+    solver.close()
+    ref.close()
 
 
 # a small-leaf front with more than 2^31 entries (the threshold is the caller's): its pivots are all zero but

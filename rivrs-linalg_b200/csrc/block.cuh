@@ -51,7 +51,7 @@ struct CtaShared {
   int tmpi;
   double dinv[IBMAX];
   unsigned two;  // bit c: a 2x2 pivot starts at c
-  alignas(16) double TT[IBMAX][IBMAX + 2];  // the factored block transposed: TT[l][j] = L(j, l) (panel_rows)
+  alignas(16) double TT[IBMAX][IBMAX + 2];  // the factored block transposed: TT[l][j] = L(j, l) (panel_row_t)
   // cta_block_factor only
   double Tb[IBMAX][IBMAX + 1];  // the other buffer of the trailing block
   double Lc[IBMAX][IBMAX + 1];  // Lc[c][r]: finished column c at the row of original index r
@@ -288,12 +288,6 @@ __device__ __forceinline__ int panel_row_t(double (&x)[IBMAX], const double (*TT
     }
   }
   return bad ? __ffs(bad) - 1 : n;
-}
-__device__ __forceinline__ int panel_row(double (&x)[IBMAX], const double (*TT)[IBMAX + 2], unsigned two,
-                                         const double* bdd, const double* bdo, const double* dinv, int n,
-                                         double bound) {
-  return n == IBMAX ? panel_row_t<true>(x, TT, two, bdd, bdo, dinv, n, bound)
-                    : panel_row_t<false>(x, TT, two, bdd, bdo, dinv, n, bound);
 }
 
 // The row's W = L D (compute_ld_into, factor.rs:1536-1563) in place of x, for

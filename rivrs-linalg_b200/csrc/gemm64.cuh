@@ -10,16 +10,14 @@
 // 256-column outer block) and the NFS x NFS contribution block
 // (compute_contribution_gemm, factor.rs:1590-1652).
 //
-// sm_100a has no FP64 tcgen05 kind.  The library uses the FP64 tensor-core
-// mma.sync (DMMA) kernel below; the register-blocked SIMT DFMA kernel
-// k_syrk_lower_t is kept as the reference formulation.  SIMT design:
-// kernel: 128 x 128 CTA tile, 256 threads (one CTA per SM: the 64 FP64
-// accumulators of a thread take 128 registers), 8 x 8 outputs per thread
-// (rows tx + 16a, columns ty + 16b so C loads and stores coalesce along
-// columns), K staged through shared memory in chunks of 16 by cp.async in a
-// three-stage pipeline (8-byte copies: panel leading dimensions are odd in
-// general; out-of-range elements are zero-filled by the copy itself).  Each output keeps one fma chain in K order, so the result is
-// bit-identical to the oracle's per-entry loop.
+// sm_100a has no FP64 tcgen05 kind: the kernel uses the FP64 tensor-core
+// mma.sync (DMMA), K staged through shared memory in chunks of 16 by cp.async in
+// a three-stage pipeline (8-byte copies: panel leading dimensions are odd in
+// general; out-of-range elements are zero-filled by the copy itself).  Each
+// 8x8x4 step adds a chain of four products to the accumulator in k order, so
+// each output keeps one fma chain in K order and the result is bit-identical to
+// the oracle's per-entry loop (checked on the device).  WR x WC warps of 32 x 32
+// outputs (4 x 4 fragments of 8 x 8); W is negated when its fragments are read.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -53,116 +51,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-// NT threads; thread (tx = tid % 16, ty = tid / 16) owns rows tx + 16x
-// (x < TM) and columns ty + (NT/16) y (y < TN) of a (16 TM) x ((NT/16) TN)
-// tile.
-template <int NT, int TM, int TN>
-struct SyrkCfg {
-  static constexpr int BM = 16 * TM, BN = (NT / 16) * TN, CSTR = NT / 16;
-  static constexpr size_t SMEM = (size_t)G_STAGES * G_BK * (BM + BN) * sizeof(double);
-};
-
-template <int NT, int TM, int TN, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_syrk_lower_t(SyrkArgs a) {
-  using Cfg = SyrkCfg<NT, TM, TN>;
-  constexpr int BM = Cfg::BM, BN = Cfg::BN, CS = Cfg::CSTR;
-  const int64_t i0 = a.r0 + (int64_t)blockIdx.y * BM;
-  const int64_t j0 = a.c0 + (int64_t)blockIdx.x * BN;
-  if (i0 >= a.r1 || j0 >= a.c1) return;
-  if (i0 + BM - 1 < j0) return;  // tile entirely above the diagonal
-  if ((a.cond && *a.cond >= a.cond_lt) || (a.skip && *a.skip)) return;
-  const int64_t K = (a.Kdev ? (int64_t)*a.Kdev : 0) + a.K;
-  extern __shared__ double gsm[];
-  // stage s: W chunk [k][BM] then L chunk [k][BN]
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int64_t nchunk = (K + G_BK - 1) / G_BK;
-  auto issue = [&](int64_t ch) {
-    double* sw = gsm + (ch % G_STAGES) * G_BK * (BM + BN);
-    double* sl = sw + G_BK * BM;
-    const int64_t k0 = ch * G_BK;
-#pragma unroll
-    for (int e = 0; e < (G_BK * BM) / NT; ++e) {
-      const int idx = tid + NT * e;
-      const int r = idx % BM, k = idx / BM;
-      const int64_t kk = k0 + k, i = i0 + r;
-      const bool v = kk < K && i < a.r1;
-      cp_async8(sw + k * BM + r, v ? a.W + (i - a.r0) + kk * a.ldw : a.W, v);
-    }
-#pragma unroll
-    for (int e = 0; e < (G_BK * BN) / NT; ++e) {
-      const int idx = tid + NT * e;
-      const int r = idx % BN, k = idx / BN;
-      const int64_t kk = k0 + k, j = j0 + r;
-      const bool v = kk < K && j < a.c1;
-      cp_async8(sl + k * BN + r, v ? a.L + j + kk * a.ldl : a.L, v);
-    }
-  };
-#pragma unroll
-  for (int s = 0; s < G_STAGES - 1; ++s) {
-    if (s < nchunk) issue(s);
-    cp_async_commit();
-  }
-  double acc[TM][TN];
-#pragma unroll
-  for (int x = 0; x < TM; ++x)
-#pragma unroll
-    for (int y = 0; y < TN; ++y) {
-      const int64_t i = i0 + tx + 16 * x, j = j0 + ty + CS * y;
-      acc[x][y] = (i < a.r1 && j < a.c1 && i >= j) ? a.C[i + j * a.ldc] : 0.0;
-    }
-  for (int64_t ch = 0; ch < nchunk; ++ch) {
-    cp_async_wait<G_STAGES - 2>();  // chunk ch has landed
-    __syncthreads();                // ... for every thread, and chunk ch-1's buffer is free
-    if (ch + G_STAGES - 1 < nchunk) issue(ch + G_STAGES - 1);
-    cp_async_commit();
-    const double* sw = gsm + (ch % G_STAGES) * G_BK * (BM + BN);
-    const double* sl = sw + G_BK * BM;
-    const int kc = (int)((K - ch * G_BK) < G_BK ? (K - ch * G_BK) : G_BK);
-    if (kc == G_BK) {
-#pragma unroll
-      for (int k = 0; k < G_BK; ++k) {
-        double wv[TM], lv[TN];
-#pragma unroll
-        for (int x = 0; x < TM; ++x) wv[x] = -sw[k * BM + tx + 16 * x];
-#pragma unroll
-        for (int y = 0; y < TN; ++y) lv[y] = sl[k * BN + ty + CS * y];
-#pragma unroll
-        for (int x = 0; x < TM; ++x)
-#pragma unroll
-          for (int y = 0; y < TN; ++y) acc[x][y] = __fma_rn(wv[x], lv[y], acc[x][y]);
-      }
-    } else {
-      for (int k = 0; k < kc; ++k) {
-        double wv[TM], lv[TN];
-#pragma unroll
-        for (int x = 0; x < TM; ++x) wv[x] = -sw[k * BM + tx + 16 * x];
-#pragma unroll
-        for (int y = 0; y < TN; ++y) lv[y] = sl[k * BN + ty + CS * y];
-#pragma unroll
-        for (int x = 0; x < TM; ++x)
-#pragma unroll
-          for (int y = 0; y < TN; ++y) acc[x][y] = __fma_rn(wv[x], lv[y], acc[x][y]);
-      }
-    }
-  }
-  cp_async_wait<0>();
-#pragma unroll
-  for (int x = 0; x < TM; ++x)
-#pragma unroll
-    for (int y = 0; y < TN; ++y) {
-      const int64_t i = i0 + tx + 16 * x, j = j0 + ty + CS * y;
-      if (i < a.r1 && j < a.c1 && i >= j) a.C[i + j * a.ldc] = acc[x][y];
-    }
-}
-
-// ---------------------------------------------------------------------------
-// FP64 tensor-core variant: mma.sync m8n8k4 (DMMA).  Each 8x8x4 step adds a
-// chain of four products to the accumulator in k order, the same
-// per-output fma sequence as the SIMT kernel and the oracle (checked bit for
-// bit on the device).  WR x WC warps of 32 x 32 outputs (4 x 4 fragments of
-// 8 x 8); W is negated when its fragments are read.
-// ---------------------------------------------------------------------------
 template <int WR, int WC>
 struct DmmaCfg {
   static constexpr int NT = 32 * WR * WC, BM = 32 * WR, BN = 32 * WC;
@@ -275,21 +163,15 @@ __global__ void __launch_bounds__(32 * WR * WC, MINB) k_syrk_dmma(SyrkArgs a) {
 // four CTAs per SM (the fastest of the measured shapes on a 9600^2 rank-1024
 // update: 31.3 TFLOP/s; 128 x 64 with 4 or 8 warps 30.3 and 30.8, 64 x 128 29.4,
 // 128 x 128 26.8; a fourth stage or tiles walked in groups of rows change nothing)
-#ifndef RVG_SYRK_WR
-#define RVG_SYRK_WR 2
-#define RVG_SYRK_WC 2
-#define RVG_SYRK_MINB 4
-#endif
-using SyrkMain = DmmaCfg<RVG_SYRK_WR, RVG_SYRK_WC>;
+constexpr int SYRK_WR = 2, SYRK_WC = 2, SYRK_MINB = 4;
+using SyrkMain = DmmaCfg<SYRK_WR, SYRK_WC>;
 constexpr int G_T = SyrkMain::NT;
 constexpr size_t G_SMEM = SyrkMain::SMEM;
-#define k_syrk_lower k_syrk_dmma<RVG_SYRK_WR, RVG_SYRK_WC, RVG_SYRK_MINB>
+constexpr auto k_syrk_lower = k_syrk_dmma<SYRK_WR, SYRK_WC, SYRK_MINB>;
 
-template <class Cfg>
-inline dim3 syrk_grid_cfg(const SyrkArgs& a) {
-  int64_t nr = (a.r1 - a.r0 + Cfg::BM - 1) / Cfg::BM, nc = (a.c1 - a.c0 + Cfg::BN - 1) / Cfg::BN;
+inline dim3 syrk_grid(const SyrkArgs& a) {
+  int64_t nr = (a.r1 - a.r0 + SyrkMain::BM - 1) / SyrkMain::BM, nc = (a.c1 - a.c0 + SyrkMain::BN - 1) / SyrkMain::BN;
   return dim3((unsigned)(nc > 0 ? nc : 0), (unsigned)(nr > 0 ? nr : 0));
 }
-inline dim3 syrk_grid(const SyrkArgs& a) { return syrk_grid_cfg<SyrkMain>(a); }
 
 }  // namespace rvg

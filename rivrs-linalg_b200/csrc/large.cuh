@@ -83,7 +83,7 @@ struct LFArgs {
   double* w;        // inner W, rows x 32 (column-major, ld = rows of the view)
   double* wo;       // pending W (column-major, ld wld): row i, pending column c at wo[(i - wrow0) + c * wld]
   int64_t wld, wrow0, wcol0;  // leading dimension, first row, this block's first pending column
-  int64_t cs, bcols, nfsb;  // outer block start, width, NFS boundary (global p)
+  int64_t cs, bcols;  // outer block start, width
   int par;          // which of the state's two blocks is the current inner block
   int win;          // the rows below the outer block keep their W (the outer block joins the window)
   int outer;        // the outer block's number (lp is one of two arrays, by its parity)

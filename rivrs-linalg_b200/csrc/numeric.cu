@@ -2200,7 +2200,6 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
   const bool mixed = front_mixed(h, s);
   const int64_t F = lf_window_cols(h, nb, mixed);
   int32_t* const lp2 = (int32_t*)(sc + m * (2 * IBMAX + lf_window_blocks(h) * nb));  // two arrays of nb
-  a.nfsb = p;
   a.o = dop;
   const int two_level = p > nb;
   const int64_t Fq = F / TC_BK;

@@ -1836,14 +1836,22 @@ inline bool front_is_large(int64_t m, bool tpp, int64_t T, int64_t mid) {
 
 // Medium fronts that would hold a wave up on one CTA go to the large fronts'
 // path (results do not depend on it).  One CTA's time grows with the front's
-// trailing tiles, the whole GPU's hardly: measured for one dense front of order
-// n (B200), 128: 130 / 103 us, 256: 366 / 253, 512: 1525 / 630, 1000: 7300 /
-// 1540, which the two models below follow.  The queue runs all its fronts at
-// once, the large path up to `ctx` at a time beside it, each further one with a
-// host thread to start: the j longest fronts move where that makes the longer of
-// the two shortest, and only if it saves a tenth.  Only fronts of order >= T / 16
-// (128 at the default threshold) count, so the threshold still turns the path
-// off; they keep the FP64 updates in every precision.
+// trailing tiles, the whole GPU's hardly.  Measured for one dense front (us on
+// one CTA / on the whole GPU; in brackets what the two models below give):
+//   order 128   152 / 130   (125 / 185)      384    803 / 378   (692 / 505)
+//         192   248 / 185   (213 / 243)      512   1415 / 481  (1288 / 661)
+//         256   363 / 236   (330 / 306)     1000   6884 / 1027 (7088 / 1561)
+// The second model is on the safe side, by 1.3 to 1.5 times: a dense front moves
+// from order 320 or so on (as routed: 320 570 us, 384 376), where alone it would
+// gain from 192 on already.  The queue runs all its fronts at once, the large
+// path up to `ctx` at a time beside it, each further one with a host thread to
+// start: the j longest fronts move where that makes the longer of the two
+// shortest, and only if it saves a tenth.  (That the queue's CTAs may have to
+// take turns, above two fronts a multiprocessor, is left out: the large path then
+// gets the multiprocessors as the queue empties: 1500 fronts of order 300 take 4.5
+// ms, with one of order 600 beside them 4.7.)  Only fronts of order >= T / 16 (128
+// at the default threshold) count, so the threshold still turns the path off; they
+// keep the FP64 updates in every precision.
 constexpr int LF_ROUTED_MAX = 16;
 double cta_front_us(double m, double k) {
   double t = 0;
@@ -3030,7 +3038,10 @@ int run_factor(rvg_handle* h, const double* d_vals, const double* d_scal) {
     }
     // ---- dense factorization
     mark(h, -1);
-    // large fronts beside the small and medium ones (one after the other while the profiling marks are on)
+    // large fronts beside the small and medium ones (one after the other while the profiling marks are on).
+    // Beside: up to two medium fronts a multiprocessor, which all run from the start; the queue's CTAs fill
+    // the GPU then, and of a longer queue the large fronts see the end only (one of order 1500 with 296 fronts of
+    // order 300: 2.5 ms; 1500 such fronts alone 4.5, with it 5.7)
     std::vector<int32_t> lf_ids(large_ids);
     lf_ids.insert(lf_ids.end(), routed_ids.begin(), routed_ids.end());
     const bool beside = !lf_ids.empty() && !(aptp_ids.empty() && tpp_ids.empty()) && !h->profiling;
@@ -3625,8 +3636,10 @@ static int solve_common(rvg_handle* h, double* d_rhs, int64_t nrhs, int64_t ldb)
   // right-hand sides per pass: 8, 4, 2 or 1.  A pass costs the factor's read
   // and the chain of its diagonal blocks whatever its width, so the last
   // columns go through one pass of the next width up (5 to 7 as 8, 3 as 4)
-  // beside columns of zeros, not through several narrow ones (KKT 36^3: a pass
-  // of 8 takes 5.4 ms, of 1 2.6 ms)
+  // beside columns of zeros, not through several narrow ones.  Passes of 1 / 2 /
+  // 4 / 8 columns take 2.45 / 3.36 / 3.76 / 5.37 ms on a KKT 36^3, 3.03 / 4.01 /
+  // 4.49 / 6.37 on a 64^3 Laplacian and 0.25 / 0.31 / 0.34 / 0.44 on a 16^3 one:
+  // 4 is less than 2 + 1 (5.81, 7.04, 0.55), 8 less than 4 + 1 (6.21, 7.53, 0.58)
   auto pass = [](int64_t left) { return left > 4 ? 8 : left > 2 ? 4 : (int)left; };
   const int rmax = pass(nrhs);
   const int64_t npad = nrhs / 8 * 8 + pass(nrhs % 8);

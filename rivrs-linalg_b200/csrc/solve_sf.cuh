@@ -31,7 +31,7 @@
 //     cols]^T x_final of those blocks (each once it is there), then the unit
 //     upper solve (L11^T) of the diagonal block; x[col] = x_final.
 //
-// The chain of diagonal blocks bounds a large front (212 blocks for order
+// The chain of diagonal blocks bounds a large front (213 blocks for order
 // 13,572), so what a block does between its predecessor's values and its own
 // is kept short:
 //   * the values are their own flags: the work vectors are filled with a
@@ -41,7 +41,8 @@
 //     instead of fence, flag, flag read and value read); the many blocks
 //     further away watch one value with one thread, to keep the traffic on
 //     those lines low;
-//   * the sums over 64 columns run as four interleaved chains;
+//   * the sums over 64 columns run as interleaved chains (forward four with up to
+//     two right-hand sides, two with more; backward four);
 //   * the diagonal block is solved by eights (sf_diag): 8 or 16 short barriers
 //     instead of 64 warp-serial steps, all right-hand sides side by side.
 // What a solve needs to know of the factor (block layout, the front of each
@@ -182,7 +183,7 @@ __device__ __forceinline__ void sf_load_strip(const double* src, int64_t m, int 
   }
 }
 
-// acc[r] -= sum_c l[c] y[r][c] over a 64-column strip: four interleaved chains per right-hand side
+// acc[r] -= sum_c l[c] y[r][c] over a 64-column strip: W interleaved chains per right-hand side
 // (columns past the block hold l = 0, y is finite or the front's result is not)
 template <int R>
 __device__ __forceinline__ void sf_strip(const double (&l)[SF_B], int n, const double (*y)[SF_B], double (&acc)[R]) {

@@ -68,6 +68,7 @@ struct LFState {
   // later launch of the front returns at once until the host clears it
   int32_t spec_bad;
   int32_t done;  // CTAs of a k_lf_update with failed columns that have finished
+  int32_t far_bne, far_skip;  // bne and spec_bad as they were when the far-field update on the far stream was forked
   int32_t valid[2];  // the outer block (its number + 1) that began last with each parity
   LFBlk b[2];    // inner block i is b[i & 1]: the update of block i factors block i + 1
 };
@@ -542,6 +543,16 @@ __global__ void __launch_bounds__(NT) k_lf_outer(LFArgs A, int64_t rem, int two_
     st->gne = g;
     if (host_gne) *host_gne = g;
   }
+}
+
+// What a far-field update on the far stream reads of the state, taken on the
+// front's stream before the fork: the chain goes on meanwhile, and the next
+// block's k_lf_begin_outer clears bne and may set spec_bad while CTAs of the
+// update have not started yet (another front's GEMM can hold their
+// multiprocessors).  One far-field update runs at a time.
+__global__ void k_lf_far(LFState* st) {
+  st->far_bne = st->bne;
+  st->far_skip = st->spec_bad;
 }
 
 // The delay swap of an outer block issued without it (k_lf_outer with swap =

@@ -2362,14 +2362,17 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
           const int64_t split = oe + far_ahead * nb;
           if (async_far && p - split >= 2 * nb) {
             // the next far_ahead blocks' columns now, the rest on the far stream beside them (both
-            // after the packs; they touch different columns)
+            // after the packs; they touch different columns).  The far part takes its counts from k_lf_far:
+            // the state itself moves on with the next blocks
+            k_lf_far<<<1, 1, 0, st>>>(a.st);
             ck(cudaEventRecord(cx.ev_fork, st), "cudaEventRecord (far-field fork)");
             ck(cudaStreamWaitEvent(cx.far_st, cx.ev_fork, 0), "cudaStreamWaitEvent (far-field fork)");
             irc = irc ? irc : launch_window_gemm(h, cx, a, m, oe, split, wd, wrow, F, pk_w, pk_l, kadd, bne_dev,
                                                  nullptr, 0, mixed, skip);
-            irc = irc ? irc : launch_window_gemm(h, cx, a, m, split, p, wd, wrow, F, pk_w, pk_l, kadd, bne_dev,
-                                                 nullptr, 0, mixed, skip, cx.far_st, h->nsm - far_sms);
+            irc = irc ? irc : launch_window_gemm(h, cx, a, m, split, p, wd, wrow, F, pk_w, pk_l, kadd, &a.st->far_bne,
+                                                 nullptr, 0, mixed, &a.st->far_skip, cx.far_st, h->nsm - far_sms);
             ck(cudaEventRecord(cx.ev_far, cx.far_st), "cudaEventRecord (far-field join)");
+            cx.launches++;
             cx.far_launches++;
             I.far = true;
           } else {

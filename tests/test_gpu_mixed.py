@@ -236,6 +236,35 @@ def test_auto_refinement_escalates_only_when_needed(rv):
     solver.close()
 
 
+def test_far_field_overlap_of_concurrent_fronts(rv):
+    """Far-field updates of eight fronts at once, each on its front's second stream: an update whose CTAs have to
+    wait for another front's takes the counts of its own window, not those the chain has reached meanwhile, and
+    runs although a later block (or its own: weak columns) turned out to be issued for the wrong column."""
+    import scipy.sparse as sp
+    n, count = 1200, 8
+    rng = np.random.default_rng(5)
+    blocks = []
+    for q in range(count):
+        a = rng.standard_normal((n, n))
+        a = a + a.T
+        weak = np.arange(250 + 130 * q, 270 + 130 * q) % n
+        a[weak, :] *= 1e-3
+        a[:, weak] *= 1e-3
+        blocks.append(sp.csc_matrix(a))
+    s = rv.problems.from_scipy("eight", sp.block_diag(blocks))
+    opts = dict(precision="mixed", mixed_flush=0, mixed_operands="bf16", large_front_threshold=1000,
+                outer_block_size=128, mixed_window=2)
+    solver = rv.SparseLDLT.analyze(s, rv.AnalyzeOptions(rv.OrderingStrategy.USER_SUPPLIED, np.arange(s.n)))
+    solver.factor(None, rv.FactorOptions(far_field_sms=0, **opts))
+    assert solver.profile()["lf_far_updates"] == 0 and solver.profile()["lf_misses"] > 0
+    ref = [x.copy() for x in solver.pivot_record()]
+    for _ in range(4):
+        solver.factor(None, rv.FactorOptions(**opts))
+        assert solver.profile()["lf_far_updates"] > 0
+        assert all(np.array_equal(x, y) for x, y in zip(solver.pivot_record(), ref))
+    solver.close()
+
+
 @pytest.mark.parametrize("case,window", [("dense_delay", 0), ("kkt26", 0), ("dense_delay", 8), ("kkt26", 8)])
 def test_far_field_overlap_is_bit_identical(rv, case, window):
     """A full window's far-field update runs on a second stream beside the next window's outer blocks but

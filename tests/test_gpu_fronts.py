@@ -52,7 +52,7 @@ def test_many_tpp_fronts(rv, orc, count):
     k = 13
     rng = np.random.default_rng(count)
     blocks = rng.standard_normal((count, k, k)) * (rng.random((count, 1, 1)) + 0.1)
-    s = rv.problems.from_scipy("many", sp.block_diag([b + b.T for b in blocks]))
+    s = rv.problems.from_scipy("many", sp.block_diag([sp.csc_matrix(b + b.T) for b in blocks]))
     solver, ref, b = run_both(rv, orc, s, order=np.arange(s.n, dtype=np.int64))
     assert_parity(rv, s, solver, ref, b, bwd=1e-12)
     solver.close()

@@ -472,17 +472,22 @@ __global__ void __launch_bounds__(NT, 2) k_lf_update(LFArgs A, int next) {
 }
 
 // row permutation of the outer block applied to the front's earlier columns
-// 0..cs (two_level_factor, factor.rs:2165-2181): 16 columns per CTA.  Nothing
+// 0..cs (two_level_factor, factor.rs:2165-2181): 16 columns per CTA, fewer where
+// blocks are so wide that 48 KB hold fewer (above 384 columns).  Nothing
 // on the front's path reads those rows again, so it runs on a stream of its own
 // beside the blocks that follow (12 to 17 us of ~290 per outer block of a
 // 13,572 front); it acts if its outer block really began, whatever a later,
 // mispredicted one has flagged meanwhile.
-constexpr int LF_PROP_COLS = 16;
-__global__ void __launch_bounds__(256) k_lf_prop(LFArgs A) {
+constexpr int LF_PROP_SMEM_MAX = 224 * 1024;  // one column of a block of 28,672
+inline int lf_prop_cols(int64_t bcols) {
+  const int64_t c = 48 * 1024 / (8 * bcols);
+  return (int)(c < 1 ? 1 : c < 16 ? c : 16);
+}
+__global__ void __launch_bounds__(256) k_lf_prop(LFArgs A, int cols) {
   if (A.st->valid[A.outer & 1] != A.outer + 1) return;
-  extern __shared__ double buf[];  // bcols x LF_PROP_COLS
-  const int64_t c0 = (int64_t)blockIdx.x * LF_PROP_COLS;
-  const int nc = (int)((A.cs - c0) < LF_PROP_COLS ? (A.cs - c0) : LF_PROP_COLS);
+  extern __shared__ double buf[];  // bcols x cols
+  const int64_t c0 = (int64_t)blockIdx.x * cols;
+  const int nc = (int)((A.cs - c0) < cols ? (A.cs - c0) : cols);
   if (nc <= 0) return;
   const int bc = (int)A.bcols;
   for (int t = threadIdx.x; t < nc * bc; t += blockDim.x) {

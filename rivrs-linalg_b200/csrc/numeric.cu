@@ -2326,7 +2326,8 @@ int factor_large_front(rvg_handle* h, LfCtx& cx, int32_t s, const Arenas& Ar, co
           ck(cudaEventRecord(cx.ev_prop_fork, st), "cudaEventRecord (row permutation fork)");
           ck(cudaStreamWaitEvent(ps, cx.ev_prop_fork, 0), "cudaStreamWaitEvent (row permutation fork)");
         }
-        k_lf_prop<<<(unsigned)((cs + LF_PROP_COLS - 1) / LF_PROP_COLS), 256, (size_t)bcols * LF_PROP_COLS * 8, ps>>>(a);
+        const int pc = lf_prop_cols(bcols);
+        k_lf_prop<<<(unsigned)((cs + pc - 1) / pc), 256, (size_t)bcols * pc * 8, ps>>>(a, pc);
         if (side_prop) {
           ck(cudaEventRecord(cx.ev_prop[opar], ps), "cudaEventRecord (row permutation)");
           prop_due[opar] = true;
@@ -3370,6 +3371,7 @@ rvg_status rvg_create(int64_t n, int64_t nsup, const int64_t* sup_begin, const i
   CK(cudaMallocHost((void**)&h->h_norms, 4 * sizeof(double)));
   if (o.graph_refactor == 2 && (rc = vm_create(h.get()))) return (rvg_status)rc;  // address-stable arenas
   if ((rc = presize_arenas(h.get()))) return (rvg_status)rc;
+  CK(cudaFuncSetAttribute(k_lf_prop, cudaFuncAttributeMaxDynamicSharedMemorySize, LF_PROP_SMEM_MAX));
   CK(cudaFuncSetAttribute(k_tpp_cta<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TPP_SMEM_MAX));
   CK(cudaFuncSetAttribute(k_syrk_lower, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G_SMEM));
   CK(cudaFuncSetAttribute(k_syrk_tc<1, TC_TF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));

@@ -135,6 +135,14 @@ def test_medium_fronts_block_sizes(rv, orc, ib, nb):
     check(rv, orc, 150, 45, "delay", small_leaf_threshold=0, inner_block_size=ib, outer_block_size=nb)
 
 
+# outer blocks whose row permutation does not fit 16 columns in a CTA's default shared memory, on fronts that the
+# wave moves to the large fronts' path and on large ones
+@pytest.mark.parametrize("nb", [448, 1024])
+@pytest.mark.parametrize("opts", [{}, {"large_front_threshold": 600}])
+def test_wide_outer_blocks(rv, orc, nb, opts):
+    check(rv, orc, nb + 170, 45, "delay", outer_block_size=nb, **opts)
+
+
 # every width a pass of the solve can have (8, 4, 2, 1 columns, the last one padded), over fronts of one and
 # several 64-column blocks with remainders
 @pytest.mark.parametrize("nrhs", [2, 3, 5, 7, 8, 9, 13])

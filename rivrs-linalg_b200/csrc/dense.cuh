@@ -111,6 +111,9 @@ struct WarpTpp {
   }
   __device__ __forceinline__ int64_t row_abs_max(int64_t p, int64_t from, int64_t to) const {  // 2695-2710
     if (from >= to) return from;
+    // the scan starts from the first entry; nothing is larger than a NaN there (and a row of NaN has no other)
+    const double first = sym(p, from);
+    if (first != first) return from;
     double bv = -1.0;
     int64_t bk = INT64_MAX;
     for (int64_t c = from + lane; c < to; c += 32) {

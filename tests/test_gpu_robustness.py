@@ -76,3 +76,20 @@ def test_power_of_two_boundaries(rv, orc, n):
     solver, ref, b = run_both(rv, orc, s)
     assert_parity(rv, s, solver, ref, b, bwd=5e-11)
     solver.close()
+
+
+def test_tpp_row_that_starts_with_nan(rv, orc):
+    """The scan for a row's largest entry starts from its first one (factor.rs:2695-2710): a NaN there is kept, and
+    names a column of the front.  (A factorization rejects NaN input; its own overflows can make one, and the
+    allocation-free entry point takes the front as it is.)"""
+    torch = pytest.importorskip("torch")
+    from test_zz_no_alloc import dense_matrix, no_alloc_call
+    for n, at in ((2, (1, 0)), (10, (1, 0)), (24, (5, 0))):
+        a = dense_matrix(n, 40 + n, "plain")
+        a[at] = a[at[::-1]] = np.nan
+        _, perm, dt, dd, do, st, _ = orc.dense_aptp(a.copy(), p=n)
+        gperm, gdt, gdd, gdo, cnt = no_alloc_call(rv, torch, a)
+        ne = int(st[0])
+        assert tuple(int(c) for c in cnt) == (ne, int(st[1]), int(st[2]))
+        assert np.array_equal(gperm[:ne], perm[:ne]) and np.array_equal(gdt[:ne], dt[:ne])
+        assert np.array_equal(gdd[:ne], dd[:ne], equal_nan=True) and np.array_equal(gdo[:ne], do[:ne], equal_nan=True)

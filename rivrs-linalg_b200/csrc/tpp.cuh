@@ -159,13 +159,15 @@ struct CtaTpp {
   __device__ int run(const DevOpts& o, int* n1, int* n2) const {
     const double u = o.threshold, small = o.small;
     const WarpTpp T{PanelView{a, ld}, m, n, lane};
+    // (with no limit, 0, the maxima cannot tell a column of zeros from one without a number: scan it)
+    const bool limit = small > 0.0;
     int ne = 0, c1 = 0, c2 = 0;
     scan(0);
     __syncthreads();
     while (ne < n) {
       const double mt = mx[0], mp = mx[1];
       const double ann = fabs(at(ne, ne)), sub = ne + 1 < m ? fabs(at(ne + 1, ne)) : 0.0;
-      if (!(ann >= small || mt >= small || (ne + 1 < m && sub >= small))) {
+      if (limit ? !(ann >= small || mt >= small || sub >= small) : T.col_small(ne, ne, m, small)) {
         zero_pivot(ne);
         ++c1;
         ne += 1;
@@ -179,16 +181,16 @@ struct CtaTpp {
         double maxt = mt, maxp = mp;
         bool tiny;
         if (p == ne + 1) {
-          tiny = !(sub >= small || fabs(at(p, p)) >= small || mp >= small);
+          tiny = limit ? !(sub >= small || fabs(at(p, p)) >= small || mp >= small) : T.col_small(p, ne, m, small);
         } else {
           tiny = T.col_small(p, ne, m, small);
           if (!tiny) {
-            const int64_t tt = T.row_abs_max(p, ne, p);
-            t = tt < p ? (int)tt : ne;  // (a row of NaN has no maximum)
+            t = (int)T.row_abs_max(p, ne, p);
             maxt = T.rc_abs_max_excl(t, ne, p);
             maxp = T.rc_abs_max_excl(p, ne, t);
           }
         }
+        if (!limit && p == ne + 1) __syncthreads();  // every warp has scanned the columns that apply_2x2 writes
         if (tiny) {
           swap(p, ne);
           zero_pivot(ne);

@@ -45,6 +45,23 @@ def test_tpp_fronts(rv, orc, k, r, kind):
     check(rv, orc, k, r, kind, nemin=1)
 
 
+# small = 0: a column of zeros is a pivot like any other (1 / 0), and the columns that it turns into NaN are zero
+# pivots; both in the shared-memory and the global-memory version
+@pytest.mark.parametrize("k,r", [(7, 3), (31, 32), (90, 40), (200, 30)])
+def test_zero_columns_without_a_limit(rv, orc, k, r):
+    s = arrow_system(rv, k, r, 7 * k + r, "plain")
+    row, col = s.rowidx, np.repeat(np.arange(s.n), np.diff(s.colptr))
+    zero = np.isin(row, [1, k // 2, k - 1]) | np.isin(col, [1, k // 2, k - 1])
+    s.values[zero] = 0.0
+    solver, ref, _ = run_both(rv, orc, s, order=np.arange(s.n, dtype=np.int64), small=0.0)
+    assert solver.inertia() == ref.inertia()
+    assert np.array_equal(solver.front_info()[:, :5], ref.front_info()[:, :5])
+    for x, y in zip(solver.pivot_record(), ref.pivot_record()):
+        assert np.array_equal(x, y, equal_nan=x.dtype == np.float64)
+    solver.close()
+    ref.close()
+
+
 # as many fronts in a wave as change the width of their CTAs (148 multiprocessors: 128 threads above 296 fronts,
 # 64 above 1184)
 @pytest.mark.parametrize("count", [297, 1185])
